@@ -54,7 +54,7 @@ enum I32Col : int {
   I_SPEC = 13,             // specimen of a batched domain (0 otherwise)
   NI32_PERSIST = 14,
   I_CELL = 14,             // scratch: cell key (Morton rank) of the particle at its pre-search position
-  I_CLASS = 15,            // scratch: pair-rule class word in sorted order
+  I_TMP = 15,              // scratch of the search's ordering
   NI32 = 16
 };
 
@@ -123,6 +123,7 @@ constexpr int MAX_NB = 100;  // MAX_NB_PER_PART, Source/Domain.h:49
 
 constexpr int MAX_CP = 64;   // contact pairs per particle
 constexpr int SUP_W = 128;   // superset entries per particle (skin reuse of the search)
+constexpr int BRICK_CAP = 4096;  // particles of a brick that the search orders in shared memory
 
 // Shared-memory staging of the mixed form's gathers.  Particles are taken in
 // blocks of STAGE_B consecutive (cell-sorted) particles; at every search each
@@ -237,6 +238,7 @@ struct DomainConst {
   int CellNo[3];
   double rec_origin[3];  // the mixed form's position records hold x - rec_origin (the cell grid's centre)
   int ncells;
+  int nbricks;         // bricks of cells (with those of the shadow buckets): the units of the storage order
   float pre_eps;       // relative margin of the FP32 neighbour prefilter
   float cell_skip_r2;  // (Cellfac * hmax + FP32 rounding margin)^2: cells farther hold no neighbour
   float CellSizef[3];  // FP32 copy of the cell size
@@ -303,6 +305,10 @@ struct DevPtrs {
   const int* cell_lin;    // Morton rank -> linear cell
   int* cell_start;        // ncells + 1
   int* cell_count;        // ncells (histogram / cursor)
+  const int* brick_cell;  // nbricks + 1: brick b holds the cells of ranks [brick_cell[b], brick_cell[b + 1])
+  int* cell_list;         // sorted position of the particle in each slot of the cells' lists (cell_start)
+  float4* cand_x;         // per slot of the cells' lists: FP32 prefilter coordinates and h of its particle
+  int4* cand_m;           // and its sorted index, original index, class word of the pair rules, specimen
   int* perm;              // new sorted position -> old sorted position
   int* inv;               // original index -> sorted position
   float* xs;              // FP32 prefilter coordinates (x - BLPF, 3 columns) and h
