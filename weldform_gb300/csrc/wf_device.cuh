@@ -76,11 +76,14 @@ enum I32Col : int {
 // besides its FP32 rounding: for a domain of half-extent D that is
 // 1.2e-10 D / |x_ij| relative (2e-8 for D = 30 mm at a 0.2 mm spacing, below
 // the 6e-8 of the FP32 rounding itself), wherever the domain sits.  A
-// velocity difference carries about 2^-33 |v| in the same way.
+// velocity difference carries about 2^-33 |v| in the same way.  The six high
+// halves lie across two groups in the order of the low halves, so the pairs
+// (x, y), (z, vx) and (vy, vz) sit in the same registers of both and a
+// neighbour's six differences take nine packed two-element FP32 instructions.
 enum RecCur : int {        // current-state groups
-  RC_XH = 0,               // x hi (xyz), h
+  RC_XV = 0,               // x hi (xyz), v hi x
   RC_L = 1,                // x lo, v lo (bf16 pairs), m/rho
-  RC_VH = 2,               // v hi (xyz), rho
+  RC_VW = 2,               // v hi y z, h, rho (uniform-particle layout: Sigma/rho^2 xz, yz)
   RC_S0 = 3,               // Sigma/rho^2 xx yy zz xy
   RC_S1 = 4,               // Sigma/rho^2 xz yz, mass, Cs
   RC_MISC = 5,             // alpha, beta, k_T, T hi
@@ -90,10 +93,9 @@ enum RecCur : int {        // current-state groups
   RC_N = 9
 };
 enum RecNext : int {       // next-step groups
-  RN_XH = 0,               // x(n+1) hi, h
+  RN_XV = 0,               // x(n+1) hi, v(n+1) hi x
   RN_L = 1,                // x(n+1) lo, v(n+1) lo (bf16 pairs), m/rho(n+1)
-  RN_VH = 2,               // v(n+1) hi, p/rho^2 at rho(n+1) (the rate gather's kinetic term;
-                           // the current group carries rho there)
+  RN_VW = 2,               // v(n+1) hi y z, h, p/rho^2 at rho(n+1) (the rate gather's kinetic term)
   RN_E = 3,                // p/rho^2 at rho(n+1), k_T, T(n+1) hi, T(n+1) lo
   RN_N = 4
 };
@@ -268,8 +270,8 @@ struct DomainConst {
   int m_pair;
   // Uniform-particle layout of the mixed records: every solid particle has the
   // same h and Cs, the pairs' masses agree (m_pair), and the staged gather is
-  // off.  The current records then carry Sigma/rho^2 xz in RC_XH.w and yz in
-  // RC_VH.w (instead of h and rho), so the acceleration gather reads four
+  // off.  The current records then carry Sigma/rho^2 xz and yz in the last two
+  // fields of RC_VW (instead of h and rho), so the acceleration gather reads four
   // groups per neighbour instead of five, rho_j = m_i / (m/rho)_j, and every
   // gather uses the kernel constants of the one h below instead of forming
   // 1/h per pair.

@@ -40,12 +40,6 @@ __device__ __forceinline__ void ff_split(double v, float& hi, float& lo) {
   hi = __double2float_rn(v);
   lo = __double2float_rn(v - (double)hi);
 }
-__device__ __forceinline__ float* rc_f(const DevPtrs& P, size_t N, int i, int q) {
-  return reinterpret_cast<float*>(P.rc + (size_t)q * N + i);
-}
-__device__ __forceinline__ float* rn_f(const DevPtrs& P, size_t N, int i, int q) {
-  return reinterpret_cast<float*>(P.rn + (size_t)q * N + i);
-}
 // Low-half group: x = (xlo0, xlo1), y = (xlo2, vlo0), z = (vlo1, vlo2) as bf16
 // pairs (first value in the low 16 bits), w = a float.  A bf16 is the upper
 // half of an FP32, so unpacking is a shift or a mask.
@@ -58,34 +52,34 @@ __device__ __forceinline__ float bf16_second(float p) { return __uint_as_float(_
 __device__ __forceinline__ float4 lo_pack(const float xl[3], const float vl[3], float w) {
   return make_float4(bf16_pair(xl[0], xl[1]), bf16_pair(xl[2], vl[0]), bf16_pair(vl[1], vl[2]), w);
 }
-__device__ __forceinline__ void lo_unpack(float4 g, float xl[3], float vl[3]) {
-  xl[0] = bf16_first(g.x); xl[1] = bf16_second(g.x); xl[2] = bf16_first(g.y);
-  vl[0] = bf16_second(g.y); vl[1] = bf16_first(g.z); vl[2] = bf16_second(g.z);
-}
 // v lo component d sits in 16-bit half 3 + d of the group.
 __device__ __forceinline__ unsigned short* lo_v_half(float4* group, int d) {
   return reinterpret_cast<unsigned short*>(group) + 3 + d;
 }
 
 // Velocity component d of particle i into the current (next) float4 groups.
+__device__ __forceinline__ float* rec_v_hi(float4* r, size_t N, int d) {  // r: the record's column base + i
+  return d == 0 ? reinterpret_cast<float*>(r + (size_t)RC_XV * N) + 3 : reinterpret_cast<float*>(r + (size_t)RC_VW * N) + d - 1;
+}
 __device__ __forceinline__ void rec_set_v(const DevPtrs& P, size_t N, int i, int d, double v, bool next) {
+  static_assert((int)RN_XV == (int)RC_XV && (int)RN_VW == (int)RC_VW && (int)RN_L == (int)RC_L, "same places in both records");
+  float4* r = (next ? P.rn : P.rc) + i;
   float h, l;
   ff_split(v, h, l);
-  if (next) { rn_f(P, N, i, RN_VH)[d] = h; *lo_v_half(P.rn + (size_t)RN_L * N + i, d) = bf16_bits(l); }
-  else { rc_f(P, N, i, RC_VH)[d] = h; *lo_v_half(P.rc + (size_t)RC_L * N + i, d) = bf16_bits(l); }
+  *rec_v_hi(r, N, d) = h;
+  *lo_v_half(r + (size_t)RC_L * N, d) = bf16_bits(l);
 }
 
 // The current velocity record of particle i from its three FP64 components
-// (the .w field and the x lo halves carried over).
+// (the other fields of the three groups carried over).
 __device__ __forceinline__ void rec_set_v3(const DevPtrs& P, size_t N, int i, const double v[3]) {
   float4* r = P.rc + i;
-  float4 h = r[(size_t)RC_VH * N];
-  float l[3];
-  ff_split(v[0], h.x, l[0]);
-  ff_split(v[1], h.y, l[1]);
-  ff_split(v[2], h.z, l[2]);
-  r[(size_t)RC_VH * N] = h;
-  for (int d = 0; d < 3; ++d) *lo_v_half(r + (size_t)RC_L * N, d) = bf16_bits(l[d]);
+  float h[3], l[3];
+  for (int d = 0; d < 3; ++d) ff_split(v[d], h[d], l[d]);
+  *rec_v_hi(r, N, 0) = h[0];
+  *reinterpret_cast<float2*>(r + (size_t)RC_VW * N) = make_float2(h[1], h[2]);
+  *lo_v_half(r + (size_t)RC_L * N, 0) = bf16_bits(l[0]);
+  reinterpret_cast<float*>(r + (size_t)RC_L * N)[2] = bf16_pair(l[1], l[2]);
 }
 
 // Batched domain: flag the particle's specimen as yielding once its plastic

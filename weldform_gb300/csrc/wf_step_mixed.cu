@@ -45,7 +45,75 @@ struct KSum {
   __device__ __forceinline__ double value() const { return (double)s - (double)c; }
 };
 
+// Packed two-element FP32 arithmetic (add/sub/mul/fma .f32x2): one issue slot
+// for two IEEE operations, each rounded as the scalar instruction rounds it.
+// The gathers are bound by instruction issue and load latency (the L1 data
+// pipe is half idle in brick order), and about two thirds of a pair's
+// instructions are FP32 arithmetic on independent components.
+__device__ __forceinline__ unsigned long long f2_bits(float2 a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+  return r;
+}
+__device__ __forceinline__ float2 f2_of(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return f2_of(r);
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return f2_of(r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return f2_of(r);
+}
+
+// Two Kahan sums side by side: the operations of KSum::add on each half.
+struct KSum2 {
+  float2 s = {0.f, 0.f}, c = {0.f, 0.f};
+  __device__ __forceinline__ void add(float2 x) {
+    float2 y = sub2(x, c);
+    float2 t = add2(s, y);
+    c = sub2(sub2(t, s), y);
+    s = t;
+  }
+  __device__ __forceinline__ double value0() const { return (double)s.x - (double)c.x; }
+  __device__ __forceinline__ double value1() const { return (double)s.y - (double)c.y; }
+};
+
 __device__ __forceinline__ float4 ld4(const float4* p) { return __ldg(p); }
+
+// Position and velocity of one record as the three float-float pairs
+// (x, y), (z, vx), (vy, vz), and the difference of two of them:
+// (hi_i - hi_j) + (lo_i - lo_j) for all six components.
+struct PosVel {
+  float2 h0, h1, h2, l0, l1, l2;
+};
+__device__ __forceinline__ PosVel posvel(float4 xv, float4 lo, float4 vw) {
+  PosVel p;
+  p.h0 = make_float2(xv.x, xv.y); p.h1 = make_float2(xv.z, xv.w); p.h2 = make_float2(vw.x, vw.y);
+  p.l0 = make_float2(bf16_first(lo.x), bf16_second(lo.x));
+  p.l1 = make_float2(bf16_first(lo.y), bf16_second(lo.y));
+  p.l2 = make_float2(bf16_first(lo.z), bf16_second(lo.z));
+  return p;
+}
+struct PairDiff {
+  float x0, x1, x2, v0, v1, v2;
+};
+__device__ __forceinline__ PairDiff pair_diff(const PosVel& a, const PosVel& b) {
+  const float2 d0 = add2(sub2(a.h0, b.h0), sub2(a.l0, b.l0));
+  const float2 d1 = add2(sub2(a.h1, b.h1), sub2(a.l1, b.l1));
+  const float2 d2 = add2(sub2(a.h2, b.h2), sub2(a.l2, b.l2));
+  return PairDiff{d0.x, d0.y, d1.x, d1.y, d2.x, d2.y};
+}
 
 // One thread per particle: block b handles particles [b*B, (b+1)*B).
 template <class Body>
@@ -54,39 +122,69 @@ __device__ __forceinline__ void run_rows(const DomainConst& K, Body body) {
   if (i < K.N) body(i);
 }
 
-// Cubic-spline gradient factor GK (Functions.cpp:74-87, 3D) from r^2 and the
-// pair smoothing length hh = (hi + hj) / 2.
-__device__ __forceinline__ float grad_kernel_f(float r2, float hh, float* r_out) {
-  float rinv = rsqrtf(r2);
-  float r = r2 * rinv;
-  float inv_h = 1.0f / hh;
-  float q = r * inv_h;
-  float ih2 = inv_h * inv_h;
-  float C = INV_PI_F * ih2 * ih2 * inv_h;
-  float w;
-  if (q < 1.0f) w = -3.0f + 2.25f * q;
-  else if (q < 2.0f) { float t = 2.0f - q; w = -0.75f * t * t * (hh * rinv); }
-  else w = 0.0f;
-  if (r2 == 0.0f) { w = -3.0f; r = 0.0f; }
-  *r_out = r;
-  return C * w;
+// Row entries k0, k0 + dk, ... of one particle, in order: key(k) is the entry,
+// load(key) its neighbour's record groups, body(key, record) the pair's terms.
+// The gathers wait for their loads (long-scoreboard stalls take more than half
+// of a warp's cycles): the rows stream from HBM and the records come from L1
+// or L2.  So the entries are loaded one turn ahead, and the records of two
+// entries before the first one's terms, at 64 (density) and 80 registers
+// (acceleration, rates): fewer resident warps with twice the loads in flight.
+// Mixed step at 982,072 particles: 1.224 ms with neither, 1.164 with the
+// entries ahead alone; with the packed arithmetic 1.069 with one record and
+// 0.972 with two (at 64, 72 and 96 registers the rate-stress kernel took 499,
+// 473 and 514 us against 425 at 80; the acceleration 291, 288 and 333 us
+// against 255).
+template <class Key, class Load, class Body>
+__device__ __forceinline__ void walk_row(int k0, int dk, int len, Key key, Load load, Body body) {
+  int n0 = k0 < len ? key(k0) : 0, n1 = k0 + dk < len ? key(k0 + dk) : 0;
+  int k = k0;
+  for (; k + dk < len; k += 2 * dk) {
+    const int e0 = n0, e1 = n1;
+    const auto r0 = load(e0);
+    const auto r1 = load(e1);
+    if (k + 2 * dk < len) n0 = key(k + 2 * dk);
+    if (k + 3 * dk < len) n1 = key(k + 3 * dk);
+    body(e0, r0);
+    body(e1, r1);
+  }
+  if (k < len) body(n0, load(n0));
 }
 
-// The same factor for a pair smoothing length hh = h that is uniform over the
-// domain: 1/h and C come precomputed (the same FP32 operations on the host).
+// 1/sqrt of a pair's r^2: the FP32 approximation without the scaling that
+// rsqrtf adds for denormal arguments.  r^2 below the smallest normal FP32 is
+// taken as coincident particles by the caller.
+__device__ __forceinline__ float rsqrt_normal(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Cubic-spline gradient factor GK (Functions.cpp:74-87, 3D) from r^2 and the
+// pair smoothing length hh = (hi + hj) / 2.  UNI: hh = h is uniform over the
+// domain, 1/h and C come precomputed (the same FP32 operations on the host).
+// Selects instead of branches: a warp's pairs fall on both sides of q = 1.
 template <bool UNI>
 __device__ __forceinline__ float grad_kernel(const DomainConst& K, float r2, float hh, float* r_out) {
-  if (!UNI) return grad_kernel_f(r2, hh, r_out);
-  float rinv = rsqrtf(r2);
+  float inv_h, C, h;
+  if (UNI) { inv_h = K.inv_h_f; C = K.gk_c_f; h = K.h_f; }
+  else {
+    inv_h = 1.0f / hh;
+    float ih2 = inv_h * inv_h;
+    C = INV_PI_F * ih2 * ih2 * inv_h;
+    h = hh;
+  }
+  const float rinv = rsqrt_normal(r2);
   float r = r2 * rinv;
-  float q = r * K.inv_h_f;
-  float w;
-  if (q < 1.0f) w = -3.0f + 2.25f * q;
-  else if (q < 2.0f) { float t = 2.0f - q; w = -0.75f * t * t * (K.h_f * rinv); }
-  else w = 0.0f;
-  if (r2 == 0.0f) { w = -3.0f; r = 0.0f; }
+  const float q = r * inv_h;
+  const float near = -3.0f + 2.25f * q, t = 2.0f - q;
+  const float far = -0.75f * t * t * (h * rinv);
+  float w = q < 2.0f ? far : 0.0f;
+  w = q < 1.0f ? near : w;
+  const bool same = r2 < 1.17549435e-38f;
+  w = same ? -3.0f : w;
+  r = same ? 0.0f : r;
   *r_out = r;
-  return K.gk_c_f * w;
+  return C * w;
 }
 
 // Kernel-gradient correction of the locking sums (gradKernelCorr): the
@@ -124,12 +222,12 @@ __global__ void k_refresh_records(DevPtrs P, DomainConst K, int force) {
   }
   ff_split(col(P, C_T, N, i), th, tl);
   float4* r = P.rc + i;
-  // uniform-particle layout: Sigma/rho^2 xz, yz in the .w slots of the x and v groups
-  float w_x = K.uni ? (float)(c2 * col(P, C_SIG + 4, N, i)) : (float)col(P, C_H, N, i);
-  float w_v = K.uni ? (float)(c2 * col(P, C_SIG + 5, N, i)) : (float)rho;
-  r[(size_t)RC_XH * N] = make_float4(xh[0], xh[1], xh[2], w_x);
+  // uniform-particle layout: Sigma/rho^2 xz, yz in the last two fields of RC_VW
+  float w_2 = K.uni ? (float)(c2 * col(P, C_SIG + 4, N, i)) : (float)col(P, C_H, N, i);
+  float w_3 = K.uni ? (float)(c2 * col(P, C_SIG + 5, N, i)) : (float)rho;
+  r[(size_t)RC_XV * N] = make_float4(xh[0], xh[1], xh[2], vh[0]);
   r[(size_t)RC_L * N] = lo_pack(xl, vl, solid ? (float)(col(P, C_MASS, N, i) / rho) : 0.f);
-  r[(size_t)RC_VH * N] = make_float4(vh[0], vh[1], vh[2], w_v);
+  r[(size_t)RC_VW * N] = make_float4(vh[1], vh[2], w_2, w_3);
   r[(size_t)RC_S0 * N] = make_float4((float)(c2 * col(P, C_SIG, N, i)), (float)(c2 * col(P, C_SIG + 1, N, i)),
                          (float)(c2 * col(P, C_SIG + 2, N, i)), (float)(c2 * col(P, C_SIG + 3, N, i)));
   r[(size_t)RC_S1 * N] = make_float4((float)(c2 * col(P, C_SIG + 4, N, i)), (float)(c2 * col(P, C_SIG + 5, N, i)),
@@ -149,18 +247,24 @@ __global__ void k_refresh_records(DevPtrs P, DomainConst K, int force) {
 // points at, so a gather can load entry k + dk's key before it consumes
 // entry k's records: the index load then overlaps the record loads instead of
 // adding a second memory latency to every iteration.
+struct AccelRec {
+  float4 xv, lo, vw, s0, s1;
+  int j;  // the neighbour's index (-1 where it is not known)
+};
 struct GlobalFetch {
   const float4* rc;
   const int* nb;  // P.nbr + i
   size_t N;
   __device__ __forceinline__ int key(int k) const { return nb_index(nb[(size_t)k * N]); }
-  template <bool UNI = false>
-  __device__ __forceinline__ int get(int j, float4& xh, float4& lo, float4& vh, float4& s0, float4& s1) const {
+  template <bool UNI>
+  __device__ __forceinline__ AccelRec get(int j) const {
     const float4* rj = rc + j;
-    xh = ld4(rj + (size_t)RC_XH * N); lo = ld4(rj + (size_t)RC_L * N); vh = ld4(rj + (size_t)RC_VH * N);
-    s0 = ld4(rj + (size_t)RC_S0 * N);
-    if (!UNI) s1 = ld4(rj + (size_t)RC_S1 * N);  // uniform layout: xz, yz ride in xh.w, vh.w
-    return j;
+    AccelRec r;
+    r.xv = ld4(rj + (size_t)RC_XV * N); r.lo = ld4(rj + (size_t)RC_L * N); r.vw = ld4(rj + (size_t)RC_VW * N);
+    r.s0 = ld4(rj + (size_t)RC_S0 * N);
+    if (!UNI) r.s1 = ld4(rj + (size_t)RC_S1 * N);  // uniform layout: xz, yz ride in vw.z, vw.w
+    r.j = j;
+    return r;
   }
 };
 struct StagedFetch {
@@ -169,50 +273,57 @@ struct StagedFetch {
   size_t N;
   int cap;
   __device__ __forceinline__ int key(int k) const { return slot[(size_t)k * N]; }
-  template <bool UNI = false>
-  __device__ __forceinline__ int get(int q, float4& xh, float4& lo, float4& vh, float4& s0, float4& s1) const {
-    xh = sh[q]; lo = sh[cap + q]; vh = sh[2 * cap + q]; s0 = sh[3 * cap + q]; s1 = sh[4 * cap + q];
-    return -1;  // the global index is not known here: no misc or TI group (AVU and !TI only)
+  template <bool UNI>
+  __device__ __forceinline__ AccelRec get(int q) const {
+    // the global index is not known here: no misc or TI group (AVU and !TI only)
+    return AccelRec{sh[q], sh[cap + q], sh[2 * cap + q], sh[3 * cap + q], sh[4 * cap + q], -1};
   }
 };
 
 // Pair sums of the acceleration of SPH particle i over row entries k0, k0 + dk, ...
 // UNI: the uniform-particle layout (DomainConst::uni): h and Cs are the
-// domain's constants, m_j = m_i, Sigma/rho^2 xz and yz come from the .w slots
-// of the x and v groups, and rho_j = m_i / (m/rho)_j.
+// domain's constants, m_j = m_i (a factor of the whole sum, applied by
+// accel_mx_value), Sigma/rho^2 xz and yz come from the last two fields of the
+// second velocity group, and rho_j = m_i / (m/rho)_j.
+struct AccelSum {
+  KSum2 a01;
+  KSum a2;
+};
+template <bool UNI>
+__device__ __forceinline__ void accel_mx_value(const DevPtrs& P, const DomainConst& K, int i, const AccelSum& a,
+                                               double v[3]) {
+  const double m = UNI ? col(P, C_MASS, (size_t)K.N, i) : 1.0;
+  v[0] = m * a.a01.value0(); v[1] = m * a.a01.value1(); v[2] = m * a.a2.value();
+}
 template <bool TI, bool AVU, bool GC, bool UNI, class Fetch>
 __device__ __forceinline__ void accel_mx_sums(const DevPtrs& P, const DomainConst& K, int i, const Fetch& F, int k0,
-                                              int dk, KSum& a0, KSum& a1, KSum& a2) {
+                                              int dk, AccelSum& a) {
   size_t N = K.N;
   const float4* ri = P.rc + i;
-  float4 xh = ld4(ri + (size_t)RC_XH * N), lo = ld4(ri + (size_t)RC_L * N), vh = ld4(ri + (size_t)RC_VH * N);
-  float xl[3], vl[3];
-  lo_unpack(lo, xl, vl);
-  float4 s0 = ld4(ri + (size_t)RC_S0 * N), s1;
+  const float4 vw = ld4(ri + (size_t)RC_VW * N);
+  const PosVel pi = posvel(ld4(ri + (size_t)RC_XV * N), ld4(ri + (size_t)RC_L * N), vw);
+  const float4 s0 = ld4(ri + (size_t)RC_S0 * N);
+  float4 s1;
   const float mass_i = UNI ? (float)col(P, C_MASS, N, i) : 0.f;
-  if (UNI) s1 = make_float4(xh.w, vh.w, mass_i, K.cs_f);
+  if (UNI) s1 = make_float4(vw.z, vw.w, mass_i, K.cs_f);
   else s1 = ld4(ri + (size_t)RC_S1 * N);
-  const float hi_ = UNI ? K.h_f : xh.w;
-  const float rhoi = UNI ? (float)col(P, C_RHO, N, i) : vh.w;
+  const float hi_ = UNI ? K.h_f : vw.z;
+  const float rhoi = UNI ? (float)col(P, C_RHO, N, i) : vw.w;
   float4 mi = AVU ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4(ri + (size_t)RC_MISC * N);
   float4 t0 = make_float4(0.f, 0.f, 0.f, 0.f), t1 = t0;
   if (TI) { t0 = ld4(ri + (size_t)RC_TI0 * N); t1 = ld4(ri + (size_t)RC_TI1 * N); }
   CorrM cm;
   if (GC) cm = load_corr(P, N, i);
   int len = P.row_len[i];
-  int next = k0 < len ? F.key(k0) : 0;
-  for (int k = k0; k < len; k += dk) {
-    float4 jxh, jlo, jvh, js0, js1;
-    int j = F.template get<UNI>(next, jxh, jlo, jvh, js0, js1);
-    if (k + dk < len) next = F.key(k + dk);
-    if (UNI) js1 = make_float4(jxh.w, jvh.w, mass_i, K.cs_f);
-    const float4* rj = P.rc + j;
-    float jxl[3], jvl[3];
-    lo_unpack(jlo, jxl, jvl);
-    float x0 = (xh.x - jxh.x) + (xl[0] - jxl[0]), x1 = (xh.y - jxh.y) + (xl[1] - jxl[1]), x2 = (xh.z - jxh.z) + (xl[2] - jxl[2]);
-    float v0 = (vh.x - jvh.x) + (vl[0] - jvl[0]), v1 = (vh.y - jvh.y) + (vl[1] - jvl[1]), v2 = (vh.z - jvh.z) + (vl[2] - jvl[2]);
-    float hh = UNI ? hi_ : 0.5f * (hi_ + jxh.w);
-    float r2 = x0 * x0 + x1 * x1 + x2 * x2, r;
+  auto key = [&](int k) { return F.key(k); };
+  auto load = [&](int e) { return F.template get<UNI>(e); };
+  walk_row(k0, dk, len, key, load, [&](int, const AccelRec& q) {
+    const float4 jlo = q.lo, jvw = q.vw, js0 = q.s0;
+    const float4 js1 = UNI ? make_float4(jvw.z, jvw.w, mass_i, K.cs_f) : q.s1;
+    const float4* rj = P.rc + q.j;
+    const PairDiff d = pair_diff(pi, posvel(q.xv, jlo, jvw));
+    float hh = UNI ? hi_ : 0.5f * (hi_ + jvw.z);
+    float r2 = d.x0 * d.x0 + d.x1 * d.x1 + d.x2 * d.x2, r;
     float GK = grad_kernel<UNI>(K, r2, hh, &r);
     float Alpha, Beta;
     if (AVU) {
@@ -223,26 +334,30 @@ __device__ __forceinline__ void accel_mx_sums(const DevPtrs& P, const DomainCons
     }
     float PIs = 0.f;
     if (Alpha != 0.f || Beta != 0.f) {
-      float dvx = v0 * x0 + v1 * x1 + v2 * x2;
-      if (dvx < 0.f) {  // Monaghan viscosity (InteractionAlt.cpp:74-94)
-        float MU = hh * dvx / (r * r + 0.01f * hh * hh);
-        float Cij = 0.5f * (s1.w + js1.w);
-        if (UNI)  // 1 / (0.5 (rho_i + rho_j)) with rho_j = m_i / (m/rho)_j
-          PIs = (Alpha * Cij * MU + Beta * MU * MU) * (2.f * jlo.w) / (rhoi * jlo.w + mass_i);
-        else
-          PIs = (Alpha * Cij * MU + Beta * MU * MU) / (0.5f * (rhoi + jvh.w));
+      float dvx = d.v0 * d.x0 + d.v1 * d.x1 + d.v2 * d.x2;
+      if (dvx < 0.f) {  // Monaghan viscosity (InteractionAlt.cpp:74-94): MU (alpha C + beta MU) / rho_bar
+        const float hv = hh * dvx, Dn = r2 + 0.01f * hh * hh;
+        const float Cij = 0.5f * (s1.w + js1.w);
+        float p;  // MU / rho_bar, one division; in UNI 1 / rho_bar = 2 V_j / (rho_i V_j + m_i) with V_j = m_i / rho_j
+        if (UNI) p = hv * (2.f * jlo.w) / (Dn * (rhoi * jlo.w + mass_i));
+        else p = hv / (Dn * (0.5f * (rhoi + jvw.w)));
+        PIs = Alpha * Cij * p;
+        if (Beta != 0.f) PIs += Beta * p * (hv / Dn);
       }
     }
-    float S0 = s0.x + js0.x + PIs, S1 = s0.y + js0.y + PIs, S2 = s0.z + js0.z + PIs;
-    float S3 = s0.w + js0.w, S4 = s1.x + js1.x, S5 = s1.y + js1.y;
+    const float2 S01 = add2(make_float2(s0.x, s0.y), make_float2(js0.x, js0.y));
+    const float2 S23 = add2(make_float2(s0.z, s0.w), make_float2(js0.z, js0.w));
+    const float2 S45 = add2(make_float2(s1.x, s1.y), make_float2(js1.x, js1.y));
+    float S0 = S01.x + PIs, S1 = S01.y + PIs, S2 = S23.x + PIs, S3 = S23.y, S4 = S45.x, S5 = S45.y;
     if (TI) {  // tensile instability (InteractionAlt.cpp:102-109)
       // The reference adds the term when either end has TI > 0; TIR is zero
       // where TI is, so adding it for every pair with a finite factor (w0 > 0,
       // TIInitDist within the support) gives the same sums without reading
       // TI_j.
       float4 jt0 = ld4(rj + (size_t)RC_TI0 * N), jt1 = ld4(rj + (size_t)RC_TI1 * N);
-      float q = r / hh, q0 = (t1.w + jt1.w) / (2.f * hh);
-      float wq = q < 1.f ? 1.f - 1.5f * q * q + 0.75f * q * q * q : (q < 2.f ? 0.25f * (2.f - q) * (2.f - q) * (2.f - q) : 0.f);
+      float qr = r / hh, q0 = (t1.w + jt1.w) / (2.f * hh);
+      float wq = qr < 1.f ? 1.f - 1.5f * qr * qr + 0.75f * qr * qr * qr
+                          : (qr < 2.f ? 0.25f * (2.f - qr) * (2.f - qr) * (2.f - qr) : 0.f);
       float w0 = q0 < 1.f ? 1.f - 1.5f * q0 * q0 + 0.75f * q0 * q0 * q0
                           : (q0 < 2.f ? 0.25f * (2.f - q0) * (2.f - q0) * (2.f - q0) : 0.f);
       if (w0 > 0.f) {
@@ -254,13 +369,12 @@ __device__ __forceinline__ void accel_mx_sums(const DevPtrs& P, const DomainCons
         S3 += f * (t0.w + jt0.w); S4 += f * (t1.x + jt1.x); S5 += f * (t1.y + jt1.y);
       }
     }
-    float g0 = GK * x0, g1 = GK * x1, g2 = GK * x2;
-    if (GC) corr_gk(cm, GK, x0, x1, x2, g0, g1, g2);
-    float mj = js1.z;
-    a0.add(mj * (g0 * S0 + g1 * S3 + g2 * S4));
-    a1.add(mj * (g0 * S3 + g1 * S1 + g2 * S5));
-    a2.add(mj * (g0 * S4 + g1 * S5 + g2 * S2));
-  }
+    float g0 = GK * d.x0, g1 = GK * d.x1, g2 = GK * d.x2;
+    if (GC) corr_gk(cm, GK, d.x0, d.x1, d.x2, g0, g1, g2);
+    if (!UNI) { const float mj = js1.z; g0 *= mj; g1 *= mj; g2 *= mj; }
+    a.a01.add(make_float2(g0 * S0 + g1 * S3 + g2 * S4, g0 * S3 + g1 * S1 + g2 * S5));
+    a.a2.add(g0 * S4 + g1 * S5 + g2 * S2);
+  });
 }
 template <bool TI, bool AVU, bool GC, bool UNI, class Fetch>
 __device__ __forceinline__ void accel_mx(const DevPtrs& P, const DomainConst& K, int i, const Fetch& F) {
@@ -269,12 +383,14 @@ __device__ __forceinline__ void accel_mx(const DevPtrs& P, const DomainConst& K,
     colw(P, C_A, N, i) = 0.0; colw(P, C_A + 1, N, i) = 0.0; colw(P, C_A + 2, N, i) = 0.0;
     return;
   }
-  KSum a0, a1, a2;
-  accel_mx_sums<TI, AVU, GC, UNI>(P, K, i, F, 0, 1, a0, a1, a2);
-  colw(P, C_A, N, i) = a0.value(); colw(P, C_A + 1, N, i) = a1.value(); colw(P, C_A + 2, N, i) = a2.value();
+  AccelSum a;
+  accel_mx_sums<TI, AVU, GC, UNI>(P, K, i, F, 0, 1, a);
+  double v[3];
+  accel_mx_value<UNI>(P, K, i, a, v);
+  for (int d = 0; d < 3; ++d) colw(P, C_A + d, N, i) = v[d];
 }
 template <bool TI, bool AVU, bool GC, bool UNI>
-__global__ void __launch_bounds__(512) k_accel_mx(DevPtrs P, DomainConst K) {
+__global__ void __maxnreg__(80) k_accel_mx(DevPtrs P, DomainConst K) {
   run_rows(K, [&](int i) { accel_mx<TI, AVU, GC, UNI>(P, K, i, GlobalFetch{P.rc, P.nbr + i, (size_t)K.N}); });
 }
 
@@ -291,9 +407,13 @@ __global__ void __launch_bounds__(512) k_accel_mx_lanes(DevPtrs P, DomainConst K
   const size_t N = K.N;
   const bool live = i < K.N;
   const bool sph = live && icol(P, I_KIND, N, i) == 0;
-  KSum a0, a1, a2;
-  if (sph) accel_mx_sums<TI, AVU, GC, UNI>(P, K, i, GlobalFetch{P.rc, P.nbr + i, N}, sub, L, a0, a1, a2);
-  double v0 = a0.value(), v1 = a1.value(), v2 = a2.value();
+  AccelSum a;
+  double v[3] = {0.0, 0.0, 0.0};
+  if (sph) {
+    accel_mx_sums<TI, AVU, GC, UNI>(P, K, i, GlobalFetch{P.rc, P.nbr + i, N}, sub, L, a);
+    accel_mx_value<UNI>(P, K, i, a, v);
+  }
+  double v0 = v[0], v1 = v[1], v2 = v[2];
   for (int off = 1; off < L; off <<= 1) {  // the whole warp takes part; L divides 32
     v0 += __shfl_xor_sync(0xffffffffu, v0, off);
     v1 += __shfl_xor_sync(0xffffffffu, v1, off);
@@ -325,9 +445,9 @@ __global__ void __launch_bounds__(2 * STAGE_B) k_accel_mx_staged(DevPtrs P, Doma
     const int* hl = P.halo + (size_t)b * cap;
     for (int s = t; s < H; s += 2 * STAGE_B) {
       const float4* rj = P.rc + hl[s];
-      sh_rec[s] = ld4(rj + (size_t)RC_XH * N);
+      sh_rec[s] = ld4(rj + (size_t)RC_XV * N);
       sh_rec[cap + s] = ld4(rj + (size_t)RC_L * N);
-      sh_rec[2 * cap + s] = ld4(rj + (size_t)RC_VH * N);
+      sh_rec[2 * cap + s] = ld4(rj + (size_t)RC_VW * N);
       sh_rec[3 * cap + s] = ld4(rj + (size_t)RC_S0 * N);
       sh_rec[4 * cap + s] = ld4(rj + (size_t)RC_S1 * N);
     }
@@ -336,12 +456,12 @@ __global__ void __launch_bounds__(2 * STAGE_B) k_accel_mx_staged(DevPtrs P, Doma
   const int p = t % STAGE_B, part = t / STAGE_B;
   const int i = b * STAGE_B + p;
   const bool sph = i < K.N && icol(P, I_KIND, N, i) == 0;
-  KSum a0, a1, a2;
+  AccelSum a;
   if (sph) {
-    if (H >= 0) accel_mx_sums<false, true, false, false>(P, K, i, StagedFetch{sh_rec, P.nslot + i, N, cap}, part, 2, a0, a1, a2);
-    else accel_mx_sums<false, true, false, false>(P, K, i, GlobalFetch{P.rc, P.nbr + i, N}, part, 2, a0, a1, a2);
+    if (H >= 0) accel_mx_sums<false, true, false, false>(P, K, i, StagedFetch{sh_rec, P.nslot + i, N, cap}, part, 2, a);
+    else accel_mx_sums<false, true, false, false>(P, K, i, GlobalFetch{P.rc, P.nbr + i, N}, part, 2, a);
   }
-  double v0 = a0.value(), v1 = a1.value(), v2 = a2.value();
+  double v0 = a.a01.value0(), v1 = a.a01.value1(), v2 = a.a2.value();
   __syncthreads();  // halo records no longer read: the odd halves pass through shared memory
   double* ex = reinterpret_cast<double*>(sh_rec);  // 3 * STAGE_B doubles (stage_cap >= 64)
   if (part == 1) { ex[p] = v0; ex[STAGE_B + p] = v1; ex[2 * STAGE_B + p] = v2; }
@@ -452,6 +572,11 @@ int configure_staging(int cap) {
   return (int)cudaFuncSetAttribute(k_accel_mx_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// A neighbour's position and velocity groups (and, for conduction, its E group).
+struct MoveRec {
+  float4 xv, lo, vw, e;
+};
+
 // ---------------------------------------------------------------- density + drift + kick
 // GC: the locking sum with corrected gradients, m_j (rho_i / rho_j) v_ij . vc_i
 // (InteractionAlt.cpp:589-605), which carries rho_i inside the sum.
@@ -470,27 +595,26 @@ __device__ __forceinline__ void density_drift_mx(const DevPtrs& P, const DomainC
   double dd = 0.0;
   bool solid = live && icol(P, I_KIND, N, i) == 0;
   const float4* ri = P.rc + i;
-  float4 xh = live ? ld4(ri + (size_t)RC_XH * N) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 vw = live ? ld4(ri + (size_t)RC_VW * N) : make_float4(0.f, 0.f, 0.f, 0.f);
   if (solid) {
-    float4 lo = ld4(ri + (size_t)RC_L * N), vh = ld4(ri + (size_t)RC_VH * N);
-    float xl[3], vl[3];
-    lo_unpack(lo, xl, vl);
+    const PosVel pi = posvel(ld4(ri + (size_t)RC_XV * N), ld4(ri + (size_t)RC_L * N), vw);
     CorrM cm;
     if (GC) cm = load_corr(P, N, i);
     float rhoif = (float)rhoi;
     KSum s;
     int len = P.row_len[i];
     const int* nb = P.nbr + i;
-    for (int k = sub; k < len; k += L) {
-      int j = nb_index(nb[(size_t)k * N]);
+    auto key = [&](int k) { return nb_index(nb[(size_t)k * N]); };
+    auto load = [&](int j) {
       const float4* rj = P.rc + j;
-      float4 jxh = ld4(rj + (size_t)RC_XH * N), jlo = ld4(rj + (size_t)RC_L * N), jvh = ld4(rj + (size_t)RC_VH * N);
-      float jxl[3], jvl[3];
-      lo_unpack(jlo, jxl, jvl);
-      float x0 = (xh.x - jxh.x) + (xl[0] - jxl[0]), x1 = (xh.y - jxh.y) + (xl[1] - jxl[1]), x2 = (xh.z - jxh.z) + (xl[2] - jxl[2]);
-      float v0 = (vh.x - jvh.x) + (vl[0] - jvl[0]), v1 = (vh.y - jvh.y) + (vl[1] - jvl[1]), v2 = (vh.z - jvh.z) + (vl[2] - jvl[2]);
+      return MoveRec{ld4(rj + (size_t)RC_XV * N), ld4(rj + (size_t)RC_L * N), ld4(rj + (size_t)RC_VW * N)};
+    };
+    walk_row(sub, L, len, key, load, [&](int, const MoveRec& q) {
+      const float4 jlo = q.lo, jvw = q.vw;
+      const PairDiff d = pair_diff(pi, posvel(q.xv, jlo, jvw));
+      const float x0 = d.x0, x1 = d.x1, x2 = d.x2, v0 = d.v0, v1 = d.v1, v2 = d.v2;
       float r;
-      float GK = grad_kernel<UNI>(K, x0 * x0 + x1 * x1 + x2 * x2, UNI ? K.h_f : 0.5f * (xh.w + jxh.w), &r);
+      float GK = grad_kernel<UNI>(K, x0 * x0 + x1 * x1 + x2 * x2, UNI ? K.h_f : 0.5f * (vw.z + jvw.z), &r);
       if (GC) {
         float g0, g1, g2;
         corr_gk(cm, GK, x0, x1, x2, g0, g1, g2);
@@ -498,7 +622,7 @@ __device__ __forceinline__ void density_drift_mx(const DevPtrs& P, const DomainC
       } else {
         s.add(jlo.w * (GK * (v0 * x0 + v1 * x1 + v2 * x2)));  // (m_j / rho_j) v_ij . (GK x_ij)
       }
-    }
+    });
     dd = s.value();
   }
   if constexpr (L > 1)
@@ -537,14 +661,14 @@ __device__ __forceinline__ void density_drift_mx(const DevPtrs& P, const DomainC
   float th, tl;
   ff_split(Tn, th, tl);
   float4* r = P.rn + i;
-  r[(size_t)RN_XH * N] = make_float4(nxh[0], nxh[1], nxh[2], UNI ? K.h_f : xh.w);
+  r[(size_t)RN_XV * N] = make_float4(nxh[0], nxh[1], nxh[2], nvh[0]);
   r[(size_t)RN_L * N] = lo_pack(nxl, nvl, (float)mrn);
   float pr2 = solid ? (float)(pn * irn * irn) : 0.f;
-  r[(size_t)RN_VH * N] = make_float4(nvh[0], nvh[1], nvh[2], pr2);  // the rate gather reads p/rho^2 here
+  r[(size_t)RN_VW * N] = make_float4(nvh[1], nvh[2], UNI ? K.h_f : vw.z, pr2);  // the rate gather reads p/rho^2 here
   r[(size_t)RN_E * N] = make_float4(pr2, ri[(size_t)RC_MISC * N].z, th, tl);
 }
 template <bool GC, bool UNI>
-__global__ void __launch_bounds__(512, 3) k_density_drift_mx(DevPtrs P, DomainConst K) {
+__global__ void __maxnreg__(64) k_density_drift_mx(DevPtrs P, DomainConst K) {
   run_rows(K, [&](int i) { density_drift_mx<GC, UNI, 1>(P, K, i, 0, true); });
 }
 template <bool GC, bool UNI, int L>
@@ -583,30 +707,35 @@ __device__ __forceinline__ void rate_mx(const DevPtrs& P, const DomainConst& K, 
   double md[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // L > 1: the lane's compensated values
   if (sph) {
     const float4* ri = P.rn + i;
-    float4 xh = ld4(ri + (size_t)RN_XH * N), lo = ld4(ri + (size_t)RN_L * N), vh = ld4(ri + (size_t)RN_VH * N);
-    float xl[3], vl[3];
-    lo_unpack(lo, xl, vl);
-    float4 e = THERMAL ? ld4(ri + (size_t)RN_E * N) : make_float4(vh.w, 0.f, 0.f, 0.f);
+    const float4 lo = ld4(ri + (size_t)RN_L * N), vw = ld4(ri + (size_t)RN_VW * N);
+    const PosVel pi = posvel(ld4(ri + (size_t)RN_XV * N), lo, vw);
+    float4 e = THERMAL ? ld4(ri + (size_t)RN_E * N) : make_float4(vw.w, 0.f, 0.f, 0.f);
     CorrM cm;
     if (GC) cm = load_corr(P, N, i);
-    KSum M[9];  // sum_j (m_j / rho_j) (-GK / 2) (v_i - v_j)_k (x_i - x_j)_l  (GC: gk_l for GK x_l)
-    KSum kin, cnd;
+    // sum_j (m_j / rho_j) (-GK / 2) (v_i - v_j)_k (x_i - x_j)_l  (GC: gk_l for
+    // GK x_l) and the kinetic-energy sum, two sums to a packed pair:
+    // (00, 01) (10, 11) (20, 21) (02, 12) (22, kinetic)
+    KSum2 M[5];
+    KSum cnd;
     const float mass_i = (float)col(P, C_MASS, N, i);
     int len = P.row_len[i];
     const int* nb = P.nbr + i;
-    for (int k = sub; k < len; k += L) {
-      int ent = nb[(size_t)k * N];
-      int j = nb_index(ent);
-      const float4* rj = P.rn + j;
-      float4 jxh = ld4(rj + (size_t)RN_XH * N), jlo = ld4(rj + (size_t)RN_L * N), jvh = ld4(rj + (size_t)RN_VH * N);
-      float jxl[3], jvl[3];
-      lo_unpack(jlo, jxl, jvl);
+    auto key = [&](int k) { return nb[(size_t)k * N]; };
+    auto load = [&](int ent) {
+      const float4* rj = P.rn + nb_index(ent);
+      MoveRec q{ld4(rj + (size_t)RN_XV * N), ld4(rj + (size_t)RN_L * N), ld4(rj + (size_t)RN_VW * N)};
+      if (THERMAL) q.e = ld4(rj + (size_t)RN_E * N);
+      return q;
+    };
+    walk_row(sub, L, len, key, load, [&](int ent, const MoveRec& q) {
+      const int j = nb_index(ent);
+      const float4 jlo = q.lo, jvw = q.vw;
       // p/rho^2 rides in the velocity group; conduction needs the E group (k_T, T)
-      float4 je = THERMAL ? ld4(rj + (size_t)RN_E * N) : make_float4(jvh.w, 0.f, 0.f, 0.f);
-      float x0 = (xh.x - jxh.x) + (xl[0] - jxl[0]), x1 = (xh.y - jxh.y) + (xl[1] - jxl[1]), x2 = (xh.z - jxh.z) + (xl[2] - jxl[2]);
-      float b0 = (vh.x - jvh.x) + (vl[0] - jvl[0]), b1 = (vh.y - jvh.y) + (vl[1] - jvl[1]), b2 = (vh.z - jvh.z) + (vl[2] - jvl[2]);
+      const float4 je = THERMAL ? q.e : make_float4(jvw.w, 0.f, 0.f, 0.f);
+      const PairDiff d = pair_diff(pi, posvel(q.xv, jlo, jvw));
+      const float x0 = d.x0, x1 = d.x1, x2 = d.x2, b0 = d.v0, b1 = d.v1, b2 = d.v2;
       float r;
-      float GK = grad_kernel<UNI>(K, x0 * x0 + x1 * x1 + x2 * x2, UNI ? K.h_f : 0.5f * (xh.w + jxh.w), &r);
+      float GK = grad_kernel<UNI>(K, x0 * x0 + x1 * x1 + x2 * x2, UNI ? K.h_f : 0.5f * (vw.z + jvw.z), &r);
       float y0 = x0, y1 = x1, y2 = x2;
       float w = jlo.w * (-0.5f * GK);
       if (GC) {  // -1/2 (float)(m_j/rho_j) (v_ij (x) gk), gk = M_i GK x_ij
@@ -614,15 +743,16 @@ __device__ __forceinline__ void rate_mx(const DevPtrs& P, const DomainConst& K, 
         w = jlo.w * -0.5f;
       }
       float wb0 = w * b0, wb1 = w * b1, wb2 = w * b2;
-      M[0].add(wb0 * y0); M[1].add(wb0 * y1); M[2].add(wb0 * y2);
-      M[3].add(wb1 * y0); M[4].add(wb1 * y1); M[5].add(wb1 * y2);
-      M[6].add(wb2 * y0); M[7].add(wb2 * y1); M[8].add(wb2 * y2);
       bool up = nb_up(ent);  // original index of j larger than i's
       float dv = GK * (b0 * x0 + b1 * x1 + b2 * x2);
       // m_P2 of the pair: m_i when the pairs' masses agree, else the column
       float mP2 = K.m_pair ? mass_i : (float)col(P, C_MASS, N, up ? j : i);
       float pk = 0.5f * mP2 * (e.x + je.x) * dv;
-      kin.add(up ? pk : -pk);
+      M[0].add(make_float2(wb0 * y0, wb0 * y1));
+      M[1].add(make_float2(wb1 * y0, wb1 * y1));
+      M[2].add(make_float2(wb2 * y0, wb2 * y1));
+      M[3].add(make_float2(wb0 * y2, wb1 * y2));
+      M[4].add(make_float2(wb2 * y2, up ? pk : -pk));
       if (THERMAL) {
         float wt = up ? jlo.w : lo.w;  // m_P2 / rho_P2 for both ends of the pair
         float dT = (e.z - je.z) + (e.w - je.w);
@@ -630,19 +760,22 @@ __device__ __forceinline__ void rate_mx(const DevPtrs& P, const DomainConst& K, 
         float gr = GC ? (x0 * y0 + x1 * y1 + x2 * y2) / (x0 * x0 + x1 * x1 + x2 * x2) : GK;
         cnd.add(wt * 4.f * (e.y * je.y) / (e.y + je.y) * dT * gr);
       }
-    }
+    });
     if constexpr (L == 1) {
       // The rate columns are FP32: each compensated sum is rounded to FP32 once
       // (s - c) and combined in FP32, which keeps the epilogue off the FP64 pipe.
-      float m[9];
-      for (int c = 0; c < 9; ++c) m[c] = M[c].s - M[c].c;
+      const float m[9] = {M[0].s.x - M[0].c.x, M[0].s.y - M[0].c.y, M[3].s.x - M[3].c.x,
+                          M[1].s.x - M[1].c.x, M[1].s.y - M[1].c.y, M[3].s.y - M[3].c.y,
+                          M[2].s.x - M[2].c.x, M[2].s.y - M[2].c.y, M[4].s.x - M[4].c.x};
       out[0] = 2.0f * m[0]; out[1] = 2.0f * m[4]; out[2] = 2.0f * m[8];
       out[3] = m[1] + m[3]; out[4] = m[2] + m[6]; out[5] = m[5] + m[7];
       out[6] = m[1] - m[3]; out[7] = m[2] - m[6]; out[8] = m[5] - m[7];
     } else {
-      for (int c = 0; c < 9; ++c) md[c] = M[c].value();
+      md[0] = M[0].value0(); md[1] = M[0].value1(); md[2] = M[3].value0();
+      md[3] = M[1].value0(); md[4] = M[1].value1(); md[5] = M[3].value1();
+      md[6] = M[2].value0(); md[7] = M[2].value1(); md[8] = M[4].value0();
     }
-    dkin = kin.value();
+    dkin = M[4].value1();
     cond = cnd.value();
   }
   if constexpr (L > 1) {
@@ -671,7 +804,7 @@ __device__ __forceinline__ void rate_mx(const DevPtrs& P, const DomainConst& K, 
   colw(P, C_DINT, N, i) = cond;  // conduction sum, consumed by k_stress_mx
 }
 template <bool THERMAL, bool GC, bool UNI>
-__global__ void __launch_bounds__(512) k_rate_mx(DevPtrs P, DomainConst K) {
+__global__ void __maxnreg__(80) k_rate_mx(DevPtrs P, DomainConst K) {
   run_rows(K, [&](int i) { rate_mx<THERMAL, GC, UNI, 1>(P, K, i, 0, true); });
 }
 template <bool THERMAL, bool GC, bool UNI, int L>
@@ -780,14 +913,14 @@ __device__ __forceinline__ void stress_mx(const DevPtrs& P, const DomainConst& K
     colw(P, C_MRHO, N, i) = col(P, C_MRHON, N, i);
     const float4* rn = P.rn + i;
     float4* rc = P.rc + i;
-    float4 nxh = rn[(size_t)RN_XH * N];
+    rc[(size_t)RC_XV * N] = rn[(size_t)RN_XV * N];
     rc[(size_t)RC_L * N] = rn[(size_t)RN_L * N];
-    float4 nvh = rn[(size_t)RN_VH * N];
+    float4 nvw = rn[(size_t)RN_VW * N];
     // the current groups carry h and rho (the acceleration gather's viscosity),
     // or in the uniform-particle layout Sigma/rho^2 xz and yz (written below
     // for SPH particles, 0 for the rest)
-    nxh.w = K.uni ? 0.f : nxh.w;
-    nvh.w = K.uni ? 0.f : (float)rho;
+    nvw.z = K.uni ? 0.f : nvw.z;
+    nvw.w = K.uni ? 0.f : (float)rho;
     float4 ne = rn[(size_t)RN_E * N];
     float4 misc = rc[(size_t)RC_MISC * N];
     maxpl = col(P, C_PLS, N, i);
@@ -870,15 +1003,14 @@ __device__ __forceinline__ void stress_mx(const DevPtrs& P, const DomainConst& K
       float c2 = 1.0f / ((float)rho * (float)rho);
       rc[(size_t)RC_S0 * N] = make_float4(c2 * (float)s.sig[0], c2 * (float)s.sig[1], c2 * (float)s.sig[2], c2 * (float)s.sig[3]);
       if (K.uni) {
-        nxh.w = c2 * (float)s.sig[4];
-        nvh.w = c2 * (float)s.sig[5];
+        nvw.z = c2 * (float)s.sig[4];
+        nvw.w = c2 * (float)s.sig[5];
       } else {
         float4 s1o = rc[(size_t)RC_S1 * N];  // mass and Cs carried over
         rc[(size_t)RC_S1 * N] = make_float4(c2 * (float)s.sig[4], c2 * (float)s.sig[5], s1o.z, s1o.w);
       }
     }
-    rc[(size_t)RC_XH * N] = nxh;
-    rc[(size_t)RC_VH * N] = nvh;
+    rc[(size_t)RC_VW * N] = nvw;
     rc[(size_t)RC_MISC * N] = make_float4(misc.x, misc.y, misc.z, ne.z);
     rc[(size_t)RC_T2 * N] = make_float4(ne.w, 0.f, 0.f, 0.f);
   }
@@ -898,17 +1030,16 @@ __global__ void __launch_bounds__(BLOCK, 3) k_stress_mx(DevPtrs P, DomainConst K
 }
 // Rate gather and stress update in one launch (one thread per particle, the
 // per-particle kernels' block size so the partial sums keep their layout):
-// the nine rates stay in registers instead of a store and a reload.  Four
-// blocks per SM cap it at the rate gather's own 64 registers (the update's
-// FP64 state spills ~150 B to L1 once per particle): at 982,072 particles the
-// step takes 1.267 against 1.313 ms with the two kernels; capped at 80
-// registers (three blocks) the lost occupancy made it 3 % slower instead.  Within
+// the nine rates stay in registers instead of a store and a reload, and one
+// warp's stress update (FP64 pipe) runs beside another's gather.  Three blocks
+// per SM leave it the 80 registers that two records in flight need (425 us at
+// 982,072 particles; 499 us at four blocks, where the records spill).  Within
 // the launch the gather reads only the next-step records, the rows and the
 // mass column, none of which the update writes, so the fusion has no
 // ordering hazard, and the results are bit-identical to k_rate_mx followed
 // by k_stress_mx.
 template <bool THERMAL, bool GC, bool UNI, bool HEAT>
-__global__ void __launch_bounds__(BLOCK, 4) k_rate_stress_mx(DevPtrs P, DomainConst K) {
+__global__ void __launch_bounds__(BLOCK, 3) k_rate_stress_mx(DevPtrs P, DomainConst K) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   RateOut ro;
   if (i < K.N) rate_mx<THERMAL, GC, UNI, 1, true>(P, K, i, 0, true, &ro);
