@@ -106,6 +106,9 @@ struct MaterialDev {
   double E;
   double K, m, eps0, eps1, sy0;                         // Hollomon
   double A, B, C, n, jm, eps_0, T_m, T_t;               // Johnson-Cook
+  // the mixed form's constants: FP32 roundings and 1 / (T_m - T_t), formed once on the host
+  float K_f, m_f, A_f, B_f, C_f, n_f, jm_f, eps_0_f;
+  double inv_Tmt;
 };
 struct BCDev {
   int zone, value_type, amp_id;
@@ -236,6 +239,7 @@ struct SpecState {
 struct DomainConst {
   int N, Nsolid, nbc_particles;
   double Cellfac, hmax, dt;
+  double inv_dt;       // 1 / dt (the fixed time step)
   double BLPF[3], CellSize[3];
   int CellNo[3];
   double rec_origin[3];  // the mixed form's position records hold x - rec_origin (the cell grid's centre)

@@ -691,7 +691,12 @@ struct wf_domain {
     DomainTables ht;
     memset(&ht, 0, sizeof(ht));
     ht.nmat = (int)mats.size();
-    for (size_t m = 0; m < mats.size(); ++m) ht.mat[m] = mats[m].dev;
+    for (size_t m = 0; m < mats.size(); ++m) {
+      MaterialDev& q = ht.mat[m] = mats[m].dev;
+      q.K_f = (float)q.K; q.m_f = (float)q.m; q.A_f = (float)q.A; q.B_f = (float)q.B; q.C_f = (float)q.C;
+      q.n_f = (float)q.n; q.jm_f = (float)q.jm; q.eps_0_f = (float)q.eps_0;
+      q.inv_Tmt = 1.0 / (q.T_m - q.T_t);
+    }
     ht.nbc = (int)bcs.size();
     for (size_t b = 0; b < bcs.size(); ++b) {
       BCDev& B = ht.bc[b];
@@ -777,7 +782,7 @@ struct wf_domain {
     CK(cudaMemcpyAsync(dnm, hnm.data(), sizeof(int) * hnm.size(), cudaMemcpyHostToDevice, stream));
     // Constants.
     K.N = N; K.Nsolid = solid_part_count; K.nbc_particles = (int)bl.size();
-    K.Cellfac = Cellfac; K.hmax = hmax; K.dt = dt;
+    K.Cellfac = Cellfac; K.hmax = hmax; K.dt = dt; K.inv_dt = 1.0 / dt;
     for (int d = 0; d < 3; ++d) { K.BLPF[d] = BLPF[d]; K.CellSize[d] = cs[d]; K.CellNo[d] = CellNo[d]; }
     // origin of the mixed form's position records: the cell grid's centre
     for (int d = 0; d < 3; ++d) K.rec_origin[d] = BLPF[d] + 0.5 * CellNo[d] * cs[d];

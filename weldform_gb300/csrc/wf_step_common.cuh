@@ -35,8 +35,120 @@ __device__ __forceinline__ double block_reduce(double v, double* sh) {
   return v;
 }
 
+// Largest (MIN: smallest) value of a warp in every lane, NaN left out as fmax
+// and fmin leave it out, by two 32-bit integer reductions of an order-keeping
+// key instead of five FP64 maxima (an FP64 instruction takes 16 cycles of an SM).
+template <bool MIN>
+__device__ __forceinline__ double warp_extreme(double v) {
+  unsigned long long k = (unsigned long long)__double_as_longlong(v);
+  const bool nan = (k & 0x7fffffffffffffffull) > 0x7ff0000000000000ull;
+  k = (k >> 63) ? ~k : k | 0x8000000000000000ull;  // ascending as unsigned
+  if (MIN) k = ~k;
+  if (nan) k = 0;  // unkeyed again a NaN, when every lane holds one
+  const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(k >> 32));
+  const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(k >> 32) == hi ? (unsigned)k : 0u);
+  k = ((unsigned long long)hi << 32) | lo;
+  if (MIN) k = ~k;
+  k = (k >> 63) ? k & 0x7fffffffffffffffull : ~k;
+  return __longlong_as_double((long long)k);
+}
+
+// Block reduction of NS sums and of an optional largest and smallest value with
+// one barrier.  The sums share a warp's halves: two of them take the first
+// addition in one instruction (lanes below 16 keep the first, the others the
+// second), four of them the second one in one, so two to four sums cost six
+// FP64 additions instead of five each; every sum's additions are those of
+// block_reduce's tree in the same order.  Warps are added in their order.
+// Sum q goes to out[q], then the largest and the smallest value (thread q
+// writes out[q]).  sh: 6 * 32 doubles, free when it is called.
+template <int NS, bool MAXMIN>
+__device__ __forceinline__ void block_reduce_all(const double (&s)[NS], double mx0, double mx1, double mn, double* sh,
+                                                 double* const* out) {
+  static_assert(NS >= 2 && NS <= 4, "two to four sums");
+  constexpr int NV = NS + 1 + (MAXMIN ? 2 : 0);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const bool up = l & 16, up8 = l & 8;
+  auto fold = [](bool u, int off, double a, double b) {  // a's sum in the lower lanes of the pair, b's in the upper
+    const double keep = u ? b : a, give = u ? a : b;
+    return keep + __shfl_xor_sync(0xffffffffu, give, off);
+  };
+  double v = fold(up, 16, s[0], s[1]);
+  if (NS > 2) {
+    const double t = NS == 4 ? fold(up, 16, s[2], s[NS - 1]) : s[NS > 2 ? 2 : 0] + __shfl_xor_sync(0xffffffffu, s[NS > 2 ? 2 : 0], 16);
+    v = fold(up8, 8, v, t);
+  } else {
+    v = v + __shfl_xor_sync(0xffffffffu, v, 8);
+  }
+  v = v + __shfl_xor_sync(0xffffffffu, v, 4);
+  v = v + __shfl_xor_sync(0xffffffffu, v, 2);
+  v = v + __shfl_xor_sync(0xffffffffu, v, 1);
+  // lane 0: sum 0, lane 16: sum 1, lane 8: sum 2, lane 24: sum 3
+  if (l == 0) sh[w] = v;
+  if (l == 16) sh[32 + w] = v;
+  if (NS > 2 && l == 8) sh[64 + w] = v;
+  if (NS > 3 && l == 24) sh[96 + w] = v;
+  const double a = warp_extreme<false>(mx0);
+  if (l == 1) sh[NS * 32 + w] = a;
+  if (MAXMIN) {
+    const double b = warp_extreme<false>(mx1), c = warp_extreme<true>(mn);
+    if (l == 2) sh[(NS + 1) * 32 + w] = b;
+    if (l == 3) sh[(NS + 2) * 32 + w] = c;
+  }
+  __syncthreads();
+  if (threadIdx.x < NV) {
+    const int q = threadIdx.x, nw = blockDim.x >> 5;
+    double r = sh[q * 32];
+    for (int k = 1; k < nw; ++k) {
+      const double o = sh[q * 32 + k];
+      r = q < NS ? r + o : (MAXMIN && q == NS + 2 ? fmin(r, o) : fmax(r, o));
+    }
+    *out[q] = r;
+  }
+}
+
+// FP32 <-> FP64 conversions of the mixed kernels on the integer pipe.  GB300
+// runs a conversion on the FP64 pipe at 2 per clock and SM, as slow as an FP64
+// add (`bench.py --pipe-rates` for the add; conversions measured 2.07), while
+// integer instructions issue at 64 lanes per clock: the ten or so integer
+// instructions below take a third of a conversion's time, and a split a
+// seventh of its four FP64-pipe instructions.  The FP64 pipe was 58 % busy in
+// the rate-stress kernel and 81 % in the kick, a third of it conversions.
+// They round as the hardware does (to nearest even); values outside the
+// normal range, other than zero, take the hardware's conversion.
+__device__ __forceinline__ double f2d(float f) {
+  const unsigned u = __float_as_uint(f), a = u & 0x7fffffffu;
+  const bool normal = a - 0x00800000u < 0x7f000000u;
+  if (normal || a == 0u) {  // exponent rebiased from 127 to 1023, mantissa shifted by 29
+    const unsigned h = normal ? (a >> 3) + 0x38000000u : 0u;
+    return __hiloint2double((int)(h | (u & 0x80000000u)), (int)(u << 29));
+  }
+  return (double)f;
+}
+__device__ __forceinline__ float d2f(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v), a = hi & 0x7fffffffu;
+  const bool normal = a - 0x38100000u < 0x0fe00000u;  // 2^-126 <= |v| < 2^128
+  if (normal || (a | lo) == 0u) {
+    // round to nearest even at bit 29; a carry out of the mantissa raises the exponent
+    const unsigned long long r = (((unsigned long long)a << 32) | lo) + 0x0fffffffu + ((lo >> 29) & 1u);
+    const unsigned f = normal ? (unsigned)(r >> 29) - 0xc0000000u : 0u;
+    return __uint_as_float(f | (hi & 0x80000000u));
+  }
+  return __double2float_rn(v);
+}
 // Float-float split of a double: hi = fl(v), lo = fl(v - hi).
 __device__ __forceinline__ void ff_split(double v, float& hi, float& lo) {
+  const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v), a = h & 0x7fffffffu;
+  if (a - 0x3b500000u < 0x0c800000u) {  // 2^-74 <= |v| < 2^126: the remainder's last bit is a normal FP32 too
+    const unsigned lsb = (l >> 29) & 1u, sign = h & 0x80000000u;
+    const unsigned long long r = (((unsigned long long)a << 32) | l) + 0x0fffffffu + lsb;
+    hi = __uint_as_float(((unsigned)(r >> 29) - 0xc0000000u) | sign);
+    // v - hi in units of the last place of v: the low 29 bits, less 2^29 where they rounded up
+    const unsigned low = l & 0x1fffffffu, up = (low + 0x0fffffffu + lsb) & 0x20000000u;
+    const unsigned scale = (((a >> 20) - 948u) << 23) | sign;  // 2^(exponent - 52)
+    lo = (float)((int)low - (int)up) * __uint_as_float(scale);
+    return;
+  }
+  if ((a | l) == 0u) { hi = __uint_as_float(h); lo = 0.0f; return; }
   hi = __double2float_rn(v);
   lo = __double2float_rn(v - (double)hi);
 }
@@ -315,10 +427,12 @@ __device__ __forceinline__ double stress_update(StressIO& s, const double sr[6],
 
 // Plastic work heat source (Particle::CalcPlasticWorkHeat, Particle.cpp:922-939):
 // q = Sigma : (Strain_pl_incr / dt) with the off-diagonal pairs doubled.
-__device__ __forceinline__ double plastic_heat(const double sig[6], const double epli[6], double dt) {
-  double f = 1. / dt;
+__device__ __forceinline__ double plastic_heat_f(const double sig[6], const double epli[6], double f) {  // f = 1 / dt
   return sig[0] * (f * epli[0]) + 2.0 * sig[3] * (f * epli[3]) + 2.0 * sig[4] * (f * epli[4]) + sig[1] * (f * epli[1]) +
          2.0 * sig[5] * (f * epli[5]) + sig[2] * (f * epli[2]);
+}
+__device__ __forceinline__ double plastic_heat(const double sig[6], const double epli[6], double dt) {
+  return plastic_heat_f(sig, epli, 1. / dt);
 }
 
 }  // namespace wf

@@ -469,8 +469,9 @@ __global__ void __launch_bounds__(BLOCK) k_contact_kick(DevPtrs P, DomainConst K
         }
     } else if (kind == 0) {  // half kick v += a * 0.5 * dt (rigid-mesh particles have a = 0)
       double vn[3];
+      const double hdt = 0.5 * dt;
       for (int d = 0; d < 3; ++d) {
-        vn[d] = col(P, C_V + d, N, i) + a[d] * 0.5 * dt;
+        vn[d] = col(P, C_V + d, N, i) + a[d] * hdt;
         colw(P, C_V + d, N, i) = vn[d];
       }
       if (K.mixed) rec_set_v3(P, N, i, vn);

@@ -42,7 +42,7 @@ struct KSum {
     c = (t - s) - y;
     s = t;
   }
-  __device__ __forceinline__ double value() const { return (double)s - (double)c; }
+  __device__ __forceinline__ double value() const { return f2d(s) - f2d(c); }
 };
 
 // Packed two-element FP32 arithmetic (add/sub/mul/fma .f32x2): one issue slot
@@ -85,8 +85,8 @@ struct KSum2 {
     c = sub2(sub2(t, s), y);
     s = t;
   }
-  __device__ __forceinline__ double value0() const { return (double)s.x - (double)c.x; }
-  __device__ __forceinline__ double value1() const { return (double)s.y - (double)c.y; }
+  __device__ __forceinline__ double value0() const { return f2d(s.x) - f2d(c.x); }
+  __device__ __forceinline__ double value1() const { return f2d(s.y) - f2d(c.y); }
 };
 
 __device__ __forceinline__ float4 ld4(const float4* p) { return __ldg(p); }
@@ -600,7 +600,7 @@ __device__ __forceinline__ void density_drift_mx(const DevPtrs& P, const DomainC
     const PosVel pi = posvel(ld4(ri + (size_t)RC_XV * N), ld4(ri + (size_t)RC_L * N), vw);
     CorrM cm;
     if (GC) cm = load_corr(P, N, i);
-    float rhoif = (float)rhoi;
+    const float rhoif = GC ? d2f(rhoi) : 0.f;
     KSum s;
     int len = P.row_len[i];
     const int* nb = P.nbr + i;
@@ -640,12 +640,13 @@ __device__ __forceinline__ void density_drift_mx(const DevPtrs& P, const DomainC
   // here, records included, instead of in a BC pass after this kernel
   double vb[3];
   const bool bc = bc_velocity(P.tab, icol(P, I_ID, N, i), P.st->Time, vb);
+  const double hdt = 0.5 * dt;
   for (int d = 0; d < 3; ++d) {
     double v = col(P, C_V + d, N, i);
     double du = v * dt;
     colw(P, C_DISP + d, N, i) = col(P, C_DISP + d, N, i) + du;
     double xn = col(P, C_X + d, N, i) + du;
-    double vn = bc ? vb[d] : (K.leapfrog ? v : v + col(P, C_A + d, N, i) * dt / 2.);
+    double vn = bc ? vb[d] : (K.leapfrog ? v : v + col(P, C_A + d, N, i) * hdt);
     if (bc) colw(P, C_A + d, N, i) = 0.0;
     colw(P, C_XN + d, N, i) = xn;
     colw(P, C_VN + d, N, i) = vn;
@@ -654,18 +655,20 @@ __device__ __forceinline__ void density_drift_mx(const DevPtrs& P, const DomainC
   }
   // Pressure of the updated density (EOS case 0, Functions.cpp:206-212) and the
   // temperature after this step's update (Thermal.cpp:727-734): both depend only
-  // on this particle, so the fused rate/energy gather can read them.
+  // on this particle, so the fused rate/energy gather can read them.  Without
+  // the thermal solver the temperature does not change: its groups stay.
   double cs = col(P, C_CS, N, i);
   double pn = col(P, C_P0, N, i) + (cs * cs) * (rn - col(P, C_RHO0, N, i));
-  double Tn = col(P, C_T, N, i) + (K.thermal_solver ? dt * col(P, C_DTDT, N, i) : 0.0);
-  float th, tl;
-  ff_split(Tn, th, tl);
   float4* r = P.rn + i;
   r[(size_t)RN_XV * N] = make_float4(nxh[0], nxh[1], nxh[2], nvh[0]);
-  r[(size_t)RN_L * N] = lo_pack(nxl, nvl, (float)mrn);
-  float pr2 = solid ? (float)(pn * irn * irn) : 0.f;
+  r[(size_t)RN_L * N] = lo_pack(nxl, nvl, d2f(mrn));
+  float pr2 = solid ? d2f(pn * irn * irn) : 0.f;
   r[(size_t)RN_VW * N] = make_float4(nvh[1], nvh[2], UNI ? K.h_f : vw.z, pr2);  // the rate gather reads p/rho^2 here
-  r[(size_t)RN_E * N] = make_float4(pr2, ri[(size_t)RC_MISC * N].z, th, tl);
+  if (K.thermal_solver) {
+    float th, tl;
+    ff_split(col(P, C_T, N, i) + dt * col(P, C_DTDT, N, i), th, tl);
+    r[(size_t)RN_E * N] = make_float4(pr2, ri[(size_t)RC_MISC * N].z, th, tl);
+  }
 }
 template <bool GC, bool UNI>
 __global__ void __maxnreg__(64) k_density_drift_mx(DevPtrs P, DomainConst K) {
@@ -717,7 +720,7 @@ __device__ __forceinline__ void rate_mx(const DevPtrs& P, const DomainConst& K, 
     // (00, 01) (10, 11) (20, 21) (02, 12) (22, kinetic)
     KSum2 M[5];
     KSum cnd;
-    const float mass_i = (float)col(P, C_MASS, N, i);
+    const float mass_i = d2f(col(P, C_MASS, N, i));
     int len = P.row_len[i];
     const int* nb = P.nbr + i;
     auto key = [&](int k) { return nb[(size_t)k * N]; };
@@ -834,20 +837,20 @@ __device__ __forceinline__ double stress_update_mx(StressMx& s, const float sr[6
                                                    double rho0, double Cs, double P0, double G, double T, int fail,
                                                    int model, const MaterialDev* M, double dt) {
   s.pressure = P0 + (Cs * Cs) * (rho - rho0);
-  float S[3][3] = {{(float)s.tau[0], (float)s.tau[3], (float)s.tau[4]},
-                   {(float)s.tau[3], (float)s.tau[1], (float)s.tau[5]},
-                   {(float)s.tau[4], (float)s.tau[5], (float)s.tau[2]}};
+  float tf[6];
+  for (int c = 0; c < 6; ++c) tf[c] = d2f(s.tau[c]);
+  float S[3][3] = {{tf[0], tf[3], tf[4]}, {tf[3], tf[1], tf[5]}, {tf[4], tf[5], tf[2]}};
   float W[3][3] = {{0.f, rr[0], rr[1]}, {-rr[0], 0.f, rr[2]}, {-rr[1], -rr[2], 0.f}};
   const int ui[6] = {0, 1, 2, 0, 0, 1}, uj[6] = {0, 1, 2, 1, 2, 2};
   float s3 = (1.0f / 3.0f) * (sr[0] + sr[1] + sr[2]);
-  float twoG = (float)(2.0 * G), dtf = (float)dt;
+  float twoG = 2.0f * d2f(G), dtf = d2f(dt);
   double t6[6];
   for (int c = 0; c < 6; ++c) {
     int a = ui[c], b = uj[c];
     float srt = S[a][2] * W[b][2] + S[a][1] * W[b][1] + S[a][0] * W[b][0];
     float rs = W[a][2] * S[2][b] + W[a][1] * S[1][b] + W[a][0] * S[0][b];
     float dev = sr[c] - (c < 3 ? s3 : 0.f);
-    t6[c] = s.tau[c] + (double)(dtf * (twoG * dev + srt + rs));
+    t6[c] = s.tau[c] + f2d(dtf * (twoG * dev + srt + rs));
   }
   float d01 = sr[0] - sr[1], d12 = sr[1] - sr[2], d20 = sr[2] - sr[0];
   s.esr = sqrtf(0.5f * (d01 * d01 + d12 * d12 + d20 * d20) + 3.0f * (sr[3] * sr[3] + sr[5] * sr[5] + sr[4] * sr[4]));
@@ -866,14 +869,13 @@ __device__ __forceinline__ double stress_update_mx(StressMx& s, const float sr[6
         for (int c = 0; c < 6; ++c) t6[c] = sc * t6[c];
     }
     if (model == 1 && M) {
-      if (s.pl_strain + M->eps0 > M->eps1) s.sigmay = (double)((float)M->K * powf((float)(s.pl_strain + M->eps0), (float)M->m));
+      if (s.pl_strain + M->eps0 > M->eps1) s.sigmay = f2d(M->K_f * powf(d2f(s.pl_strain + M->eps0), M->m_f));
       else s.sigmay = M->sy0;
     } else if (model == 2 && M) {
-      float Th = (float)((T - M->T_t) / (M->T_m - M->T_t));
+      float Th = d2f((T - M->T_t) * M->inv_Tmt);
       float f = 1.0f;
-      if (s.esr > (float)M->eps_0) f = 1.0f + (float)M->C * logf(s.esr / (float)M->eps_0);
-      s.sigmay = (double)(((float)M->A + (float)M->B * powf((float)s.pl_strain, (float)M->n)) * f *
-                          (1.0f - powf(Th, (float)M->jm)));
+      if (s.esr > M->eps_0_f) f = 1.0f + M->C_f * logf(s.esr / M->eps_0_f);
+      s.sigmay = f2d((M->A_f + M->B_f * powf(d2f(s.pl_strain), M->n_f)) * f * (1.0f - powf(Th, M->jm_f)));
     }
     sy = s.sigmay;
     if (!(sy > 0.0 && tJ2 <= sy * sy)) {
@@ -888,7 +890,7 @@ __device__ __forceinline__ double stress_update_mx(StressMx& s, const float sr[6
     }
   }
   for (int c = 0; c < 6; ++c) s.tau[c] = t6[c];
-  for (int c = 0; c < 6; ++c) s.sig[c] = (c < 3 ? -s.pressure : 0.0) + t6[c];
+  for (int c = 0; c < 6; ++c) s.sig[c] = c < 3 ? t6[c] - s.pressure : t6[c];
   return dep;
 }
 
@@ -899,7 +901,7 @@ __device__ __forceinline__ double stress_update_mx(StressMx& s, const float sr[6
 // included) for the block reductions.
 template <bool HEAT, bool THERMAL, bool FUSED>
 __device__ __forceinline__ void stress_mx(const DevPtrs& P, const DomainConst& K, int i, const RateOut& ro) {
-  __shared__ double sh[32];
+  __shared__ double sh[6 * 32];
   size_t N = K.N;
   double dt = P.st->deltat;
   double plw = 0.0, maxpl = 0.0, maxT = -1e300, minT = 1e300, dkin = 0.0, dint = 0.0;
@@ -910,7 +912,8 @@ __device__ __forceinline__ void stress_mx(const DevPtrs& P, const DomainConst& K
     }
     double rho = col(P, C_RHON, N, i);
     colw(P, C_RHO, N, i) = rho;
-    colw(P, C_MRHO, N, i) = col(P, C_MRHON, N, i);
+    const double mrho = col(P, C_MRHON, N, i);
+    colw(P, C_MRHO, N, i) = mrho;
     const float4* rn = P.rn + i;
     float4* rc = P.rc + i;
     rc[(size_t)RC_XV * N] = rn[(size_t)RN_XV * N];
@@ -920,9 +923,8 @@ __device__ __forceinline__ void stress_mx(const DevPtrs& P, const DomainConst& K
     // or in the uniform-particle layout Sigma/rho^2 xz and yz (written below
     // for SPH particles, 0 for the rest)
     nvw.z = K.uni ? 0.f : nvw.z;
-    nvw.w = K.uni ? 0.f : (float)rho;
-    float4 ne = rn[(size_t)RN_E * N];
-    float4 misc = rc[(size_t)RC_MISC * N];
+    const float rhof = d2f(rho);
+    nvw.w = K.uni ? 0.f : rhof;
     maxpl = col(P, C_PLS, N, i);
     const bool sph = icol(P, I_KIND, N, i) == 0;
     if constexpr (FUSED) {  // the columns k_rate_mx leaves behind (C_DINT: overwritten below for SPH particles)
@@ -945,10 +947,12 @@ __device__ __forceinline__ void stress_mx(const DevPtrs& P, const DomainConst& K
       double T = col(P, C_T, N, i);
       double dep = stress_update_mx(s, sr, rr, rho, col(P, C_RHO0, N, i), col(P, C_CS, N, i), col(P, C_P0, N, i),
                                     col(P, C_G, N, i), T, icol(P, I_FAIL, N, i), icol(P, I_MODEL, N, i), Mt, dt);
+      double srd[6];
       for (int c = 0; c < 6; ++c) {
         colw(P, C_TAU + c, N, i) = s.tau[c];
         colw(P, C_SIG + c, N, i) = s.sig[c];
-        colw(P, C_EPS + c, N, i) = dt * (double)sr[c] + col(P, C_EPS + c, N, i);
+        srd[c] = f2d(sr[c]);
+        colw(P, C_EPS + c, N, i) = dt * srd[c] + col(P, C_EPS + c, N, i);
       }
       // Strain_pl_incr = dep / sigma_y (sigma - tr-free part) and Strain_pl += it
       // (Particle.cpp:1040-1058); kept from the last plastic step otherwise.
@@ -966,18 +970,16 @@ __device__ __forceinline__ void stress_mx(const DevPtrs& P, const DomainConst& K
           colw(P, C_EPL + c, N, i) = col(P, C_EPL + c, N, i) + epli[c];
         }
       }
-      double srd[6];
-      for (int c = 0; c < 6; ++c) srd[c] = (double)sr[c];
       if (HEAT) {
         double q = col(P, C_QPL, N, i);
         if (s.delta_pl_strain > 0.0) {
           if (!(dep > 0.0))
             for (int c = 0; c < 6; ++c) epli[c] = col(P, C_EPLI + c, N, i);
-          q = plastic_heat(s.sig, epli, dt);
+          q = plastic_heat_f(s.sig, epli, K.auto_ts || K.auto_ts_acc ? 1. / dt : K.inv_dt);
         }
         colw(P, C_QPL, N, i) = q;
         colw(P, C_PSEN, N, i) = col(P, C_PSEN, N, i) + q * dt;
-        plw = col(P, C_MASS, N, i) / rho * q;
+        plw = mrho * q;
       }
       if (THERMAL) {  // T(n+1) (already in the next record), then CalcTempInc's dTdt
         T += dt * col(P, C_DTDT, N, i);
@@ -991,37 +993,40 @@ __device__ __forceinline__ void stress_mx(const DevPtrs& P, const DomainConst& K
         for (int c = 0; c < 3; ++c) srd[c] = srd[c] + st;
       }
       for (int c = 0; c < 6; ++c) colw(P, C_SR + c, N, i) = srd[c];
-      for (int c = 0; c < 3; ++c) colw(P, C_RR + c, N, i) = (double)rr[c];
+      for (int c = 0; c < 3; ++c) colw(P, C_RR + c, N, i) = f2d(rr[c]);
       colw(P, C_P, N, i) = s.pressure; colw(P, C_PLS, N, i) = s.pl_strain; colw(P, C_DPLS, N, i) = s.delta_pl_strain;
-      colw(P, C_SY, N, i) = s.sigmay; colw(P, C_EP, N, i) = s.Ep; colw(P, C_ESR, N, i) = (double)s.esr;
+      colw(P, C_SY, N, i) = s.sigmay; colw(P, C_EP, N, i) = s.Ep; colw(P, C_ESR, N, i) = f2d(s.esr);
       maxpl = s.pl_strain;
       mark_yield(P, K, N, i, s.pl_strain);
       // CalcIntEnergyEqn (Particle.cpp:941-950)
-      dint = col(P, C_MRHO, N, i) * (s.tau[0] * srd[0] + 2.0 * s.tau[3] * srd[3] + 2.0 * s.tau[4] * srd[4] +
+      dint = mrho * (s.tau[0] * srd[0] + 2.0 * s.tau[3] * srd[3] + 2.0 * s.tau[4] * srd[4] +
                                      s.tau[1] * srd[1] + 2.0 * s.tau[5] * srd[5] + s.tau[2] * srd[2]);
       colw(P, C_DINT, N, i) = dint;
-      float c2 = 1.0f / ((float)rho * (float)rho);
-      rc[(size_t)RC_S0 * N] = make_float4(c2 * (float)s.sig[0], c2 * (float)s.sig[1], c2 * (float)s.sig[2], c2 * (float)s.sig[3]);
+      float c2 = 1.0f / (rhof * rhof);
+      rc[(size_t)RC_S0 * N] = make_float4(c2 * d2f(s.sig[0]), c2 * d2f(s.sig[1]), c2 * d2f(s.sig[2]), c2 * d2f(s.sig[3]));
+      const float s4 = c2 * d2f(s.sig[4]), s5 = c2 * d2f(s.sig[5]);
       if (K.uni) {
-        nvw.z = c2 * (float)s.sig[4];
-        nvw.w = c2 * (float)s.sig[5];
+        nvw.z = s4;
+        nvw.w = s5;
       } else {
         float4 s1o = rc[(size_t)RC_S1 * N];  // mass and Cs carried over
-        rc[(size_t)RC_S1 * N] = make_float4(c2 * (float)s.sig[4], c2 * (float)s.sig[5], s1o.z, s1o.w);
+        rc[(size_t)RC_S1 * N] = make_float4(s4, s5, s1o.z, s1o.w);
       }
     }
     rc[(size_t)RC_VW * N] = nvw;
-    rc[(size_t)RC_MISC * N] = make_float4(misc.x, misc.y, misc.z, ne.z);
-    rc[(size_t)RC_T2 * N] = make_float4(ne.w, 0.f, 0.f, 0.f);
+    if (THERMAL) {
+      const float4 ne = rn[(size_t)RN_E * N];
+      reinterpret_cast<float*>(rc + (size_t)RC_MISC * N)[3] = ne.z;
+      rc[(size_t)RC_T2 * N] = make_float4(ne.w, 0.f, 0.f, 0.f);
+    }
   }
-  double r;
-  r = block_reduce<1>(maxpl, sh); if (threadIdx.x == 0) P.partials[S_MAXPL * K.nblocks + blockIdx.x] = r;
-  r = block_reduce<0>(dkin, sh); if (threadIdx.x == 0) P.partials[S_DKIN * K.nblocks + blockIdx.x] = r;
-  r = block_reduce<0>(dint, sh); if (threadIdx.x == 0) P.partials[S_DINT * K.nblocks + blockIdx.x] = r;
-  if (HEAT) { r = block_reduce<0>(plw, sh); if (threadIdx.x == 0) P.partials[S_PLW * K.nblocks + blockIdx.x] = r; }
-  if (THERMAL) {
-    r = block_reduce<1>(maxT, sh); if (threadIdx.x == 0) P.partials[S_MAXT * K.nblocks + blockIdx.x] = r;
-    r = block_reduce<2>(minT, sh); if (threadIdx.x == 0) P.partials[S_MINT * K.nblocks + blockIdx.x] = r;
+  auto part = [&](int slot) { return P.partials + (size_t)slot * K.nblocks + blockIdx.x; };
+  if constexpr (HEAT) {
+    double* const o[6] = {part(S_DKIN), part(S_DINT), part(S_PLW), part(S_MAXPL), part(S_MAXT), part(S_MINT)};
+    block_reduce_all<3, THERMAL>({dkin, dint, plw}, maxpl, maxT, minT, sh, o);
+  } else {
+    double* const o[5] = {part(S_DKIN), part(S_DINT), part(S_MAXPL), part(S_MAXT), part(S_MINT)};
+    block_reduce_all<2, THERMAL>({dkin, dint}, maxpl, maxT, minT, sh, o);
   }
 }
 template <bool HEAT, bool THERMAL>
