@@ -46,7 +46,9 @@ enum F64Col : int {
   C_XN = 107, C_VN = 110, C_RHON = 113, C_MRHON = 114, C_TIR = 115,
   C_PR2N = 121,            // next-step Pressure / Density^2 (plain form; read by the fused rate gather)
   C_TN = 122,              // next-step temperature (plain form)
-  NF64 = 123
+  C_CSUM = 123,            // contact sums of a particle in contact (one rigid mesh): |force|, reaction,
+                           // external work, force (3)
+  NF64 = 129
 };
 enum I32Col : int {
   I_ID = 0, I_IDORIG, I_NWS, I_MAT, I_MODEL, I_FAIL, I_MATERIAL, I_NB, I_KIND, I_ELEM, I_MESH, I_ORIG,
@@ -216,6 +218,7 @@ struct StepState {
                        // searches clear it)
   int errors;
   int surface_count;
+  int cp_count;        // particles with contact pairs (DevPtrs::cp_list)
   unsigned long long dyn_friction;  // contact-pair evaluations that took the dynamic-friction branch
   // Verlet-skin reuse of the neighbour search (DomainConst::skin_on)
   unsigned long long maxdisp2_bits;  // largest squared displacement since the superset was built (as bits)
@@ -327,6 +330,7 @@ struct DevPtrs {
                           // acceleration and density passes
   int* cp_len;            // contact pairs per particle
   int* cp;                // ELL, width MAX_CP
+  int* cp_list;           // particles that have contact pairs (StepState::cp_count of them, in any order)
   const int* bc_list;     // original indices of particles carrying a BC zone id
   // rigid meshes
   double* node;           // 3 * nnodes (SoA: x[nnodes], y, z)

@@ -684,6 +684,7 @@ struct wf_domain {
     P.cp_len = dalloc<int>(n);
     CK(cudaMemsetAsync(P.cp_len, 0, sizeof(int) * n, stream));
     P.cp = contact ? dalloc<int>((size_t)MAX_CP * n) : dalloc<int>(1);
+    P.cp_list = dalloc<int>(contact ? n : 1);
     std::vector<int> inv0(n);
     std::iota(inv0.begin(), inv0.end(), 0);
     CK(cudaMemcpyAsync(P.inv, inv0.data(), sizeof(int) * n, cudaMemcpyHostToDevice, stream));
@@ -885,6 +886,7 @@ struct wf_domain {
                {P.cp, contact ? sizeof(int) * MAX_CP * n : sizeof(int)}, {P.node, sizeof(double) * hnode.size()},
                {P.node_v, sizeof(double) * hnode.size()}, {P.elem_normal, sizeof(double) * hnorm.size()},
                {P.elem_pplane, sizeof(double) * hpp.size()}, {P.elem_particle, sizeof(int) * hep.size()}};
+    if (contact) regions.push_back({P.cp_list, sizeof(int) * n});
     if (stage_ready)
       regions.insert(regions.end(), {{P.halo, sizeof(int) * nsb * stage_cap}, {P.halo_len, sizeof(int) * nsb},
                                      {P.nslot, sizeof(unsigned short) * MAX_NB * n}});

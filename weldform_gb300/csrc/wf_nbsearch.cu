@@ -864,6 +864,7 @@ __global__ void k_contact_pairs(DevPtrs P, DomainConst K) {
   }
   for (int k = 0; k < cnt; ++k) P.cp[(size_t)k * N + i] = row[k];
   P.cp_len[i] = cnt;
+  if (cnt > 0) P.cp_list[atomicAdd(&P.st->cp_count, 1)] = i;
   if (overflow) atomicOr(&P.st->errors, ERR_CONTACT_OVERFLOW);
   npairs += (unsigned)cnt;
   }
@@ -879,6 +880,7 @@ __global__ void k_search_begin(DevPtrs P) {
   P.st->pair_count = 0;
   P.st->contact_pair_count = 0;
   P.st->surface_count = 0;
+  P.st->cp_count = 0;
   P.st->nan_count = 0;
   P.st->maxdisp2_bits = 0;
   P.st->nb_searches += 1;

@@ -361,8 +361,161 @@ __global__ void k_bc(DevPtrs P, DomainConst K, int vcol) {
 __device__ __forceinline__ double dot3(const double a[3], const double b[3]) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
 __device__ __forceinline__ double norm3(const double a[3]) { return sqrt(dot3(a, a)); }
 
-// NM: per-mesh force accumulators a thread keeps — 0 without contact, 1 with
-// one rigid mesh (kept in registers), MAX_MESHES with several (indexed by the
+// Contact with one rigid mesh (Contact_Wang.cpp:15-348), several lanes per
+// particle that has contact pairs.  Each pair's predicted position depends on
+// the acceleration that earlier pairs added, so the pairs are taken in order;
+// but of a particle's ~30 pairs one or two lie over its projection, and the
+// others change nothing.  The lanes test a chunk of pairs at the current
+// acceleration, the first one that is in contact is applied by all of them,
+// and the lanes after it test again: the order of a serial walk, with its
+// chain of ~30 dependent FP64 pair tests cut to the pairs in contact.  A thread
+// per particle in the kick kernel took 350 us of that chain's latency at
+// 1,171,832 particles (a few warps per SM) and 60 us at 11,976; this takes 54
+// and 15 us.  More lanes shorten the chain and multiply the FP64 work that all
+// of a particle's lanes share: 54 us with 4 lanes against 116, 83 and 141 with
+// 8, 16 and 32 at the large size, 27 against 23, 17 and 15 at the small one.
+// So a particle gets the widest group that keeps the particles in contact
+// within four warps per SM.  The sums of each particle go to its C_CSUM
+// columns, which the kick kernel adds in particle order.
+constexpr int CONTACT_THREADS = 152 * 128;
+__global__ void __launch_bounds__(128) k_contact_force(DevPtrs P, DomainConst K) {
+  const size_t N = K.N;
+  const int count = P.st->cp_count;
+  int G = 32;
+  while (G > 4 && (long long)count * G > CONTACT_THREADS) G >>= 1;
+  const int lane = threadIdx.x & 31, sub = lane & (G - 1), base_lane = lane - sub;
+  const unsigned gmask = (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << base_lane;
+  const int groups = gridDim.x * blockDim.x / G;
+  const double dt = P.st->deltat;  // the step's time step before AdaptiveTimeStep (prev_deltat)
+  unsigned ndyn = 0;               // pairs in the dynamic-friction branch (lane 0 of the group counts)
+  for (int g = (blockIdx.x * blockDim.x + threadIdx.x) / G; g < count; g += groups) {
+    const int i = P.cp_list[g];
+    const int ncp = P.cp_len[i];
+    double a[3], x[3], v[3];
+    for (int d = 0; d < 3; ++d) { a[d] = col(P, C_A + d, N, i); x[d] = col(P, C_X + d, N, i); v[d] = col(P, C_V + d, N, i); }
+    const double m1 = col(P, C_MASS, N, i), h1 = col(P, C_H, N, i);
+    if (P.tx && sub == 0)
+      for (int d = 0; d < 3; ++d) P.tx[(size_t)(TX_APRE + d) * N + i] = a[d];
+    double cf[3] = {0, 0, 0}, cfv[3] = {0, 0, 0}, dcont = 0.0, cfsum = 0.0, crsum = 0.0, extw = 0.0;
+    double kij = -1.0, psi = 0.0, im1 = 0.0;  // pair stiffness, damping, 1 / m1: formed at the first pair in contact
+    for (int base = 0; base < ncp; base += G) {
+      bool have = base + sub < ncp;
+      double n2[3] = {0, 0, 0}, v2[3] = {0, 0, 0}, pplane = 0.0, node[3][3];
+      if (have) {
+        const int p2 = P.cp[(size_t)(base + sub) * N + i];
+        const int e = icol(P, I_ELEM, N, p2);
+        for (int d = 0; d < 3; ++d) { n2[d] = col(P, C_NORMAL + d, N, p2); v2[d] = col(P, C_V + d, N, p2); }
+        pplane = P.elem_pplane[e];
+        for (int c = 0; c < 3; ++c) {
+          const int nd = P.elem_node[3 * e + c];
+          for (int d = 0; d < 3; ++d) node[c][d] = P.node[(size_t)d * P.nnodes + nd];
+        }
+        // Most of the chunk's triangles are not under the particle: left out
+        // here by the inside test in FP32 on coordinates relative to the
+        // particle, which the acceleration does not enter (the projection moves
+        // along the normal only), with a margin of 2e-5 of its products over
+        // their FP32 rounding; the FP64 test below decides the rest.
+        float fn[3], q[3][3];
+        for (int d = 0; d < 3; ++d) {
+          fn[d] = d2f(n2[d]);
+          for (int c = 0; c < 3; ++c) q[c][d] = d2f(node[c][d] - x[d]);
+        }
+#pragma unroll
+        for (int ii = 0; ii < 3; ++ii) {
+          const float* pa = q[ii];
+          const float* pb = q[ii == 2 ? 0 : ii + 1];
+          // (pb - pa) x (0 - pa) . n = -(pb x pa) . n
+          const float t0 = pb[1] * pa[2], t1 = pb[2] * pa[1], t2 = pb[2] * pa[0], t3 = pb[0] * pa[2], t4 = pb[0] * pa[1], t5 = pb[1] * pa[0];
+          const float e2 = -((t0 - t1) * fn[0] + (t2 - t3) * fn[1] + (t4 - t5) * fn[2]);
+          const float mag = fabsf(t0) + fabsf(t1) + fabsf(t2) + fabsf(t3) + fabsf(t4) + fabsf(t5);
+          if (e2 < -2e-5f * mag) have = false;
+        }
+      }
+      int from = 0;  // lanes of the chunk not yet taken in order
+      while (__any_sync(gmask, have && sub >= from)) {
+        double xp[3], dist = 0.0;
+        for (int d = 0; d < 3; ++d) xp[d] = x[d] + v[d] * dt + a[d] * dt * dt / 2.0;
+        bool hit = have && sub >= from;
+        if (hit) {
+          dist = dot3(n2, xp) - pplane;
+          hit = dist < h1;
+        }
+        if (hit) {
+          const double qj[3] = {x[0] - dist * n2[0], x[1] - dist * n2[1], x[2] - dist * n2[2]};
+#pragma unroll
+          for (int ii = 0; ii < 3; ++ii) {
+            if (!hit) break;
+            const int jj = ii == 2 ? 0 : ii + 1;
+            const double* pa = node[ii];
+            const double* pb = node[jj];
+            double u[3] = {pb[0] - pa[0], pb[1] - pa[1], pb[2] - pa[2]};
+            double w[3] = {qj[0] - pa[0], qj[1] - pa[1], qj[2] - pa[2]};
+            double c[3] = {u[1] * w[2] - u[2] * w[1], u[2] * w[0] - u[0] * w[2], u[0] * w[1] - u[1] * w[0]};
+            if (dot3(c, n2) < 0.0) hit = false;
+          }
+        }
+        const unsigned hits = __ballot_sync(gmask, hit);
+        if (!hits) break;
+        const int first = __ffs(hits) - 1;  // lane of the first pair in contact
+        double nn[3], vv[3];
+        for (int d = 0; d < 3; ++d) { nn[d] = __shfl_sync(gmask, n2[d], first); vv[d] = __shfl_sync(gmask, v2[d], first); }
+        const double dst = __shfl_sync(gmask, dist, first);
+        const double vr[3] = {v[0] - vv[0], v[1] - vv[1], v[2] - vv[2]};
+        const double delta_ = -dot3(nn, vr);
+        const double delta = h1 - dst;
+        if (kij < 0.0) {
+          im1 = 1.0 / m1;
+          if (K.contact_alg == 1) {
+            double rho1 = col(P, C_RHO0, N, i), cs = col(P, C_CS, N, i), G = col(P, C_G, N, i);
+            double bulk = cs * cs * rho1;
+            double dS = pow(m1 / rho1, 0.33333);
+            kij = K.PFAC * (9. * bulk * G / (3. * bulk + G) * dS);
+          } else if (K.contact_alg == 2) {
+            kij = K.PFAC * pow(m1 / col(P, C_RHO, N, i), 2.0 / 3.0);
+          } else {
+            kij = 2.0 * m1 / (dt * dt);
+          }
+          psi = K.DFAC == 0.0 ? 0.0 : 2. * m1 * sqrt(kij * im1) * K.DFAC;
+        }
+        const double s = kij * delta - psi * delta_;
+        for (int d = 0; d < 3; ++d) cf[d] = s * nn[d];
+        dcont = delta;
+        for (int d = 0; d < 3; ++d) a[d] = a[d] + cf[d] * im1;
+        if (K.friction_sta > 0.) {
+          double du[3];
+          for (int d = 0; d < 3; ++d) du[d] = (xp[d] - x[d]) - vv[d] * dt;
+          double dn = dot3(du, nn);
+          double tg[3];
+          for (int d = 0; d < 3; ++d) tg[d] = kij * (du[d] - dn * nn[d]);
+          double ntg = norm3(tg), ncf = norm3(cf);
+          if (ntg < K.friction_sta * ncf) {
+            for (int d = 0; d < 3; ++d) { double q = tg[d] * im1; cf[d] -= q; a[d] -= q; }
+          } else {  // dynamic branch (Contact_Wang.cpp:284-290)
+            if (sub == 0) ++ndyn;
+            const double fs = K.friction_dyn * ncf / ntg;
+            for (int d = 0; d < 3; ++d) { double td = fs * tg[d]; cf[d] -= td; a[d] -= td * im1; }
+          }
+        }
+        cfsum += norm3(cf);
+        for (int d = 0; d < 3; ++d) cfv[d] += cf[d];
+        crsum += dot3(a, nn) * m1;
+        extw += dot3(cf, vv);
+        from = first - base_lane + 1;
+      }
+    }
+    if (sub == 0) {
+      for (int d = 0; d < 3; ++d) { colw(P, C_CF + d, N, i) = cf[d]; colw(P, C_A + d, N, i) = a[d]; }
+      colw(P, C_DCONT, N, i) = dcont;
+      colw(P, C_CSUM, N, i) = cfsum; colw(P, C_CSUM + 1, N, i) = crsum; colw(P, C_CSUM + 2, N, i) = extw;
+      for (int d = 0; d < 3; ++d) colw(P, C_CSUM + 3 + d, N, i) = cfv[d];
+    }
+  }
+  if (ndyn) atomicAdd(&P.st->dyn_friction, (unsigned long long)ndyn);
+}
+
+// NM: rigid meshes — 0 without contact; 1: the pairs were taken by
+// k_contact_force, whose sums this kernel adds; with several a thread walks its
+// particle's pairs and keeps MAX_MESHES force accumulators (indexed by the
 // pair's mesh, so they live in local memory).
 template <int NM>
 __global__ void __launch_bounds__(BLOCK) k_contact_kick(DevPtrs P, DomainConst K) {
@@ -380,9 +533,17 @@ __global__ void __launch_bounds__(BLOCK) k_contact_kick(DevPtrs P, DomainConst K
   if (i < K.N) {
     int kind = icol(P, I_KIND, N, i);
     double a[3] = {col(P, C_A, N, i), col(P, C_A + 1, N, i), col(P, C_A + 2, N, i)};
-    if (P.tx)
+    if (P.tx && !(NM == 1 && kind == 0 && P.cp_len[i] > 0))  // taped by k_contact_force where there are pairs
       for (int d = 0; d < 3; ++d) P.tx[(size_t)(TX_APRE + d) * N + i] = a[d];
-    if (CONTACT) {
+    if (NM == 1) {
+      if (kind == 0 && P.cp_len[i] > 0) {
+        cfsum = col(P, C_CSUM, N, i); crsum = col(P, C_CSUM + 1, N, i); extw = col(P, C_CSUM + 2, N, i);
+        for (int d = 0; d < 3; ++d) cfv[0][d] = col(P, C_CSUM + 3 + d, N, i);
+      } else {
+        for (int d = 0; d < 3; ++d) colw(P, C_CF + d, N, i) = 0.0;
+        colw(P, C_DCONT, N, i) = 0.0;
+      }
+    } else if (CONTACT) {
       double cf[3] = {0, 0, 0}, dcont = 0.0;
       int ncp = kind == 0 ? P.cp_len[i] : 0;
       if (ncp > 0) {
@@ -448,8 +609,7 @@ __global__ void __launch_bounds__(BLOCK) k_contact_kick(DevPtrs P, DomainConst K
             }
           }
           cfsum += norm3(cf);
-          if (NM == 1) for (int d = 0; d < 3; ++d) cfv[0][d] += cf[d];  // the only mesh
-          else if (m < NV) for (int d = 0; d < 3; ++d) cfv[m][d] += cf[d];
+          if (m < NV) for (int d = 0; d < 3; ++d) cfv[m][d] += cf[d];
           crsum += dot3(a, n2) * m1;
           extw += dot3(cf, v2);
         }
@@ -491,19 +651,23 @@ __global__ void __launch_bounds__(BLOCK) k_contact_kick(DevPtrs P, DomainConst K
     if (threadIdx.x == 0) P.partials[S_DTA * K.nblocks + blockIdx.x] = r;
   }
   if (CONTACT) {
-    // one counter update per warp (a per-pair atomic on one address serialised
-    // the kernel on contact-heavy steps)
-    unsigned wdyn = __reduce_add_sync(0xffffffffu, ndyn);
-    if ((threadIdx.x & 31) == 0 && wdyn) atomicAdd(&P.st->dyn_friction, (unsigned long long)wdyn);
-    double r;
-    r = block_reduce<0>(cfsum, sh); if (threadIdx.x == 0) P.partials[S_CFSUM * K.nblocks + blockIdx.x] = r;
-    r = block_reduce<0>(crsum, sh); if (threadIdx.x == 0) P.partials[S_CRSUM * K.nblocks + blockIdx.x] = r;
-    r = block_reduce<0>(extw, sh); if (threadIdx.x == 0) P.partials[S_EXTW * K.nblocks + blockIdx.x] = r;
+    if (NM > 1) {
+      // one counter update per warp (a per-pair atomic on one address serialised
+      // the kernel on contact-heavy steps)
+      unsigned wdyn = __reduce_add_sync(0xffffffffu, ndyn);
+      if ((threadIdx.x & 31) == 0 && wdyn) atomicAdd(&P.st->dyn_friction, (unsigned long long)wdyn);
+    }
+    // most blocks hold no particle in contact: their sums are zero
+    const bool some = __syncthreads_or(cfsum != 0.0 || crsum != 0.0 || extw != 0.0);
+    auto sum = [&](double v, int slot) {
+      const double r = some ? block_reduce<0>(v, sh) : 0.0;
+      if (threadIdx.x == 0) P.partials[(size_t)slot * K.nblocks + blockIdx.x] = r;
+    };
+    sum(cfsum, S_CFSUM);
+    sum(crsum, S_CRSUM);
+    sum(extw, S_EXTW);
     for (int m = 0; m < K.nmeshes && m < NV; ++m)
-      for (int d = 0; d < 3; ++d) {
-        r = block_reduce<0>(cfv[m][d], sh);
-        if (threadIdx.x == 0) P.partials[(S_CFVEC + 3 * m + d) * K.nblocks + blockIdx.x] = r;
-      }
+      for (int d = 0; d < 3; ++d) sum(cfv[m][d], S_CFVEC + 3 * m + d);
   }
 }
 
@@ -1040,7 +1204,13 @@ void launch_contact_kick(const DevPtrs& P, const DomainConst& K, cudaStream_t s)
     mark(s, "k_dt_tests");
   }
   if (!K.contact) k_contact_kick<0><<<K.nblocks, K.pblock, 0, s>>>(P, K);
-  else if (K.nmeshes == 1) k_contact_kick<1><<<K.nblocks, K.pblock, 0, s>>>(P, K);
+  else if (K.nmeshes == 1) {
+    // a few blocks per SM stride over the particles in contact
+    const long long most = (32LL * K.Nsolid + 127) / 128;
+    k_contact_force<<<(int)(most < 152 * 4 ? most : 152 * 4), 128, 0, s>>>(P, K);
+    mark(s, "k_contact_force");
+    k_contact_kick<1><<<K.nblocks, K.pblock, 0, s>>>(P, K);
+  }
   else k_contact_kick<MAX_MESHES><<<K.nblocks, K.pblock, 0, s>>>(P, K);
   mark(s, "k_contact_kick");
   if (K.leapfrog) {  // GeneralAfter, time-step control, then the full kick (the caller's BC pass follows)
