@@ -286,6 +286,10 @@ struct DomainConst {
   float h_f, cs_f;     // that h and Cs
   float inv_h_f;       // 1 / h
   float gk_c_f;        // 1 / (pi h^5): the 3D cubic spline's gradient factor GK = gk_c_f * w(q)
+  // the plain form's kernel constants for uni: 1/h, and GradKernel = near0 +
+  // near1 q for q < 1, far (2 - q)^2 / r for q < 2
+  double u_inv_h, u_near0, u_near1, u_far;
+  int lanes64;         // lanes per particle of the plain form's gathers (1, 2 or 4)
   int stage_cap;       // halo capacity of the staged gathers (0: staging off)
   int freeze_nb;       // 1: neighbour and contact topology searched only at the first step
   int nan_check;       // 1: a non-finite position at a search, or non-finite energy sums, raise ERR_NAN

@@ -180,6 +180,11 @@ struct wf_domain {
   // 8,004 particles best with 8 lanes, 29,520 with 4, 44,880 with 2 (135
   // against 142 us), 79,856 and up with 1).
   static int auto_lanes(long long n) { return n < 20000 ? 8 : (n < 40000 ? 4 : (n < 64000 ? 2 : 1)); }
+  // The plain form's gathers wait out FP64 latency while an SM holds few warps
+  // (8,004 particles: 295 us per step with one lane, 184 with two, 168 with
+  // four, 174 with eight); from ~20,000 particles the FP64 pipe is full with
+  // one (21,600: 402, 402 and 406 us; 30,600: 487, 494 and 493).
+  static int auto_lanes64(long long n) { return n < 16000 ? 4 : (n < 24000 ? 2 : 1); }
   int glanes_now() const { return glanes ? glanes : auto_lanes(hp.N); }
   int pblock_now() const { return pblock ? pblock : auto_block(hp.N); }
   int graph_key() const {
@@ -939,6 +944,7 @@ struct wf_domain {
     k.mixed = precision == WF_PRECISION_MIXED;
     k.gblock = gblock_now();
     k.glanes = glanes_now();
+    k.lanes64 = auto_lanes64(hp.N);
     k.pblock = pblock_now();
     k.fuse_rs = fuse_rs;
     k.nblocks = (int)((hp.N + k.pblock - 1) / k.pblock);
@@ -1094,6 +1100,11 @@ struct wf_domain {
     float ih = 1.0f / K.h_f, ih2 = ih * ih;
     K.inv_h_f = ih;
     K.gk_c_f = 0.318309886183790671538f * ih2 * ih2 * ih;
+    const double dih = 1.0 / h0, C = dih * dih * dih * dih * (1.0 / PI);
+    K.u_inv_h = dih;
+    K.u_near0 = -3.0 * C * dih;
+    K.u_near1 = 2.25 * C * dih;
+    K.u_far = -0.75 * C;
   }
   // Alpha, Beta, mass, h or Cs written after the prologue: re-evaluate the
   // flags on the device columns (any order) and recapture the step with the

@@ -28,6 +28,8 @@
 // canonical order; a pair term is evaluated from the particle's own side
 // (x_i - x_j), which equals the reference's (min, max)-ordered pair value
 // with the reduction's sign applied.
+#include <type_traits>
+
 #include "wf_step_common.cuh"
 #include "wf_launch.h"
 
@@ -148,6 +150,35 @@ __device__ __forceinline__ PairGeo pair_geo(double xi0, double xi1, double xi2, 
   return g;
 }
 
+// FP64 instructions bound the plain form's gathers (GB300 issues one per 16
+// cycles and SM; 85-87 % of that rate before, with 71 of them per pair in the
+// acceleration, 15 in the density and 80 in the rates).  The uniform-particle
+// forms below (DomainConst::uni, no tensile term, no gradient correction) take
+// 39, 11 and 41: constants of the one h are formed on the host, compares read
+// the exponent word, the pair mass is a factor of the whole sum, and the nine
+// products v_k x_l are summed once instead of in symmetric and antisymmetric
+// parts.  Same FP64 throughout.
+struct UniGeo {
+  double r2, ir, GK;
+};
+__device__ __forceinline__ UniGeo uni_geo(const DomainConst& K, double x0, double x1, double x2) {
+  UniGeo g;
+  g.r2 = x0 * x0 + x1 * x1 + x2 * x2;
+  g.ir = g.r2 > 0.0 ? rsqrt(g.r2) : 0.0;
+  const double q = g.r2 * g.ir * K.u_inv_h;
+  const int hq = __double2hiint(q);  // q >= 0: its high word orders as q does (NaN above both bounds)
+  const double t = 2.0 - q;
+  const double near = K.u_near0 + K.u_near1 * q, far = (K.u_far * g.ir) * (t * t);
+  g.GK = hq < 0x3ff00000 ? near : (hq < 0x40000000 ? far : 0.0);
+  return g;
+}
+// Sum over the L lanes of a particle (all lanes end with it).
+template <int L>
+__device__ __forceinline__ double lane_sum(double v) {
+  for (int off = 1; off < L; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
+}
+
 // ---------------------------------------------------------------- tensile instability
 // StartAcceleration's TIR (Domain.cpp:1557-1569): TIR = V diag(f(L)) V^T for
 // the eigen-decomposition of Sigma, f(l) = -TI l / rho^2 for l > 0, else 0;
@@ -240,14 +271,9 @@ __device__ __forceinline__ void corr_grad(const DevPtrs& P, size_t N, int i, dou
 }
 
 // ---------------------------------------------------------------- accel
-__global__ void __launch_bounds__(BLOCK) k_accel(DevPtrs P, DomainConst K) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= K.N) return;
+// The pair sums of SPH particle i over row entries k0, k0 + dk, ...
+__device__ __forceinline__ void accel_sums(const DevPtrs& P, const DomainConst& K, int i, int k0, int dk, double out[3]) {
   size_t N = K.N;
-  if (icol(P, I_KIND, N, i) != 0) {  // StartAcceleration resets a for every particle
-    colw(P, C_A, N, i) = 0.0; colw(P, C_A + 1, N, i) = 0.0; colw(P, C_A + 2, N, i) = 0.0;
-    return;
-  }
   double xi0 = col(P, C_X, N, i), xi1 = col(P, C_X + 1, N, i), xi2 = col(P, C_X + 2, N, i);
   double vi0 = col(P, C_V, N, i), vi1 = col(P, C_V + 1, N, i), vi2 = col(P, C_V + 2, N, i);
   double hi = col(P, C_H, N, i), rhoi = col(P, C_RHO, N, i), csi = col(P, C_CS, N, i);
@@ -261,7 +287,7 @@ __global__ void __launch_bounds__(BLOCK) k_accel(DevPtrs P, DomainConst K) {
   // The last step's rate pass formed GradKernel at these positions and rows
   // unless this step searched (or the host touched the state).
   const bool reuse = P.st->gk_valid && !P.st->do_search;
-  for (int k = 0; k < len; ++k) {
+  for (int k = k0; k < len; k += dk) {
     int j = nb_index(P.nbr[(size_t)k * N + i]);
     PairGeo g;
     if (reuse) {
@@ -324,7 +350,74 @@ __global__ void __launch_bounds__(BLOCK) k_accel(DevPtrs P, DomainConst K) {
     a1 += g0 * S3 + g1 * S1 + g2 * S5;
     a2 += g0 * S4 + g1 * S5 + g2 * S2;
   }
-  colw(P, C_A, N, i) = a0; colw(P, C_A + 1, N, i) = a1; colw(P, C_A + 2, N, i) = a2;
+  out[0] = a0; out[1] = a1; out[2] = a2;
+}
+// Uniform particles: a = m (sum g S_j + S_i sum g + sum PI g), g = GK x_ij.
+__device__ __forceinline__ void accel_sums_uni(const DevPtrs& P, const DomainConst& K, int i, int k0, int dk,
+                                               double out[3]) {
+  const size_t N = K.N;
+  const double xi0 = col(P, C_X, N, i), xi1 = col(P, C_X + 1, N, i), xi2 = col(P, C_X + 2, N, i);
+  const double vi0 = col(P, C_V, N, i), vi1 = col(P, C_V + 1, N, i), vi2 = col(P, C_V + 2, N, i);
+  const double rhoi = col(P, C_RHO, N, i), h = col(P, C_H, N, i), cs = col(P, C_CS, N, i);
+  const double Alpha = col(P, C_ALPHA, N, i), Beta = col(P, C_BETA, N, i);
+  const bool visc = K.av_uniform ? Alpha != 0.0 || Beta != 0.0 : true;
+  const double eps = 0.01 * h * h;
+  double a0 = 0, a1 = 0, a2 = 0, G0 = 0, G1 = 0, G2 = 0;
+  const int len = P.row_len[i];
+  const bool reuse = P.st->gk_valid && !P.st->do_search;  // as in accel_sums
+  int next = k0 < len ? P.nbr[(size_t)k0 * N + i] : 0;
+  for (int k = k0; k < len; k += dk) {
+    const int j = nb_index(next);
+    if (k + dk < len) next = P.nbr[(size_t)(k + dk) * N + i];
+    const double x0 = xi0 - col(P, C_X, N, j), x1 = xi1 - col(P, C_X + 1, N, j), x2 = xi2 - col(P, C_X + 2, N, j);
+    double GK;
+    if (reuse) {
+      GK = P.gk[(size_t)k * N + i];
+    } else {
+      GK = uni_geo(K, x0, x1, x2).GK;
+      P.gk[(size_t)k * N + i] = GK;  // for the density pass (same x(n), h)
+    }
+    const double g0 = GK * x0, g1 = GK * x1, g2 = GK * x2;
+    if (visc) {
+      const double dvx = (vi0 - col(P, C_V, N, j)) * x0 + (vi1 - col(P, C_V + 1, N, j)) * x1 + (vi2 - col(P, C_V + 2, N, j)) * x2;
+      if (__double2hiint(dvx) < 0) {  // the sign (-0 adds nothing): MU (alpha C + beta MU) / rho_bar, MU = h dvx / Dn
+        const double al = K.av_uniform ? Alpha : 0.5 * (Alpha + col(P, C_ALPHA, N, j));
+        const double be = K.av_uniform ? Beta : 0.5 * (Beta + col(P, C_BETA, N, j));
+        const double Dn = eps + x0 * x0 + x1 * x1 + x2 * x2;
+        const double hv = h * dvx, rs = rhoi + col(P, C_RHO, N, j);
+        double num = 2.0 * hv * (al * cs), den = Dn * rs;
+        if (be != 0.0) { num = 2.0 * hv * (al * cs * Dn + be * hv); den *= Dn; }
+        const double PIs = num / den;
+        a0 += PIs * g0; a1 += PIs * g1; a2 += PIs * g2;
+      }
+    }
+    G0 += g0; G1 += g1; G2 += g2;
+    const double S3 = col(P, C_SRHO + 3, N, j), S4 = col(P, C_SRHO + 4, N, j), S5 = col(P, C_SRHO + 5, N, j);
+    a0 += g0 * col(P, C_SRHO, N, j) + g1 * S3 + g2 * S4;
+    a1 += g0 * S3 + g1 * col(P, C_SRHO + 1, N, j) + g2 * S5;
+    a2 += g0 * S4 + g1 * S5 + g2 * col(P, C_SRHO + 2, N, j);
+  }
+  const double m = col(P, C_MASS, N, i);
+  const double T3 = col(P, C_SRHO + 3, N, i), T4 = col(P, C_SRHO + 4, N, i), T5 = col(P, C_SRHO + 5, N, i);
+  out[0] = m * (a0 + (G0 * col(P, C_SRHO, N, i) + G1 * T3 + G2 * T4));
+  out[1] = m * (a1 + (G0 * T3 + G1 * col(P, C_SRHO + 1, N, i) + G2 * T5));
+  out[2] = m * (a2 + (G0 * T4 + G1 * T5 + G2 * col(P, C_SRHO + 2, N, i)));
+}
+// L lanes per particle: with one, a small domain's few warps wait out each
+// other's FP64 latency (8,004 particles: two warps per SM).
+template <bool UNI, int L>
+__global__ void __launch_bounds__(512) k_accel(DevPtrs P, DomainConst K) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / L, sub = t % L;
+  const size_t N = K.N;
+  const bool live = i < K.N;
+  double a[3] = {0.0, 0.0, 0.0};  // StartAcceleration resets a for every particle
+  if (live && icol(P, I_KIND, N, i) == 0) {
+    if (UNI) accel_sums_uni(P, K, i, sub, L, a);
+    else accel_sums(P, K, i, sub, L, a);
+  }
+  if (L > 1) for (int d = 0; d < 3; ++d) a[d] = lane_sum<L>(a[d]);
+  if (live && sub == 0)
+    for (int d = 0; d < 3; ++d) colw(P, C_A + d, N, i) = a[d];
 }
 
 // ---------------------------------------------------------------- BCs
@@ -672,44 +765,63 @@ __global__ void __launch_bounds__(BLOCK) k_contact_kick(DevPtrs P, DomainConst K
 }
 
 // ---------------------------------------------------------------- density + drift + kick
-__global__ void __launch_bounds__(BLOCK) k_density_drift(DevPtrs P, DomainConst K) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= K.N) return;
-  size_t N = K.N;
-  double dt = P.st->deltat;
-  double xi0 = col(P, C_X, N, i), xi1 = col(P, C_X + 1, N, i), xi2 = col(P, C_X + 2, N, i);
-  double vi0 = col(P, C_V, N, i), vi1 = col(P, C_V + 1, N, i), vi2 = col(P, C_V + 2, N, i);
-  double rhoi = col(P, C_RHO, N, i);
+// rho_i dot / rho_i (with gradient correction: rho dot) over entries k0, k0 + dk, ...
+__device__ __forceinline__ double density_sum(const DevPtrs& P, const DomainConst& K, int i, int k0, int dk) {
+  const size_t N = K.N;
+  const double xi0 = col(P, C_X, N, i), xi1 = col(P, C_X + 1, N, i), xi2 = col(P, C_X + 2, N, i);
+  const double vi0 = col(P, C_V, N, i), vi1 = col(P, C_V + 1, N, i), vi2 = col(P, C_V + 2, N, i);
+  const double rhoi = col(P, C_RHO, N, i);
   double dd = 0.0;
-  if (P.tx) {
-    P.tx[(size_t)(TX_VH + 0) * N + i] = vi0; P.tx[(size_t)(TX_VH + 1) * N + i] = vi1;
-    P.tx[(size_t)(TX_VH + 2) * N + i] = vi2;
-  }
-  if (icol(P, I_KIND, N, i) == 0) {
-    int len = P.row_len[i];
-    for (int k = 0; k < len; ++k) {
-      int j = nb_index(P.nbr[(size_t)k * N + i]);
-      // x(n) and h are the acceleration pass's: its GradKernel of this entry is reused
-      PairGeo g;
-      g.x0 = xi0 - col(P, C_X, N, j); g.x1 = xi1 - col(P, C_X + 1, N, j); g.x2 = xi2 - col(P, C_X + 2, N, j);
-      g.GK = P.gk[(size_t)k * N + i];
-      double v0 = vi0 - col(P, C_V, N, j), v1 = vi1 - col(P, C_V + 1, N, j), v2 = vi2 - col(P, C_V + 2, N, j);
-      if (K.gradcorr) {  // locking form m_j (rho_i/rho_j) v_ij . vc_i (InteractionAlt.cpp:589-605)
-        double vc[3];
-        corr_grad(P, N, i, g.GK, g.x0, g.x1, g.x2, vc);
-        double t1 = v0 * vc[0] + v1 * vc[1] + v2 * vc[2];
-        dd += col(P, C_MASS, N, j) * (rhoi / col(P, C_RHO, N, j)) * t1;
-        continue;
-      }
-      double pd = v0 * (g.GK * g.x0) + v1 * (g.GK * g.x1) + v2 * (g.GK * g.x2);
-      dd += col(P, C_MRHO, N, j) * pd;
+  const int len = P.row_len[i];
+  int next = k0 < len ? P.nbr[(size_t)k0 * N + i] : 0;
+  for (int k = k0; k < len; k += dk) {
+    const int j = nb_index(next);
+    if (k + dk < len) next = P.nbr[(size_t)(k + dk) * N + i];
+    // x(n) and h are the acceleration pass's: its GradKernel of this entry is reused
+    const double GK = P.gk[(size_t)k * N + i];
+    const double x0 = xi0 - col(P, C_X, N, j), x1 = xi1 - col(P, C_X + 1, N, j), x2 = xi2 - col(P, C_X + 2, N, j);
+    const double v0 = vi0 - col(P, C_V, N, j), v1 = vi1 - col(P, C_V + 1, N, j), v2 = vi2 - col(P, C_V + 2, N, j);
+    if (K.gradcorr) {  // locking form m_j (rho_i/rho_j) v_ij . vc_i (InteractionAlt.cpp:589-605)
+      double vc[3];
+      corr_grad(P, N, i, GK, x0, x1, x2, vc);
+      dd += col(P, C_MASS, N, j) * (rhoi / col(P, C_RHO, N, j)) * (v0 * vc[0] + v1 * vc[1] + v2 * vc[2]);
+    } else {
+      dd += (col(P, C_MRHO, N, j) * GK) * (v0 * x0 + v1 * x1 + v2 * x2);
     }
-    if (!K.gradcorr) dd *= rhoi;
   }
+  return dd;
+}
+// L lanes per particle; the lanes' sums go through shared memory, so that the
+// first blockDim / L threads finish a particle each in full warps.
+template <int L>
+__global__ void __launch_bounds__(512) k_density_drift(DevPtrs P, DomainConst K) {
+  __shared__ double s_dd[L > 1 ? 256 : 1];
+  const int PB = blockDim.x / L;  // particles per block
+  const size_t N = K.N;
+  int i = blockIdx.x * PB + threadIdx.x / L;
+  double dd = 0.0;
+  if (i < K.N && icol(P, I_KIND, N, i) == 0) dd = density_sum(P, K, i, threadIdx.x % L, L);
+  if (L > 1) {
+    dd = lane_sum<L>(dd);
+    if (threadIdx.x % L == 0) s_dd[threadIdx.x / L] = dd;
+    __syncthreads();
+    if (threadIdx.x >= PB) return;
+    dd = s_dd[threadIdx.x];
+    i = blockIdx.x * PB + threadIdx.x;
+  }
+  if (i >= K.N) return;
+  const double dt = P.st->deltat;
+  const double rhoi = col(P, C_RHO, N, i);
+  const bool solid = icol(P, I_KIND, N, i) == 0;
+  double v[3], x[3];
+  for (int d = 0; d < 3; ++d) { v[d] = col(P, C_V + d, N, i); x[d] = col(P, C_X + d, N, i); }
+  if (P.tx)
+    for (int d = 0; d < 3; ++d) P.tx[(size_t)(TX_VH + d) * N + i] = v[d];
+  if (solid && !K.gradcorr) dd *= rhoi;
   colw(P, C_DRHO, N, i) = dd;
   double rn = rhoi + dt * dd;
   colw(P, C_RHON, N, i) = rn;
-  colw(P, C_MRHON, N, i) = icol(P, I_KIND, N, i) == 0 ? col(P, C_MASS, N, i) / rn : 0.0;
+  colw(P, C_MRHON, N, i) = solid ? col(P, C_MASS, N, i) / rn : 0.0;
   // Next-step pressure over density^2 (EOS case 0 of the updated density, the
   // expression the stress update evaluates) and next-step temperature
   // (Thermal.cpp:727-734): the fused rate gather reads both for neighbours.
@@ -719,7 +831,6 @@ __global__ void __launch_bounds__(BLOCK) k_density_drift(DevPtrs P, DomainConst 
     colw(P, C_PR2N, N, i) = pn / (rn * rn);
     if (K.thermal_solver) colw(P, C_TN, N, i) = col(P, C_T, N, i) + dt * col(P, C_DTDT, N, i);
   }
-  double v[3] = {vi0, vi1, vi2}, x[3] = {xi0, xi1, xi2};
   // GeneralAfter on the next-step velocity (SolverKickDrift.cpp:267) applied
   // here instead of in a BC pass after this kernel
   double vb[3];
@@ -748,92 +859,179 @@ __global__ void k_kick_leapfrog(DevPtrs P, DomainConst K) {
 }
 
 // ---------------------------------------------------------------- rate + stress
-__global__ void __launch_bounds__(BLOCK) k_rate_stress(DevPtrs P, DomainConst K) {
-  __shared__ double sh[32];
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+// The rate sums of SPH particle i (strain rate xx yy zz xy xz yz, rotation
+// rate xy xz yz, kinetic-energy sum, conduction sum) over entries k0, k0 + dk, ...
+struct Rates {
+  double sr[6] = {0, 0, 0, 0, 0, 0}, rr[3] = {0, 0, 0}, dkin = 0.0, cond = 0.0;
+};
+__device__ __forceinline__ void rate_sums(const DevPtrs& P, const DomainConst& K, int i, int k0, int dk, Rates& R) {
+  const size_t N = K.N;
+  double x[3], v[3];
+  for (int d = 0; d < 3; ++d) { x[d] = col(P, C_XN + d, N, i); v[d] = col(P, C_VN + d, N, i); }
+  double hi = col(P, C_H, N, i);
+  double inv_hi = 1.0 / hi;
+  double (&sr)[6] = R.sr;
+  double (&rr)[3] = R.rr;
+  // CalcKinEnergyEqn and CalcTempInc pair sums, on the same positions and
+  // velocities as the rates (Domain.cpp:1752-1808, Thermal.cpp:53-219)
+  double dkin = 0.0, cond = 0.0;
+  double massi = col(P, C_MASS, N, i), mrhoi = col(P, C_MRHON, N, i), pri = col(P, C_PR2N, N, i);
+  double Ti = 0.0, ki = 0.0;
+  if (K.thermal_solver) { Ti = col(P, C_TN, N, i); ki = col(P, C_KT, N, i); }
+  int len = P.row_len[i];
+  for (int k = k0; k < len; k += dk) {
+    int e = P.nbr[(size_t)k * N + i];
+    int j = nb_index(e);
+    PairGeo g = pair_geo(x[0], x[1], x[2], hi, inv_hi, col(P, C_XN, N, j), col(P, C_XN + 1, N, j), col(P, C_XN + 2, N, j),
+                         col(P, C_H, N, j));
+    P.gk[(size_t)k * N + i] = g.GK;  // x(n+1) is the next step's x(n): its acceleration pass reuses it
+    double b0 = v[0] - col(P, C_VN, N, j), b1 = v[1] - col(P, C_VN + 1, N, j), b2 = v[2] - col(P, C_VN + 2, N, j);
+    {
+      double dv = g.GK * (b0 * g.x0 + b1 * g.x1 + b2 * g.x2);
+      bool up = nb_up(e);  // original index of j larger than i's
+      // pair (P1 = smaller original index): 0.5 m_P2 (p1/d1^2 + p2/d2^2) v12.(GK x12)
+      double pk = 0.5 * (up ? col(P, C_MASS, N, j) : massi) * (pri + col(P, C_PR2N, N, j)) * dv;
+      dkin += up ? pk : -pk;
+      if (K.thermal_solver) {
+        double kj = col(P, C_KT, N, j);
+        double w = up ? col(P, C_MRHON, N, j) : mrhoi;  // m_P2 / rho_P2 for both ends
+        double gx[3] = {g.GK * g.x0, g.GK * g.x1, g.GK * g.x2};
+        if (K.gradcorr) {  // Mult(gradCorrM_i, GK x_ij) (Thermal.cpp:90-107)
+          double c3[3];
+          for (int q = 0; q < 3; ++q)
+            c3[q] = gx[0] * col(P, C_GCM + 3 * q, N, i) + gx[1] * col(P, C_GCM + 3 * q + 1, N, i) +
+                    gx[2] * col(P, C_GCM + 3 * q + 2, N, i);
+          gx[0] = c3[0]; gx[1] = c3[1]; gx[2] = c3[2];
+        }
+        double dxx = g.x0 * gx[0] + g.x1 * gx[1] + g.x2 * gx[2];
+        cond += w * 4. * (ki * kj) / (ki + kj) * (Ti - col(P, C_TN, N, j)) * dxx / (g.r * g.r);
+      }
+    }
+    if (K.gradcorr) {  // locking form: (float)(m_j/rho_j) with v_ij (x) vc_i (InteractionAlt.cpp:330-350, 425-450)
+      double gk[3];
+      corr_grad(P, N, i, g.GK, g.x0, g.x1, g.x2, gk);
+      double bv[3] = {b0, b1, b2};
+      double wf = (double)(float)(col(P, C_MASS, N, j) / col(P, C_RHON, N, j));
+      const int ua[6] = {0, 1, 2, 0, 0, 1}, ub[6] = {0, 1, 2, 1, 2, 2};
+      for (int c = 0; c < 6; ++c) {
+        double gab = bv[ua[c]] * gk[ub[c]], gba = bv[ub[c]] * gk[ua[c]];
+        sr[c] += wf * (-0.5 * (gab + gba));
+      }
+      rr[0] += wf * (-0.5 * (bv[0] * gk[1] - bv[1] * gk[0]));
+      rr[1] += wf * (-0.5 * (bv[0] * gk[2] - bv[2] * gk[0]));
+      rr[2] += wf * (-0.5 * (bv[1] * gk[2] - bv[2] * gk[1]));
+      continue;
+    }
+    // (m_j/rho_j) (-GK/2) (v_ij (x) x_ij +- x_ij (x) v_ij): u = (m_j/rho_j)(-GK/2) v_ij
+    // enters every entry; the diagonal collects u_a x_a and is doubled once
+    // after the loop (exact in binary).
+    double wf = col(P, C_MRHON, N, j) * (-0.5 * g.GK);
+    double u0 = wf * b0, u1 = wf * b1, u2 = wf * b2;
+    sr[0] += u0 * g.x0;
+    sr[1] += u1 * g.x1;
+    sr[2] += u2 * g.x2;
+    sr[3] += u0 * g.x1; sr[3] += u1 * g.x0;
+    sr[4] += u0 * g.x2; sr[4] += u2 * g.x0;
+    sr[5] += u1 * g.x2; sr[5] += u2 * g.x1;
+    rr[0] += u0 * g.x1; rr[0] -= u1 * g.x0;
+    rr[1] += u0 * g.x2; rr[1] -= u2 * g.x0;
+    rr[2] += u1 * g.x2; rr[2] -= u2 * g.x1;
+  }
+  if (!K.gradcorr)
+    for (int c = 0; c < 3; ++c) sr[c] = 2.0 * sr[c];
+  R.dkin = dkin; R.cond = cond;
+}
+// The same for uniform particles without gradient correction.
+__device__ __forceinline__ void rate_sums_uni(const DevPtrs& P, const DomainConst& K, int i, int k0, int dk, Rates& R) {
+  const size_t N = K.N;
+  const double xi0 = col(P, C_XN, N, i), xi1 = col(P, C_XN + 1, N, i), xi2 = col(P, C_XN + 2, N, i);
+  const double vi0 = col(P, C_VN, N, i), vi1 = col(P, C_VN + 1, N, i), vi2 = col(P, C_VN + 2, N, i);
+  const double pri = col(P, C_PR2N, N, i);
+  double Ti = 0.0, ki = 0.0, mrhoi = 0.0;
+  if (K.thermal_solver) { Ti = col(P, C_TN, N, i); ki = col(P, C_KT, N, i); mrhoi = col(P, C_MRHON, N, i); }
+  double M[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // sum (m_j / rho_j) GK v_k x_l
+  double dkin = 0.0, cond = 0.0;
+  const int len = P.row_len[i];
+  int next = k0 < len ? P.nbr[(size_t)k0 * N + i] : 0;
+  for (int k = k0; k < len; k += dk) {
+    const int e = next, j = nb_index(e);
+    if (k + dk < len) next = P.nbr[(size_t)(k + dk) * N + i];
+    const double x0 = xi0 - col(P, C_XN, N, j), x1 = xi1 - col(P, C_XN + 1, N, j), x2 = xi2 - col(P, C_XN + 2, N, j);
+    const double b0 = vi0 - col(P, C_VN, N, j), b1 = vi1 - col(P, C_VN + 1, N, j), b2 = vi2 - col(P, C_VN + 2, N, j);
+    const double mrhoj = col(P, C_MRHON, N, j);
+    const UniGeo g = uni_geo(K, x0, x1, x2);
+    P.gk[(size_t)k * N + i] = g.GK;  // x(n+1) is the next step's x(n): its acceleration pass reuses it
+    const double pk = (pri + col(P, C_PR2N, N, j)) * (g.GK * (b0 * x0 + b1 * x1 + b2 * x2));
+    // pair (P1 = smaller original index): added to P1, subtracted from P2
+    dkin += __hiloint2double(__double2hiint(pk) ^ (int)(~(unsigned)e & NB_UP), __double2loint(pk));
+    const double w = mrhoj * g.GK;
+    const double u0 = w * b0, u1 = w * b1, u2 = w * b2;
+    M[0] += u0 * x0; M[1] += u0 * x1; M[2] += u0 * x2;
+    M[3] += u1 * x0; M[4] += u1 * x1; M[5] += u1 * x2;
+    M[6] += u2 * x0; M[7] += u2 * x1; M[8] += u2 * x2;
+    if (K.thermal_solver) {
+      // 4 ki kj / (ki + kj) (Ti - Tj) x.(GK x) / r^2 with x.x = r^2; the
+      // reference's 0/0 of coincident particles stays a NaN
+      const double kj = col(P, C_KT, N, j);
+      const double c = kj == ki ? ki + ki : 4. * (ki * kj) / (ki + kj);
+      const double gr = g.r2 > 0.0 ? g.GK : __longlong_as_double(0x7ff8000000000000ll);
+      cond += (nb_up(e) ? mrhoj : mrhoi) * c * (Ti - col(P, C_TN, N, j)) * gr;  // m_P2 / rho_P2 for both ends
+    }
+  }
+  R.dkin = 0.5 * col(P, C_MASS, N, i) * dkin;
+  R.cond = cond;
+  R.sr[0] = -M[0]; R.sr[1] = -M[4]; R.sr[2] = -M[8];
+  R.sr[3] = -0.5 * (M[1] + M[3]); R.sr[4] = -0.5 * (M[2] + M[6]); R.sr[5] = -0.5 * (M[5] + M[7]);
+  R.rr[0] = -0.5 * (M[1] - M[3]); R.rr[1] = -0.5 * (M[2] - M[6]); R.rr[2] = -0.5 * (M[5] - M[7]);
+}
+// L lanes per particle in the gather; the lanes' sums go through shared memory,
+// so that the first blockDim / L threads update a particle each in full warps
+// (the update is ~270 FP64 instructions, as many as a lane's share of a row).
+template <bool UNI, int L>
+__global__ void __launch_bounds__(L > 1 ? 512 : BLOCK) k_rate_stress(DevPtrs P, DomainConst K) {
+  __shared__ double sh[6 * 32];
+  __shared__ double s_r[L > 1 ? 11 : 1][L > 1 ? 256 : 1];
+  const int PB = blockDim.x / L;  // particles per block
   size_t N = K.N;
   double dt = P.st->deltat;
   double plw = 0.0, maxpl = 0.0, maxT = -1e300, minT = 1e300, dkin_b = 0.0, dint = 0.0;
+  Rates R;
+  int i = blockIdx.x * PB + threadIdx.x / L;
+  if (i < K.N && icol(P, I_KIND, N, i) == 0) {
+    if (UNI) rate_sums_uni(P, K, i, threadIdx.x % L, L, R);
+    else rate_sums(P, K, i, threadIdx.x % L, L, R);
+  }
+  if constexpr (L > 1) {
+    const int p = threadIdx.x / L;
+    auto put = [&](int q, double v) {
+      v = lane_sum<L>(v);
+      if (threadIdx.x % L == 0) s_r[q][p] = v;
+    };
+    for (int c = 0; c < 6; ++c) put(c, R.sr[c]);
+    for (int c = 0; c < 3; ++c) put(6 + c, R.rr[c]);
+    put(9, R.dkin);
+    if (K.thermal_solver) put(10, R.cond);
+    __syncthreads();
+    i = threadIdx.x < PB ? blockIdx.x * PB + threadIdx.x : K.N;
+    if (i < K.N) {
+      for (int c = 0; c < 6; ++c) R.sr[c] = s_r[c][threadIdx.x];
+      for (int c = 0; c < 3; ++c) R.rr[c] = s_r[6 + c][threadIdx.x];
+      R.dkin = s_r[9][threadIdx.x];
+      if (K.thermal_solver) R.cond = s_r[10][threadIdx.x];
+    }
+  }
+  double (&sr)[6] = R.sr;
+  double (&rr)[3] = R.rr;
   if (i < K.N) {
     // Next-step buffers become the current state for this particle.
-    double x[3], v[3];
-    for (int d = 0; d < 3; ++d) { x[d] = col(P, C_XN + d, N, i); v[d] = col(P, C_VN + d, N, i); }
+    for (int d = 0; d < 3; ++d) { colw(P, C_X + d, N, i) = col(P, C_XN + d, N, i); colw(P, C_V + d, N, i) = col(P, C_VN + d, N, i); }
     double rho = col(P, C_RHON, N, i);
-    for (int d = 0; d < 3; ++d) { colw(P, C_X + d, N, i) = x[d]; colw(P, C_V + d, N, i) = v[d]; }
+    const double mrhoi = col(P, C_MRHON, N, i);
     colw(P, C_RHO, N, i) = rho;
-    colw(P, C_MRHO, N, i) = col(P, C_MRHON, N, i);
+    colw(P, C_MRHO, N, i) = mrhoi;
     maxpl = col(P, C_PLS, N, i);
     if (icol(P, I_KIND, N, i) == 0) {
-      double hi = col(P, C_H, N, i);
-      double inv_hi = 1.0 / hi;
-      double sr[6] = {0, 0, 0, 0, 0, 0}, rr[3] = {0, 0, 0};
-      // CalcKinEnergyEqn and CalcTempInc pair sums, on the same positions and
-      // velocities as the rates (Domain.cpp:1752-1808, Thermal.cpp:53-219)
-      double dkin = 0.0, cond = 0.0;
-      double massi = col(P, C_MASS, N, i), mrhoi = col(P, C_MRHON, N, i), pri = col(P, C_PR2N, N, i);
-      double Ti = 0.0, ki = 0.0;
-      if (K.thermal_solver) { Ti = col(P, C_TN, N, i); ki = col(P, C_KT, N, i); }
-      int len = P.row_len[i];
-      for (int k = 0; k < len; ++k) {
-        int e = P.nbr[(size_t)k * N + i];
-        int j = nb_index(e);
-        PairGeo g = pair_geo(x[0], x[1], x[2], hi, inv_hi, col(P, C_XN, N, j), col(P, C_XN + 1, N, j), col(P, C_XN + 2, N, j),
-                             col(P, C_H, N, j));
-        P.gk[(size_t)k * N + i] = g.GK;  // x(n+1) is the next step's x(n): its acceleration pass reuses it
-        double b0 = v[0] - col(P, C_VN, N, j), b1 = v[1] - col(P, C_VN + 1, N, j), b2 = v[2] - col(P, C_VN + 2, N, j);
-        {
-          double dv = g.GK * (b0 * g.x0 + b1 * g.x1 + b2 * g.x2);
-          bool up = nb_up(e);  // original index of j larger than i's
-          // pair (P1 = smaller original index): 0.5 m_P2 (p1/d1^2 + p2/d2^2) v12.(GK x12)
-          double pk = 0.5 * (up ? col(P, C_MASS, N, j) : massi) * (pri + col(P, C_PR2N, N, j)) * dv;
-          dkin += up ? pk : -pk;
-          if (K.thermal_solver) {
-            double kj = col(P, C_KT, N, j);
-            double w = up ? col(P, C_MRHON, N, j) : mrhoi;  // m_P2 / rho_P2 for both ends
-            double gx[3] = {g.GK * g.x0, g.GK * g.x1, g.GK * g.x2};
-            if (K.gradcorr) {  // Mult(gradCorrM_i, GK x_ij) (Thermal.cpp:90-107)
-              double c3[3];
-              for (int q = 0; q < 3; ++q)
-                c3[q] = gx[0] * col(P, C_GCM + 3 * q, N, i) + gx[1] * col(P, C_GCM + 3 * q + 1, N, i) +
-                        gx[2] * col(P, C_GCM + 3 * q + 2, N, i);
-              gx[0] = c3[0]; gx[1] = c3[1]; gx[2] = c3[2];
-            }
-            double dxx = g.x0 * gx[0] + g.x1 * gx[1] + g.x2 * gx[2];
-            cond += w * 4. * (ki * kj) / (ki + kj) * (Ti - col(P, C_TN, N, j)) * dxx / (g.r * g.r);
-          }
-        }
-        if (K.gradcorr) {  // locking form: (float)(m_j/rho_j) with v_ij (x) vc_i (InteractionAlt.cpp:330-350, 425-450)
-          double gk[3];
-          corr_grad(P, N, i, g.GK, g.x0, g.x1, g.x2, gk);
-          double bv[3] = {b0, b1, b2};
-          double wf = (double)(float)(col(P, C_MASS, N, j) / col(P, C_RHON, N, j));
-          const int ua[6] = {0, 1, 2, 0, 0, 1}, ub[6] = {0, 1, 2, 1, 2, 2};
-          for (int c = 0; c < 6; ++c) {
-            double gab = bv[ua[c]] * gk[ub[c]], gba = bv[ub[c]] * gk[ua[c]];
-            sr[c] += wf * (-0.5 * (gab + gba));
-          }
-          rr[0] += wf * (-0.5 * (bv[0] * gk[1] - bv[1] * gk[0]));
-          rr[1] += wf * (-0.5 * (bv[0] * gk[2] - bv[2] * gk[0]));
-          rr[2] += wf * (-0.5 * (bv[1] * gk[2] - bv[2] * gk[1]));
-          continue;
-        }
-        // (m_j/rho_j) (-GK/2) (v_ij (x) x_ij +- x_ij (x) v_ij): u = (m_j/rho_j)(-GK/2) v_ij
-        // enters every entry; the diagonal collects u_a x_a and is doubled once
-        // after the loop (exact in binary).
-        double wf = col(P, C_MRHON, N, j) * (-0.5 * g.GK);
-        double u0 = wf * b0, u1 = wf * b1, u2 = wf * b2;
-        sr[0] += u0 * g.x0;
-        sr[1] += u1 * g.x1;
-        sr[2] += u2 * g.x2;
-        sr[3] += u0 * g.x1; sr[3] += u1 * g.x0;
-        sr[4] += u0 * g.x2; sr[4] += u2 * g.x0;
-        sr[5] += u1 * g.x2; sr[5] += u2 * g.x1;
-        rr[0] += u0 * g.x1; rr[0] -= u1 * g.x0;
-        rr[1] += u0 * g.x2; rr[1] -= u2 * g.x0;
-        rr[2] += u1 * g.x2; rr[2] -= u2 * g.x1;
-      }
-      if (!K.gradcorr)
-        for (int c = 0; c < 3; ++c) sr[c] = 2.0 * sr[c];
+      const double dkin = R.dkin, cond = R.cond;
       StressIO s;
       for (int c = 0; c < 6; ++c) {
         s.tau[c] = col(P, C_TAU + c, N, i); s.eps[c] = col(P, C_EPS + c, N, i);
@@ -895,15 +1093,9 @@ __global__ void __launch_bounds__(BLOCK) k_rate_stress(DevPtrs P, DomainConst K)
       dkin_b = dkin;
     }
   }
-  double r;
-  r = block_reduce<0>(dkin_b, sh); if (threadIdx.x == 0) P.partials[S_DKIN * K.nblocks + blockIdx.x] = r;
-  r = block_reduce<0>(dint, sh); if (threadIdx.x == 0) P.partials[S_DINT * K.nblocks + blockIdx.x] = r;
-  r = block_reduce<1>(maxpl, sh); if (threadIdx.x == 0) P.partials[S_MAXPL * K.nblocks + blockIdx.x] = r;
-  if (K.pl_heating) { r = block_reduce<0>(plw, sh); if (threadIdx.x == 0) P.partials[S_PLW * K.nblocks + blockIdx.x] = r; }
-  if (K.thermal_solver) {
-    r = block_reduce<1>(maxT, sh); if (threadIdx.x == 0) P.partials[S_MAXT * K.nblocks + blockIdx.x] = r;
-    r = block_reduce<2>(minT, sh); if (threadIdx.x == 0) P.partials[S_MINT * K.nblocks + blockIdx.x] = r;
-  }
+  auto part = [&](int slot) { return P.partials + (size_t)slot * K.nblocks + blockIdx.x; };
+  double* const o[6] = {part(S_DKIN), part(S_DINT), part(S_PLW), part(S_MAXPL), part(S_MAXT), part(S_MINT)};
+  block_reduce_all<3, true>({dkin_b, dint, plw}, maxpl, maxT, minT, sh, o);
 }
 
 
@@ -1252,17 +1444,45 @@ void launch_tensile(const DevPtrs& P, const DomainConst& K, cudaStream_t s) {
   mark(s, "k_tensile");
 }
 
+template <bool UNI, int L>
+static void launch_accel64(const DevPtrs& P, const DomainConst& K, cudaStream_t s) {
+  k_accel<UNI, L><<<K.nblocks, K.pblock * L, 0, s>>>(P, K);
+}
+template <bool UNI, int L>
+static void launch_rate64(const DevPtrs& P, const DomainConst& K, cudaStream_t s) {
+  k_rate_stress<UNI, L><<<K.nblocks, K.pblock * L, 0, s>>>(P, K);
+}
 void launch_step_fp64_body(const DevPtrs& P, const DomainConst& K, cudaStream_t s) {
-  int nb = K.nblocks;
+  // lanes per particle within blocks of at most 512 threads
+  const int L = K.lanes64 > 1 && K.pblock * K.lanes64 <= 512 ? K.lanes64 : 1;
+  const bool uni_a = K.uni && !K.ti && !K.gradcorr, uni_r = K.uni && !K.gradcorr;
+  auto with_lanes = [&](auto f) {
+    switch (L) {
+      case 2: f(std::integral_constant<int, 2>{}); break;
+      case 4: f(std::integral_constant<int, 4>{}); break;
+      default: f(std::integral_constant<int, 1>{});
+    }
+  };
   launch_tensile(P, K, s);
-  k_accel<<<nb, K.pblock, 0, s>>>(P, K);
+  with_lanes([&](auto l) {
+    constexpr int LL = decltype(l)::value;
+    if (uni_a) launch_accel64<true, LL>(P, K, s);
+    else launch_accel64<false, LL>(P, K, s);
+  });
   mark(s, "k_accel");
   launch_bc(P, K, C_V, s);
   launch_contact_kick(P, K, s);
   if (K.leapfrog) launch_bc(P, K, C_V, s);  // kick-drift: applied by the kick kernel
-  k_density_drift<<<nb, K.pblock, 0, s>>>(P, K);  // and the next-step BC by this one
+  with_lanes([&](auto l) {  // and the next-step BC by this one
+    constexpr int LL = decltype(l)::value;
+    k_density_drift<LL><<<K.nblocks, K.pblock * LL, 0, s>>>(P, K);
+  });
   mark(s, "k_density_drift");
-  k_rate_stress<<<nb, K.pblock, 0, s>>>(P, K);
+  with_lanes([&](auto l) {
+    constexpr int LL = decltype(l)::value;
+    if (uni_r) launch_rate64<true, LL>(P, K, s);
+    else launch_rate64<false, LL>(P, K, s);
+  });
   mark(s, "k_rate_stress");
   launch_step_tail(P, K, s);
 }
