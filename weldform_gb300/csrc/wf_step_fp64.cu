@@ -161,14 +161,16 @@ __device__ __forceinline__ PairGeo pair_geo(double xi0, double xi1, double xi2, 
 struct UniGeo {
   double r2, ir, GK;
 };
+// Explicit roundings: the rate pass's value and the acceleration pass's own (after
+// a rewind or a search) are the same bits whatever surrounds the call.
 __device__ __forceinline__ UniGeo uni_geo(const DomainConst& K, double x0, double x1, double x2) {
   UniGeo g;
-  g.r2 = x0 * x0 + x1 * x1 + x2 * x2;
+  g.r2 = fma(x2, x2, fma(x1, x1, __dmul_rn(x0, x0)));
   g.ir = g.r2 > 0.0 ? rsqrt(g.r2) : 0.0;
-  const double q = g.r2 * g.ir * K.u_inv_h;
+  const double q = __dmul_rn(__dmul_rn(g.r2, g.ir), K.u_inv_h);
   const int hq = __double2hiint(q);  // q >= 0: its high word orders as q does (NaN above both bounds)
-  const double t = 2.0 - q;
-  const double near = K.u_near0 + K.u_near1 * q, far = (K.u_far * g.ir) * (t * t);
+  const double t = __dsub_rn(2.0, q);
+  const double near = fma(K.u_near1, q, K.u_near0), far = __dmul_rn(__dmul_rn(K.u_far, g.ir), __dmul_rn(t, t));
   g.GK = hq < 0x3ff00000 ? near : (hq < 0x40000000 ? far : 0.0);
   return g;
 }
@@ -287,16 +289,18 @@ __device__ __forceinline__ void accel_sums(const DevPtrs& P, const DomainConst& 
   // The last step's rate pass formed GradKernel at these positions and rows
   // unless this step searched (or the host touched the state).
   const bool reuse = P.st->gk_valid && !P.st->do_search;
+  const bool uni = K.uni && !K.gradcorr;  // the rate pass then forms GradKernel by uni_geo: so does this one
   for (int k = k0; k < len; k += dk) {
     int j = nb_index(P.nbr[(size_t)k * N + i]);
     PairGeo g;
-    if (reuse) {
+    if (reuse || uni) {
       double hj = col(P, C_H, N, j);
       g.x0 = xi0 - col(P, C_X, N, j); g.x1 = xi1 - col(P, C_X + 1, N, j); g.x2 = xi2 - col(P, C_X + 2, N, j);
       g.r2 = g.x0 * g.x0 + g.x1 * g.x1 + g.x2 * g.x2;
       g.hh = hj == hi ? hi : (hi + hj) / 2;
       g.r = K.ti ? sqrt(g.r2) : 0.0;  // the tensile term alone needs r
-      g.GK = P.gk[(size_t)k * N + i];
+      if (reuse) g.GK = P.gk[(size_t)k * N + i];
+      else P.gk[(size_t)k * N + i] = g.GK = uni_geo(K, g.x0, g.x1, g.x2).GK;
     } else {
       g = pair_geo(xi0, xi1, xi2, hi, inv_hi, col(P, C_X, N, j), col(P, C_X + 1, N, j), col(P, C_X + 2, N, j),
                    col(P, C_H, N, j));

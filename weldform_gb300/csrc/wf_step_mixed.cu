@@ -78,17 +78,25 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   return f2_of(r);
 }
 
-// Two Kahan sums side by side: the operations of KSum::add on each half.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)), "l"(f2_bits(c)));
+  return f2_of(r);
+}
+
+// Two Kahan sums side by side, value s - c each.  A product enters without
+// being rounded: the compensation is subtracted in its multiply-add.
 struct KSum2 {
-  float2 s = {0.f, 0.f}, c = {0.f, 0.f};
-  __device__ __forceinline__ void add(float2 x) {
-    float2 y = sub2(x, c);
+  float2 s = {0.f, 0.f}, nc = {0.f, 0.f};  // nc = -c
+  __device__ __forceinline__ void add_y(float2 y) {
     float2 t = add2(s, y);
-    c = sub2(sub2(t, s), y);
+    nc = sub2(y, sub2(t, s));
     s = t;
   }
-  __device__ __forceinline__ double value0() const { return f2d(s.x) - f2d(c.x); }
-  __device__ __forceinline__ double value1() const { return f2d(s.y) - f2d(c.y); }
+  __device__ __forceinline__ void add(float2 x) { add_y(add2(x, nc)); }
+  __device__ __forceinline__ void add_prod(float2 a, float2 b) { add_y(fma2(a, b, nc)); }
+  __device__ __forceinline__ double value0() const { return f2d(s.x) + f2d(nc.x); }
+  __device__ __forceinline__ double value1() const { return f2d(s.y) + f2d(nc.y); }
 };
 
 __device__ __forceinline__ float4 ld4(const float4* p) { return __ldg(p); }
@@ -284,18 +292,14 @@ struct StagedFetch {
 
 // Pair sums of the acceleration of SPH particle i over row entries k0, k0 + dk, ...
 // UNI: the uniform-particle layout (DomainConst::uni): h and Cs are the
-// domain's constants, m_j = m_i (a factor of the whole sum, applied by
-// accel_mx_value), Sigma/rho^2 xz and yz come from the last two fields of the
-// second velocity group, and rho_j = m_i / (m/rho)_j.
+// domain's constants, m_j = m_i, Sigma/rho^2 xz and yz come from the last two
+// fields of the second velocity group, and rho_j = m_i / (m/rho)_j.
 struct AccelSum {
   KSum2 a01;
   KSum a2;
 };
-template <bool UNI>
-__device__ __forceinline__ void accel_mx_value(const DevPtrs& P, const DomainConst& K, int i, const AccelSum& a,
-                                               double v[3]) {
-  const double m = UNI ? col(P, C_MASS, (size_t)K.N, i) : 1.0;
-  v[0] = m * a.a01.value0(); v[1] = m * a.a01.value1(); v[2] = m * a.a2.value();
+__device__ __forceinline__ void accel_mx_value(const AccelSum& a, double v[3]) {
+  v[0] = a.a01.value0(); v[1] = a.a01.value1(); v[2] = a.a2.value();
 }
 template <bool TI, bool AVU, bool GC, bool UNI, class Fetch>
 __device__ __forceinline__ void accel_mx_sums(const DevPtrs& P, const DomainConst& K, int i, const Fetch& F, int k0,
@@ -338,13 +342,12 @@ __device__ __forceinline__ void accel_mx_sums(const DevPtrs& P, const DomainCons
     if (Alpha != 0.f || Beta != 0.f) {
       float dvx = d.v0 * d.x0 + d.v1 * d.x1 + d.v2 * d.x2;
       if (dvx < 0.f) {  // Monaghan viscosity (InteractionAlt.cpp:74-94): MU (alpha C + beta MU) / rho_bar
-        const float hv = hh * dvx, Dn = r2 + 0.01f * hh * hh;
-        const float Cij = 0.5f * (s1.w + js1.w);
-        float p;  // MU / rho_bar, one division; in UNI 1 / rho_bar = 2 V_j / (rho_i V_j + m_i) with V_j = m_i / rho_j
-        if (UNI) p = hv * (2.f * jlo.w) / (Dn * (rhoi * jlo.w + mass_i));
-        else p = hv / (Dn * (0.5f * (rhoi + jvw.w)));
-        PIs = Alpha * Cij * p;
-        if (Beta != 0.f) PIs += Beta * p * (hv / Dn);
+        float MU = hh * dvx / (r * r + 0.01f * hh * hh);
+        float Cij = 0.5f * (s1.w + js1.w);
+        if (UNI)  // 1 / (0.5 (rho_i + rho_j)) with rho_j = m_i / (m/rho)_j
+          PIs = (Alpha * Cij * MU + Beta * MU * MU) * (2.f * jlo.w) / (rhoi * jlo.w + mass_i);
+        else
+          PIs = (Alpha * Cij * MU + Beta * MU * MU) / (0.5f * (rhoi + jvw.w));
       }
     }
     const float2 S01 = add2(make_float2(s0.x, s0.y), make_float2(js0.x, js0.y));
@@ -373,9 +376,17 @@ __device__ __forceinline__ void accel_mx_sums(const DevPtrs& P, const DomainCons
     }
     float g0 = GK * d.x0, g1 = GK * d.x1, g2 = GK * d.x2;
     if (GC) corr_gk(cm, GK, d.x0, d.x1, d.x2, g0, g1, g2);
-    if (!UNI) { const float mj = js1.z; g0 *= mj; g1 *= mj; g2 *= mj; }
-    a.a01.add(make_float2(g0 * S0 + g1 * S3 + g2 * S4, g0 * S3 + g1 * S1 + g2 * S5));
-    a.a2.add(g0 * S4 + g1 * S5 + g2 * S2);
+    const float mj = js1.z;
+    // The roundings are spelled out, so that a contact run, which amplifies the
+    // last bit of an acceleration, does not depend on how the compiler contracts
+    // this expression in one kernel or another.
+    auto dot = [](bool second, float a, float b, float c, float d, float e, float f) {  // a b + c d + e f
+      return __fmaf_rn(e, f, second ? __fmaf_rn(a, b, __fmul_rn(c, d)) : __fmaf_rn(c, d, __fmul_rn(a, b)));
+    };
+    const float E0 = dot(TI, g0, S0, g1, S3, g2, S4), E1 = dot(!TI, g0, S3, g1, S1, g2, S5);
+    const float E2 = dot(true, g0, S4, g1, S5, g2, S2);
+    a.a01.add_prod(make_float2(mj, mj), make_float2(E0, E1));
+    a.a2.add(mj * E2);
   });
 }
 template <bool TI, bool AVU, bool GC, bool UNI, class Fetch>
@@ -388,7 +399,7 @@ __device__ __forceinline__ void accel_mx(const DevPtrs& P, const DomainConst& K,
   AccelSum a;
   accel_mx_sums<TI, AVU, GC, UNI>(P, K, i, F, 0, 1, a);
   double v[3];
-  accel_mx_value<UNI>(P, K, i, a, v);
+  accel_mx_value(a, v);
   for (int d = 0; d < 3; ++d) colw(P, C_A + d, N, i) = v[d];
 }
 template <bool TI, bool AVU, bool GC, bool UNI>
@@ -413,7 +424,7 @@ __global__ void __launch_bounds__(512) k_accel_mx_lanes(DevPtrs P, DomainConst K
   double v[3] = {0.0, 0.0, 0.0};
   if (sph) {
     accel_mx_sums<TI, AVU, GC, UNI>(P, K, i, GlobalFetch{P.rc, P.nbr + i, N}, sub, L, a);
-    accel_mx_value<UNI>(P, K, i, a, v);
+    accel_mx_value(a, v);
   }
   double v0 = v[0], v1 = v[1], v2 = v[2];
   for (int off = 1; off < L; off <<= 1) {  // the whole warp takes part; L divides 32
@@ -611,7 +622,7 @@ __device__ __forceinline__ void density_drift_mx(const DevPtrs& P, const DomainC
       const float4* rj = P.rc + j;
       return MoveRec{ld4(rj + (size_t)RC_XV * N), ld4(rj + (size_t)RC_L * N), ld4(rj + (size_t)RC_VW * N)};
     };
-    walk_row(sub, L, len, key, load, [&](int, const MoveRec& q) {
+    auto pair = [&](int, const MoveRec& q) {
       const float4 jlo = q.lo, jvw = q.vw;
       const PairDiff d = pair_diff(pi, posvel(q.xv, jlo, jvw));
       const float x0 = d.x0, x1 = d.x1, x2 = d.x2, v0 = d.v0, v1 = d.v1, v2 = d.v2;
@@ -624,7 +635,12 @@ __device__ __forceinline__ void density_drift_mx(const DevPtrs& P, const DomainC
       } else {
         s.add(jlo.w * (GK * (v0 * x0 + v1 * x1 + v2 * x2)));  // (m_j / rho_j) v_ij . (GK x_ij)
       }
-    });
+    };
+    if constexpr (L == 1) {
+      walk_row(sub, L, len, key, load, pair);
+    } else {  // a lane's few entries need no pipelining (8,004 particles: 14.4 us either way)
+      for (int k = sub; k < len; k += L) pair(0, load(key(k)));
+    }
     dd = s.value();
   }
   if constexpr (L > 1)
@@ -753,11 +769,12 @@ __device__ __forceinline__ void rate_mx(const DevPtrs& P, const DomainConst& K, 
       // m_P2 of the pair: m_i when the pairs' masses agree, else the column
       float mP2 = K.m_pair ? mass_i : (float)col(P, C_MASS, N, up ? j : i);
       float pk = 0.5f * mP2 * (e.x + je.x) * dv;
-      M[0].add(make_float2(wb0 * y0, wb0 * y1));
-      M[1].add(make_float2(wb1 * y0, wb1 * y1));
-      M[2].add(make_float2(wb2 * y0, wb2 * y1));
-      M[3].add(make_float2(wb0 * y2, wb1 * y2));
-      M[4].add(make_float2(wb2 * y2, up ? pk : -pk));
+      const float2 y01 = make_float2(y0, y1);
+      M[0].add_prod(make_float2(wb0, wb0), y01);
+      M[1].add_prod(make_float2(wb1, wb1), y01);
+      M[2].add_prod(make_float2(wb2, wb2), y01);
+      M[3].add_prod(make_float2(wb0, wb1), make_float2(y2, y2));
+      M[4].add_prod(make_float2(wb2, up ? pk : -pk), make_float2(y2, 1.0f));
       if (THERMAL) {
         float wt = up ? jlo.w : lo.w;  // m_P2 / rho_P2 for both ends of the pair
         float dT = (e.z - je.z) + (e.w - je.w);
@@ -769,9 +786,9 @@ __device__ __forceinline__ void rate_mx(const DevPtrs& P, const DomainConst& K, 
     if constexpr (L == 1) {
       // The rate columns are FP32: each compensated sum is rounded to FP32 once
       // (s - c) and combined in FP32, which keeps the epilogue off the FP64 pipe.
-      const float m[9] = {M[0].s.x - M[0].c.x, M[0].s.y - M[0].c.y, M[3].s.x - M[3].c.x,
-                          M[1].s.x - M[1].c.x, M[1].s.y - M[1].c.y, M[3].s.y - M[3].c.y,
-                          M[2].s.x - M[2].c.x, M[2].s.y - M[2].c.y, M[4].s.x - M[4].c.x};
+      const float m[9] = {M[0].s.x + M[0].nc.x, M[0].s.y + M[0].nc.y, M[3].s.x + M[3].nc.x,
+                          M[1].s.x + M[1].nc.x, M[1].s.y + M[1].nc.y, M[3].s.y + M[3].nc.y,
+                          M[2].s.x + M[2].nc.x, M[2].s.y + M[2].nc.y, M[4].s.x + M[4].nc.x};
       out[0] = 2.0f * m[0]; out[1] = 2.0f * m[4]; out[2] = 2.0f * m[8];
       out[3] = m[1] + m[3]; out[4] = m[2] + m[6]; out[5] = m[5] + m[7];
       out[6] = m[1] - m[3]; out[7] = m[2] - m[6]; out[8] = m[5] - m[7];
