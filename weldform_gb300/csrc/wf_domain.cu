@@ -1217,8 +1217,7 @@ struct wf_domain {
     }
     K.av_alpha = (float)a0;
     K.av_beta = (float)b0;
-    // the staged gather copies the five-group layout
-    K.uni = (K.m_pair && h_uniform && cs_uniform && !stage && h0 > 0) ? 1 : 0;
+    K.uni = (K.m_pair && h_uniform && cs_uniform && h0 > 0) ? 1 : 0;
     K.h_f = (float)h0;
     K.cs_f = (float)c0;
     // the FP32 operations of the per-pair kernel factor at hh = h
@@ -1738,9 +1737,7 @@ int wf_set_domain_i32(wf_domain* d, const char* name, int v) {
   if (n == "gather_staging") {  // shared-memory staged acceleration gather of the mixed form
     if (d->prepared && v && !d->stage_ready)
       return set_err(WF_ERR_STATE, "gather_staging must be set before the prologue (it allocates the halo lists)");
-    d->stage = v != 0;
-    if (d->prepared)  // the uniform-particle record layout is off while staging is on
-      return guard([&] { d->refresh_uniform(); return WF_OK; });
+    d->stage = v != 0;  // the step graph is captured again at the next step
     return WF_OK;
   }
   if (n == "stage_cap") {

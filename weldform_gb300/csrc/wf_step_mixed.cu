@@ -278,7 +278,7 @@ struct GlobalFetch {
   }
 };
 struct StagedFetch {
-  const float4* sh;            // 5 groups of cap records in shared memory
+  const float4* sh;            // 5 groups (uniform layout: 4) of cap records in shared memory
   const unsigned short* slot;  // P.nslot + i
   size_t N;
   int cap;
@@ -286,7 +286,11 @@ struct StagedFetch {
   template <bool UNI>
   __device__ __forceinline__ AccelRec get(int q) const {
     // the global index is not known here: no misc or TI group (AVU and !TI only)
-    return AccelRec{sh[q], sh[cap + q], sh[2 * cap + q], sh[3 * cap + q], sh[4 * cap + q], -1};
+    AccelRec r;
+    r.xv = sh[q]; r.lo = sh[cap + q]; r.vw = sh[2 * cap + q]; r.s0 = sh[3 * cap + q];
+    if (!UNI) r.s1 = sh[4 * cap + q];
+    r.j = -1;
+    return r;
   }
 };
 
@@ -449,6 +453,7 @@ __global__ void __launch_bounds__(512) k_accel_mx_lanes(DevPtrs P, DomainConst K
 // each half is a Kahan sum and the two are added in FP64.  A block whose halo
 // exceeded the capacity (halo_len -1) reads global memory with the same split,
 // so results do not depend on the capacity.
+template <bool UNI>
 __global__ void __launch_bounds__(2 * STAGE_B) k_accel_mx_staged(DevPtrs P, DomainConst K) {
   extern __shared__ float4 sh_rec[];
   const int b = blockIdx.x, t = threadIdx.x, cap = K.stage_cap;
@@ -462,7 +467,7 @@ __global__ void __launch_bounds__(2 * STAGE_B) k_accel_mx_staged(DevPtrs P, Doma
       sh_rec[cap + s] = ld4(rj + (size_t)RC_L * N);
       sh_rec[2 * cap + s] = ld4(rj + (size_t)RC_VW * N);
       sh_rec[3 * cap + s] = ld4(rj + (size_t)RC_S0 * N);
-      sh_rec[4 * cap + s] = ld4(rj + (size_t)RC_S1 * N);
+      if (!UNI) sh_rec[4 * cap + s] = ld4(rj + (size_t)RC_S1 * N);
     }
   }
   __syncthreads();
@@ -471,8 +476,8 @@ __global__ void __launch_bounds__(2 * STAGE_B) k_accel_mx_staged(DevPtrs P, Doma
   const bool sph = i < K.N && icol(P, I_KIND, N, i) == 0;
   AccelSum a;
   if (sph) {
-    if (H >= 0) accel_mx_sums<false, true, false, false>(P, K, i, StagedFetch{sh_rec, P.nslot + i, N, cap}, part, 2, a);
-    else accel_mx_sums<false, true, false, false>(P, K, i, GlobalFetch{P.rc, P.nbr + i, N}, part, 2, a);
+    if (H >= 0) accel_mx_sums<false, true, false, UNI>(P, K, i, StagedFetch{sh_rec, P.nslot + i, N, cap}, part, 2, a);
+    else accel_mx_sums<false, true, false, UNI>(P, K, i, GlobalFetch{P.rc, P.nbr + i, N}, part, 2, a);
   }
   double v0 = a.a01.value0(), v1 = a.a01.value1(), v2 = a.a2.value();
   __syncthreads();  // halo records no longer read: the odd halves pass through shared memory
@@ -581,8 +586,11 @@ void launch_halo_build(const DevPtrs& P, const DomainConst& K, cudaStream_t s) {
 }
 
 int configure_staging(int cap) {
-  size_t bytes = (size_t)5 * cap * sizeof(float4);
-  return (int)cudaFuncSetAttribute(k_accel_mx_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  const int g = cap * (int)sizeof(float4);
+  cudaError_t e = cudaFuncSetAttribute(k_accel_mx_staged<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 5 * g);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_accel_mx_staged<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * g);
+  return (int)e;
 }
 
 // A neighbour's position and velocity groups (and, for conduction, its E group).
@@ -1133,7 +1141,9 @@ void launch_step_mixed(const DevPtrs& P, const DomainConst& K, double* fscratch,
   launch_tensile(P, K, s);
   const bool staged = K.stage_cap > 0 && P.halo && !K.ti && K.av_uniform && !K.gradcorr;
   if (staged) {
-    k_accel_mx_staged<<<nblk(K.N, STAGE_B), 2 * STAGE_B, (size_t)5 * K.stage_cap * sizeof(float4), s>>>(P, K);
+    const size_t g = (size_t)K.stage_cap * sizeof(float4);
+    if (K.uni) k_accel_mx_staged<true><<<nblk(K.N, STAGE_B), 2 * STAGE_B, 4 * g, s>>>(P, K);
+    else k_accel_mx_staged<false><<<nblk(K.N, STAGE_B), 2 * STAGE_B, 5 * g, s>>>(P, K);
   } else if (K.ti) {
     if (K.av_uniform) launch_accel_mx<true, true>(P, K, ng, gb, s);
     else launch_accel_mx<true, false>(P, K, ng, gb, s);
