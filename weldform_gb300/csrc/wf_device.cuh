@@ -223,6 +223,7 @@ struct StepState {
   // Verlet-skin reuse of the neighbour search (DomainConst::skin_on)
   unsigned long long maxdisp2_bits;  // largest squared displacement since the superset was built (as bits)
   int search_full;     // this step's search re-sorts and rebuilds the superset (else: filter only)
+  unsigned skin_blocks;  // blocks of k_skin_check that are done
   int sup_valid;       // a superset exists and every row fitted in SUP_W
   long long nb_full_searches;
   int nan_count;       // particles with a non-finite position at the last search

@@ -741,6 +741,7 @@ struct wf_domain {
     // grid cells, then as many shadow buckets for particles with a non-finite position
     P.cell_start = dalloc<int>(2 * ncells + 1);
     P.cell_count = dalloc<int>(2 * ncells);
+    CK(cudaMemsetAsync(P.cell_count, 0, sizeof(int) * 2 * ncells, stream));
     {
       int* db = dalloc<int>(brick.size());
       CK(cudaMemcpyAsync(db, brick.data(), sizeof(int) * brick.size(), cudaMemcpyHostToDevice, stream));
@@ -754,6 +755,7 @@ struct wf_domain {
     P.perm = dalloc<int>(n);
     P.inv = dalloc<int>(n);
     P.xs = dalloc<float>(4 * n);
+    P.cellc = dalloc<long long>(n);
     P.row_len = dalloc<int>(n);
     P.row_split = dalloc<int>(n);
     P.nbr = dalloc<int>((size_t)MAX_NB * n);
@@ -958,8 +960,7 @@ struct wf_domain {
       P.sup = dalloc<int>((size_t)SUP_W * n);
       P.sup_len = dalloc<int>(n);
       P.xref = dalloc<double>((size_t)3 * n);
-      P.cellc = dalloc<long long>(n);
-    }
+      }
     if (K.nspec > 0) {  // one rebuild schedule per specimen, as a run of it alone starts
       std::vector<SpecState> sp(K.nspec);
       for (SpecState& q : sp) { memset(&q, 0, sizeof(q)); q.nb_cleared = 1; }
@@ -1004,7 +1005,7 @@ struct wf_domain {
     // SolverKickDrift.cpp:72-96: with contact, a search + CalculateSurface(1)
     // before the loop; the first step searches again (ClearNbData).
     if (contact) {
-      launch_force_search(P, stream);
+      launch_force_search(P, kconst(), stream);
       launch_neighbour_search(P, kconst(), d_fscratch, d_iscratch, stream);
       K.id_free_surf = 1;
     }
@@ -1534,7 +1535,7 @@ struct wf_domain {
   void search_now() {
     if (!prepared) throw CudaError{WF_ERR_STATE, "neighbour search before the solver prologue"};
     use_device();
-    wf::launch_force_search(P, stream);
+    wf::launch_force_search(P, kconst(), stream);
     wf::launch_neighbour_search(P, kconst(), d_fscratch, d_iscratch, stream);
     shadows_valid = false;  // the search reorders particles
     invalidate_gk();

@@ -21,7 +21,7 @@
 // particle's superset over a 5 x 5 x 5 stencil at the pair radius plus the
 // skin (k_nbr_fill<true>), and a later search whose particles all moved less
 // than half the skin skips steps 1-5 and filters the supersets with the same
-// exact rules (k_skin_check, k_search_mode, k_cell_coords, k_nbr_filter).
+// exact rules (k_skin_check, k_nbr_filter).
 // The radius test rij / h <= Cellfac is decided bit-exactly: an FP32 distance
 // prefilter with a proven-safe relative margin accepts or rejects clear cases,
 // and everything inside the margin is decided by the reference's FP64
@@ -30,8 +30,8 @@
 // Every kernel checks st->do_search first (the re-sorting ones also
 // search_full), so the search can sit inside a captured step and cost only
 // an empty launch on steps that do not rebuild.
-#include "wf_device.cuh"
 #include "wf_launch.h"
+#include "wf_step_common.cuh"
 
 namespace wf {
 
@@ -99,11 +99,6 @@ __global__ void k_rows_save(DevPtrs P, DomainConst K) {
   }
 }
 
-__global__ void k_zero_int(DevPtrs P, int* a, long long n, int gate) {
-  if (gate && !searching_full(P)) return;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) a[k] = 0;
-}
-
 // ---- exclusive scan of an int array into an int array (three phases) ------
 constexpr int SCAN_THREADS = 1024;
 constexpr int SCAN_ITEMS = 4;
@@ -153,7 +148,8 @@ __global__ void k_scan_top(DevPtrs P, long long* tot, int nb) {
     __syncthreads();
   }
 }
-__global__ void k_scan_down(DevPtrs P, const int* in, long long n, const long long* tot, int* out, int* total_out) {
+// The counts are zeroed as they are read: the scatter uses them as cursors next.
+__global__ void k_scan_down(DevPtrs P, int* in, long long n, const long long* tot, int* out, int* total_out) {
   if (!searching_full(P)) return;
   __shared__ long long sh[SCAN_THREADS];
   long long base = (long long)blockIdx.x * SCAN_TILE;
@@ -162,6 +158,7 @@ __global__ void k_scan_down(DevPtrs P, const int* in, long long n, const long lo
   for (int k = 0; k < SCAN_ITEMS; ++k) {
     long long idx = base + (long long)threadIdx.x * SCAN_ITEMS + k;
     vals[k] = (idx < n) ? in[idx] : 0;
+    if (idx < n) in[idx] = 0;
     s += vals[k];
   }
   long long total;
@@ -172,6 +169,31 @@ __global__ void k_scan_down(DevPtrs P, const int* in, long long n, const long lo
     ex += vals[k];
   }
   if (total_out && blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) *total_out = (int)ex;
+}
+
+// The three phases by one block, for grids of a few tiles.
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_one(DevPtrs P, int* in, int n, int* out, int* total_out) {
+  if (!searching_full(P)) return;
+  __shared__ long long sh[SCAN_THREADS];
+  long long carry = 0;
+  for (int base = 0; base < n; base += SCAN_TILE) {
+    int v[SCAN_ITEMS];
+    long long s = 0, total;
+    for (int k = 0; k < SCAN_ITEMS; ++k) {
+      const int idx = base + (int)threadIdx.x * SCAN_ITEMS + k;
+      v[k] = idx < n ? in[idx] : 0;
+      if (idx < n) in[idx] = 0;
+      s += v[k];
+    }
+    long long ex = block_exclusive_scan(s, sh, &total) + carry;
+    for (int k = 0; k < SCAN_ITEMS; ++k) {
+      const int idx = base + (int)threadIdx.x * SCAN_ITEMS + k;
+      if (idx < n) out[idx] = (int)ex;
+      ex += v[k];
+    }
+    carry += total;
+  }
+  if (threadIdx.x == 0) *total_out = (int)carry;
 }
 
 __global__ void k_scatter(DevPtrs P, DomainConst K) {
@@ -265,6 +287,8 @@ __global__ void __launch_bounds__(BRICK_T) k_sort_bricks(DevPtrs P, DomainConst 
       __syncthreads();
       for (int e = t; e < n; e += BRICK_T) P.perm[s0 + e] = tmp[s0 + e];
     }
+    // the cells' counts (the scatter's cursors) back to zero for the next search
+    for (int c = P.brick_cell[b] + t; c < P.brick_cell[b + 1]; c += BRICK_T) P.cell_count[c] = 0;
     __syncthreads();  // the shared keys are reused by the next brick
   }
 }
@@ -301,6 +325,33 @@ __device__ __forceinline__ bool is_contact_id(const DomainConst& K, int id) {
   return false;
 }
 
+// The FP32 prefilter coordinates of particle p, and its cell coordinates at the
+// current positions (ListGenerate's clamped cell index, Neighbour.cpp:185-218,
+// the same FP64 expression as k_cell_keys), 21 bits per axis, -1 for a
+// non-finite position.  COVER: the filter leaves the cell test out, so only
+// the finiteness is recorded.
+template <bool COVER>
+__device__ __forceinline__ float4 search_coords(const DevPtrs& P, const DomainConst& K, int p) {
+  const size_t N = K.N;
+  long long code = 0;
+  bool finite = true;
+  for (int d = 0; d < 3; ++d) {
+    double xd = P.f[(C_X + d) * N + p];
+    finite = finite && isfinite(xd);
+    if (!COVER) {
+      int q = (int)floor(__ddiv_rn(__dsub_rn(xd, K.BLPF[d]), K.CellSize[d]));
+      if (q < 0) q = 0;
+      if (q >= K.CellNo[d]) q = K.CellNo[d] - 1;
+      code = (code << 21) | (long long)q;
+    }
+  }
+  const float4 x = make_float4((float)(P.f[(C_X + 0) * N + p] - K.BLPF[0]), (float)(P.f[(C_X + 1) * N + p] - K.BLPF[1]),
+                               (float)(P.f[(C_X + 2) * N + p] - K.BLPF[2]), (float)P.f[C_H * N + p]);
+  P.cellc[p] = finite ? code : -1;
+  reinterpret_cast<float4*>(P.xs)[p] = x;
+  return x;
+}
+
 // Map original -> sorted index, element -> mesh particle, and the FP32
 // prefilter coordinates (relative to BLPF, plus h); and for each slot of the
 // cells' lists what the candidate test of a stencil scan reads, in slot order:
@@ -315,10 +366,7 @@ __global__ void k_after_permute(DevPtrs P, DomainConst K) {
   P.inv[o] = p;
   int kind = P.i[I_KIND * N + p];
   if (kind == 1) P.elem_particle[P.i[I_ELEM * N + p]] = p;
-  const float4 x = make_float4((float)(P.f[(C_X + 0) * N + p] - K.BLPF[0]), (float)(P.f[(C_X + 1) * N + p] - K.BLPF[1]),
-                               (float)(P.f[(C_X + 2) * N + p] - K.BLPF[2]), (float)P.f[C_H * N + p]);
-  reinterpret_cast<float4*>(P.xs)[p] = x;
-  P.cand_x[s] = x;
+  P.cand_x[s] = !K.skin_on || K.cells_cover ? search_coords<true>(P, K, p) : search_coords<false>(P, K, p);
   // class word for the pair rules: bit 0 rigid-mesh particle, bit 1 carries a
   // contact-surface id, bits 2.. material index
   P.cand_m[s] = make_int4(p, o, kind | (is_contact_id(K, P.i[I_ID * N + p]) ? 2 : 0) | (P.i[I_MATERIAL * N + p] << 2),
@@ -604,70 +652,49 @@ __global__ void __launch_bounds__(FILL_WARPS * 32) k_nbr_fill(DevPtrs P, DomainC
 // ---- Verlet-skin reuse -------------------------------------------------------
 // Largest squared displacement since the superset was built (a non-finite
 // position gives NaN, whose bit pattern exceeds every finite one: a full
-// search follows).
+// search follows), and what the filter reads at the current positions
+// (search_coords; in a batched domain only for the specimens that search: no
+// pair leaves a specimen).  The block that finishes last decides between a
+// full search and the filter: a filter suffices while every particle has moved
+// less than skin / 2 since the superset was built, since a pair within its
+// radius now was then within the radius plus the skin.
+template <bool COVER>
 __global__ void k_skin_check(DevPtrs P, DomainConst K) {
-  if (!searching(P) || !K.skin_on || !P.st->sup_valid) return;
-  const size_t N = K.N;
-  double m = 0.0;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < K.N; p += gridDim.x * blockDim.x) {
-    double d0 = P.f[(C_X + 0) * N + p] - P.xref[p];
-    double d1 = P.f[(C_X + 1) * N + p] - P.xref[N + p];
-    double d2 = P.f[(C_X + 2) * N + p] - P.xref[2 * N + p];
-    double d = d0 * d0 + d1 * d1 + d2 * d2;
-    if (!(d <= m)) m = d;
-  }
-  unsigned long long b = (unsigned long long)__double_as_longlong(m);
-  for (int off = 16; off > 0; off >>= 1) {
-    unsigned long long o = __shfl_down_sync(0xffffffffu, b, off);
-    b = o > b ? o : b;
-  }
-  if ((threadIdx.x & 31) == 0 && b) atomicMax(&P.st->maxdisp2_bits, b);
-}
-
-// Full search or filter only: a filter suffices while every particle has
-// moved less than skin / 2 since the superset was built, since a pair within
-// its radius now was then within the radius plus the skin.
-__global__ void k_search_mode(DevPtrs P, DomainConst K) {
+  if (!searching(P)) return;
+  __shared__ bool last;
   StepState* s = P.st;
-  if (!s->do_search) return;
-  const double md2 = __longlong_as_double((long long)s->maxdisp2_bits);
+  const size_t N = K.N;
+  if (s->sup_valid) {
+    double m = 0.0;
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < K.N; p += gridDim.x * blockDim.x) {
+      double d0 = P.f[(C_X + 0) * N + p] - P.xref[p];
+      double d1 = P.f[(C_X + 1) * N + p] - P.xref[N + p];
+      double d2 = P.f[(C_X + 2) * N + p] - P.xref[2 * N + p];
+      double d = d0 * d0 + d1 * d1 + d2 * d2;
+      if (!(d <= m)) m = d;
+      if (K.nspec == 0 || P.sp[P.i[I_SPEC * N + p]].do_search) search_coords<COVER>(P, K, p);
+    }
+    unsigned long long b = (unsigned long long)__double_as_longlong(m);
+    for (int off = 16; off > 0; off >>= 1) {
+      unsigned long long o = __shfl_down_sync(0xffffffffu, b, off);
+      b = o > b ? o : b;
+    }
+    if ((threadIdx.x & 31) == 0 && b) atomicMax(&s->maxdisp2_bits, b);
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&s->skin_blocks, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last || threadIdx.x != 0) return;
+  s->skin_blocks = 0;
+  __threadfence();
+  const double md2 = __longlong_as_double((long long)*(volatile unsigned long long*)&s->maxdisp2_bits);
   const double half = 0.5 * K.skin;
-  const bool filter_only = K.skin_on && s->sup_valid && md2 <= half * half;
+  const bool filter_only = s->sup_valid && md2 <= half * half;
   s->search_full = filter_only ? 0 : 1;
   if (!filter_only) {
     s->nb_full_searches += 1;
-    if (K.skin_on) s->sup_valid = 1;  // the superset build clears it again if a row does not fit
-  }
-}
-
-// Cell coordinates at the current positions (ListGenerate's clamped cell
-// index, Neighbour.cpp:185-218, the same FP64 expression as k_cell_keys),
-// 21 bits per axis, -1 for a non-finite position; and the FP32 prefilter
-// coordinates.  COVER: the filter leaves the cell test out, so only the
-// finiteness is recorded.  In a batched domain only the particles of the
-// specimens that search are needed (no pair leaves a specimen).
-template <bool COVER>
-__global__ void k_cell_coords(DevPtrs P, DomainConst K) {
-  if (!searching(P) || !K.skin_on || !P.st->sup_valid) return;
-  const size_t N = K.N;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < K.N; p += gridDim.x * blockDim.x) {
-    if (K.nspec > 0 && !P.sp[P.i[I_SPEC * N + p]].do_search) continue;
-    long long code = 0;
-    bool finite = true;
-    for (int d = 0; d < 3; ++d) {
-      double xd = P.f[(C_X + d) * N + p];
-      finite = finite && isfinite(xd);
-      if (!COVER) {
-        int q = (int)floor(__ddiv_rn(__dsub_rn(xd, K.BLPF[d]), K.CellSize[d]));
-        if (q < 0) q = 0;
-        if (q >= K.CellNo[d]) q = K.CellNo[d] - 1;
-        code = (code << 21) | (long long)q;
-      }
-    }
-    P.cellc[p] = finite ? code : -1;
-    reinterpret_cast<float4*>(P.xs)[p] =
-        make_float4((float)(P.f[(C_X + 0) * N + p] - K.BLPF[0]), (float)(P.f[(C_X + 1) * N + p] - K.BLPF[1]),
-                    (float)(P.f[(C_X + 2) * N + p] - K.BLPF[2]), (float)P.f[C_H * N + p]);
+    s->sup_valid = 1;  // the superset build clears it again if a row does not fit
   }
 }
 
@@ -872,19 +899,11 @@ __global__ void k_contact_pairs(DevPtrs P, DomainConst K) {
   if ((threadIdx.x & 31) == 0 && npairs) atomicAdd(&P.st->contact_pair_count, (unsigned long long)npairs);
 }
 
-__global__ void k_force_search(DevPtrs P) { P.st->do_search = 1; }
-void launch_force_search(const DevPtrs& P, cudaStream_t s) { k_force_search<<<1, 1, 0, s>>>(P); }
-
-__global__ void k_search_begin(DevPtrs P) {
-  if (!searching(P)) return;
-  P.st->pair_count = 0;
-  P.st->contact_pair_count = 0;
-  P.st->surface_count = 0;
-  P.st->cp_count = 0;
-  P.st->nan_count = 0;
-  P.st->maxdisp2_bits = 0;
-  P.st->nb_searches += 1;
+__global__ void k_force_search(DevPtrs P, DomainConst K) {
+  P.st->do_search = 1;
+  search_begin(P, K);
 }
+void launch_force_search(const DevPtrs& P, const DomainConst& K, cudaStream_t s) { k_force_search<<<1, 1, 0, s>>>(P, K); }
 
 // ---------------------------------------------------------------- host side
 static inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
@@ -898,32 +917,29 @@ void launch_neighbour_search(const DevPtrs& P, const DomainConst& K, double* fsc
   auto grid = [&](long long n) { int b = nblk(n, T); return b < G ? b : G; };
   // buckets: ncells grid cells (Morton ranks), then ncells shadow buckets
   const long long nbk = 2LL * K.ncells;
-  int nz = grid(nbk);
-  k_search_begin<<<1, 1, 0, s>>>(P);
-  mark(s, "k_search_begin");
   if (K.skin_on) {
-    k_skin_check<<<grid(K.N), T, 0, s>>>(P, K);
+    if (K.cells_cover) k_skin_check<true><<<grid(K.N), T, 0, s>>>(P, K);
+    else k_skin_check<false><<<grid(K.N), T, 0, s>>>(P, K);
     mark(s, "k_skin_check");
   }
-  k_search_mode<<<1, 1, 0, s>>>(P, K);
-  mark(s, "k_search_mode");
   if (K.nspec > 0) {
     k_rows_save<<<grid(K.N), T, 0, s>>>(P, K);
     mark(s, "k_rows_save");
   }
-  k_zero_int<<<nz, T, 0, s>>>(P, P.cell_count, nbk, 1);
-  mark(s, "k_zero_int");
   k_cell_keys<<<grid(K.N), T, 0, s>>>(P, K);
   mark(s, "k_cell_keys");
-  int nb = nblk(nbk, SCAN_TILE);
-  k_scan_reduce<<<nb, SCAN_THREADS, 0, s>>>(P, P.cell_count, nbk, P.scan_tmp);
-  mark(s, "k_scan_reduce");
-  k_scan_top<<<1, SCAN_THREADS, 0, s>>>(P, P.scan_tmp, nb);
-  mark(s, "k_scan_top");
-  k_scan_down<<<nb, SCAN_THREADS, 0, s>>>(P, P.cell_count, nbk, P.scan_tmp, P.cell_start, P.cell_start + nbk);
-  mark(s, "k_scan_down");
-  k_zero_int<<<nz, T, 0, s>>>(P, P.cell_count, nbk, 1);
-  mark(s, "k_zero_int");
+  if (nbk <= 16 * SCAN_TILE) {  // two launches saved against 4 us more at 16 tiles, when a search re-sorts
+    k_scan_one<<<1, SCAN_THREADS, 0, s>>>(P, P.cell_count, (int)nbk, P.cell_start, P.cell_start + nbk);
+    mark(s, "k_scan_one");
+  } else {
+    int nb = nblk(nbk, SCAN_TILE);
+    k_scan_reduce<<<nb, SCAN_THREADS, 0, s>>>(P, P.cell_count, nbk, P.scan_tmp);
+    mark(s, "k_scan_reduce");
+    k_scan_top<<<1, SCAN_THREADS, 0, s>>>(P, P.scan_tmp, nb);
+    mark(s, "k_scan_top");
+    k_scan_down<<<nb, SCAN_THREADS, 0, s>>>(P, P.cell_count, nbk, P.scan_tmp, P.cell_start, P.cell_start + nbk);
+    mark(s, "k_scan_down");
+  }
   k_scatter<<<grid(K.N), T, 0, s>>>(P, K);
   mark(s, "k_scatter");
   k_sort_bricks<<<K.nbricks < 152 * 2 ? K.nbricks : 152 * 2, BRICK_T, 0, s>>>(P, K);
@@ -945,9 +961,6 @@ void launch_neighbour_search(const DevPtrs& P, const DomainConst& K, double* fsc
   }
   mark(s, "k_nbr_fill");
   if (K.skin_on) {
-    if (K.cells_cover) k_cell_coords<true><<<grid(K.N), T, 0, s>>>(P, K);
-    else k_cell_coords<false><<<grid(K.N), T, 0, s>>>(P, K);
-    mark(s, "k_cell_coords");
     int groups = nblk(K.N, FILL_ROWS), cap = 152 * 4;
     if (K.cells_cover) k_nbr_filter<true><<<groups < cap ? groups : cap, FILL_WARPS * 32, 0, s>>>(P, K);
     else k_nbr_filter<false><<<groups < cap ? groups : cap, FILL_WARPS * 32, 0, s>>>(P, K);

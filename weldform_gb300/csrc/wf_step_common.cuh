@@ -14,6 +14,20 @@ __device__ __forceinline__ double col(const DevPtrs& P, int c, size_t N, int i) 
 __device__ __forceinline__ double& colw(const DevPtrs& P, int c, size_t N, int i) { return P.f[(size_t)c * N + i]; }
 __device__ __forceinline__ int icol(const DevPtrs& P, int c, size_t N, int i) { return P.i[(size_t)c * N + i]; }
 
+// Counters of a search that begins, by the thread that decides it; without the
+// Verlet-skin reuse every search re-sorts (with it, k_skin_check decides).
+__device__ __forceinline__ void search_begin(const DevPtrs& P, const DomainConst& K) {
+  StepState* s = P.st;
+  s->pair_count = 0;
+  s->contact_pair_count = 0;
+  s->surface_count = 0;
+  s->cp_count = 0;
+  s->nan_count = 0;
+  s->maxdisp2_bits = 0;
+  s->nb_searches += 1;
+  if (!K.skin_on) { s->search_full = 1; s->nb_full_searches += 1; }
+}
+
 // Deterministic block reduction (fixed shuffle tree, then fixed order across
 // warps) of one value per thread; the result is valid in thread 0.
 template <int OP>  // 0 sum, 1 max, 2 min

@@ -83,7 +83,10 @@ __global__ void k_schedule(DevPtrs P, DomainConst K, unsigned long long cond) {
   // the first step's search the rows, contact pairs and surface flags stay.
   if (K.freeze_nb && !s->isfirst) search = regular = 0;
   if (K.nspec > 0) { search = any_search; regular = any_regular; }
-  if (search) s->nb_cleared = 0;
+  if (search) {
+    s->nb_cleared = 0;
+    search_begin(P, K);
+  }
   s->do_search = search;
   // CalcGradCorrMatrix: kick-drift at its first step (SolverKickDrift.cpp:189-191),
   // leapfrog after every regular search and at the first step (SolverLeapfrog.cpp:186-204)
@@ -91,7 +94,8 @@ __global__ void k_schedule(DevPtrs P, DomainConst K, unsigned long long cond) {
   if (cond) cudaGraphSetConditional((cudaGraphConditionalHandle)cond, search ? 1u : 0u);
 }
 
-__global__ void k_step_end(DevPtrs P, DomainConst K) {
+// Time and the rebuild schedule after the step (one block of k_finalize).
+__device__ __forceinline__ void step_end(const DevPtrs& P, const DomainConst& K) {
   StepState* s = P.st;
   for (int q = threadIdx.x; q < K.nspec; q += blockDim.x) {  // each specimen's own cadence
     SpecState& sp = P.sp[q];
@@ -1104,10 +1108,30 @@ __global__ void __launch_bounds__(L > 1 ? 512 : BLOCK) k_rate_stress(DevPtrs P, 
 
 
 // ---------------------------------------------------------------- reductions
-// One block per slot; each thread sums a fixed strided subset, then a fixed tree.
+// TriMesh::Update: node_v = m_v + m_w x node; node += node_v dt.
+__device__ __forceinline__ void mesh_node(const DevPtrs& P, const DomainConst& K, int n) {
+  if (n >= P.nnodes) return;
+  int m = P.node_mesh[n];
+  const double* mv = P.st->mesh_v[m];
+  const double* mw = P.st->mesh_w[m];
+  double p[3] = {P.node[n], P.node[P.nnodes + n], P.node[2 * P.nnodes + n]};
+  double vr[3] = {mw[1] * p[2] - mw[2] * p[1], mw[2] * p[0] - mw[0] * p[2], mw[0] * p[1] - mw[1] * p[0]};
+  if (!K.contact_mesh_auto_update) return;
+  for (int d = 0; d < 3; ++d) {
+    double nv = mv[d] + vr[d];
+    P.node_v[d * P.nnodes + n] = nv;
+    P.node[d * P.nnodes + n] = p[d] + nv * P.st->deltat;
+  }
+}
+// One block per slot; each thread sums a fixed strided subset, then a fixed
+// tree.  The block after the slots closes the step, and the ones after that
+// move the rigid meshes' nodes: neither reads what a slot writes, and a launch
+// of its own for each costs a small domain ~1.5 us of its step.
 __global__ void k_finalize(DevPtrs P, DomainConst K) {
   __shared__ double sh[1024];
   int slot = blockIdx.x;
+  if (slot == NSLOTS) { step_end(P, K); return; }
+  if (slot > NSLOTS) { mesh_node(P, K, (slot - NSLOTS - 1) * blockDim.x + threadIdx.x); return; }
   bool active = (slot == S_DINT || slot == S_DKIN || slot == S_MAXPL) ||
                 (K.pl_heating && slot == S_PLW) || (K.thermal_solver && (slot == S_MAXT || slot == S_MINT)) ||
                 (K.contact && (slot == S_CFSUM || slot == S_CRSUM || slot == S_EXTW ||
@@ -1157,22 +1181,6 @@ __global__ void k_finalize(DevPtrs P, DomainConst K) {
 }
 
 // ---------------------------------------------------------------- rigid meshes
-// TriMesh::Update: node_v = m_v + m_w x node; node += node_v dt.
-__global__ void k_mesh_nodes(DevPtrs P, DomainConst K) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= P.nnodes) return;
-  int m = P.node_mesh[n];
-  const double* mv = P.st->mesh_v[m];
-  const double* mw = P.st->mesh_w[m];
-  double p[3] = {P.node[n], P.node[P.nnodes + n], P.node[2 * P.nnodes + n]};
-  double vr[3] = {mw[1] * p[2] - mw[2] * p[1], mw[2] * p[0] - mw[0] * p[2], mw[0] * p[1] - mw[1] * p[0]};
-  if (!K.contact_mesh_auto_update) return;
-  for (int d = 0; d < 3; ++d) {
-    double nv = mv[d] + vr[d];
-    P.node_v[d * P.nnodes + n] = nv;
-    P.node[d * P.nnodes + n] = p[d] + nv * P.st->deltat;
-  }
-}
 // CalcNormals + UpdatePlaneCoeff per element (Mesh.cpp:222-256), then
 // UpdateContactParticles (Contact.cpp:41-55) for the element's particle.
 __global__ void k_mesh_elems(DevPtrs P, DomainConst K) {
@@ -1393,6 +1401,13 @@ void launch_bc(const DevPtrs& P, const DomainConst& K, int vcol, cudaStream_t s)
   k_bc<<<nbc, BLOCK, 0, s>>>(P, K, vcol);
   mark(s, "k_bc");
 }
+// GeneralAfter between the acceleration and the first kick.  The kick kernel
+// applies the same values to its particle after the kick (a = 0, v = value,
+// whatever they were), so without anything that reads them in between (contact,
+// the time-step tests, leapfrog's own order, the tape) this pass is left out.
+void launch_bc_before_kick(const DevPtrs& P, const DomainConst& K, cudaStream_t s) {
+  if (K.contact || K.leapfrog || K.auto_ts || K.auto_ts_acc || P.tx) launch_bc(P, K, C_V, s);
+}
 void launch_contact_kick(const DevPtrs& P, const DomainConst& K, cudaStream_t s) {
   bool adapt = K.auto_ts || K.auto_ts_acc;
   if (K.auto_ts && !K.leapfrog) {  // kick-drift: the velocity criterion sees v before the first kick
@@ -1425,16 +1440,13 @@ void launch_contact_kick(const DevPtrs& P, const DomainConst& K, cudaStream_t s)
   }
 }
 void launch_step_tail(const DevPtrs& P, const DomainConst& K, cudaStream_t s) {
-  k_finalize<<<NSLOTS, 1024, 0, s>>>(P, K);
+  const bool meshes = K.contact && P.nelem > 0;
+  k_finalize<<<NSLOTS + 1 + (meshes ? nblk(P.nnodes, 1024) : 0), 1024, 0, s>>>(P, K);
   mark(s, "k_finalize");
-  if (K.contact && P.nelem > 0) {
-    k_mesh_nodes<<<nblk(P.nnodes, BLOCK), BLOCK, 0, s>>>(P, K);
-    mark(s, "k_mesh_nodes");
+  if (meshes) {
     k_mesh_elems<<<nblk(P.nelem, BLOCK), BLOCK, 0, s>>>(P, K);
     mark(s, "k_mesh_elems");
   }
-  k_step_end<<<1, 256, 0, s>>>(P, K);
-  mark(s, "k_step_end");
 }
 
 void launch_step_fp64(const DevPtrs& P, const DomainConst& K, double* fscratch, int* iscratch, cudaStream_t s) {
@@ -1474,7 +1486,7 @@ void launch_step_fp64_body(const DevPtrs& P, const DomainConst& K, cudaStream_t 
     else launch_accel64<false, LL>(P, K, s);
   });
   mark(s, "k_accel");
-  launch_bc(P, K, C_V, s);
+  launch_bc_before_kick(P, K, s);
   launch_contact_kick(P, K, s);
   if (K.leapfrog) launch_bc(P, K, C_V, s);  // kick-drift: applied by the kick kernel
   with_lanes([&](auto l) {  // and the next-step BC by this one

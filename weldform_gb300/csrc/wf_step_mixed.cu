@@ -1152,7 +1152,7 @@ void launch_step_mixed(const DevPtrs& P, const DomainConst& K, double* fscratch,
     else launch_accel_mx<false, false>(P, K, ng, gb, s);
   }
   mark(s, staged ? "k_accel_mx_staged" : "k_accel_mx");
-  launch_bc(P, K, C_V, s);
+  launch_bc_before_kick(P, K, s);
   launch_contact_kick(P, K, s);
   if (K.leapfrog) launch_bc(P, K, C_V, s);  // kick-drift: applied by the kick kernel
   if (K.gradcorr) {
