@@ -96,12 +96,75 @@ __device__ __forceinline__ bool bc_value(const DomainTables* T, int id, double t
 #define TMP(c, p) A.Tmp[(size_t)(c) * N + (p)]
 #define QA(c) A.Q[(size_t)(c) * N + i]
 
+// The adjoint gathers split a row over L lanes like the plain form's: lane sums
+// by shuffles, then through shared memory to the first blockDim / L threads,
+// which finish a particle each in full warps (R1's and R3's epilogues are as
+// long as a row).  At 18,258 particles one thread per particle is four warps
+// per SM, too few to cover the FP64 latency.
+// Reverse sweep of 20 steps, ms with 1, 2 and 4 lanes: 25.2, 19.0, 18.4 at 5,682
+// particles; 25.6, 19.4, 18.6 at 9,156; 30.0, 28.7, 29.4 at 18,258; from there
+// the FP64 pipe is full (45.4, 47.0, 47.0 at 32,912).
+static int adj_lanes(long long n) { return n < 14000 ? 4 : (n < 24000 ? 2 : 1); }
+constexpr int ADJ_LANE_BLOCK = 64;  // particles per block with more than one lane
+template <int L, int NS>
+__device__ __forceinline__ bool adj_fold(double (&s)[NS], double (*sh)[L > 1 ? ADJ_LANE_BLOCK : 1], int N, int& i) {
+  if constexpr (L > 1) {
+    const int p = threadIdx.x / L, PB = blockDim.x / L;
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+      for (int off = 1; off < L; off <<= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], off);
+      if (threadIdx.x % L == 0) sh[q][p] = s[q];
+    }
+    __syncthreads();
+    if (threadIdx.x >= PB) return false;
+    i = blockIdx.x * PB + threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < NS; ++q) s[q] = sh[q][threadIdx.x];
+  }
+  return i < N;
+}
+
 // ---------------------------------------------------------------- R1: thermal + radial return
-__global__ void __launch_bounds__(BLOCK) k_adj_thermal_stress(AdjPtrs A, DomainConst K) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= K.N) return;
+// Conduction adjoint sums: d/dT', d/dx' (3), d/drho'.
+__device__ __forceinline__ void adj_conduction(const AdjPtrs& A, const DomainConst& K, int i, int k0, int dk, double (&out)[5]) {
+  if (!K.thermal_solver) return;
   const DevPtrs& S = A.S;
   size_t N = K.N;
+  double lxn[3] = {0, 0, 0}, lrhon = 0.0, ltn = 0.0;
+  const double lci = TMP(J_LC, i), inv_rhoN = 1.0 / FE(C_RHO, i);
+  double xi[3] = {FE(C_X, i), FE(C_X + 1, i), FE(C_X + 2, i)};
+  double hi = col(S, C_H, N, i), ki = col(S, C_KT, N, i), Ti = FE(C_T, i), wi = FE(C_MRHO, i);
+  double inv_hi = 1.0 / hi;
+  int len = S.row_len[i];
+  for (int k = k0; k < len; k += dk) {
+    int e = S.nbr[(size_t)k * N + i];
+    int j = nb_index(e);
+    GeoD g = geo_d(xi, hi, inv_hi, FE(C_X, j), FE(C_X + 1, j), FE(C_X + 2, j), col(S, C_H, N, j));
+    A.gk_end[(size_t)k * N + i] = g.GK;  // R2 reads the same end-state geometry
+    A.dg_end[(size_t)k * N + i] = g.dGr;
+    double lcj = TMP(J_LC, j);
+    double d = lci - lcj;
+    bool up = nb_up(e);  // j has the larger original index: P2 = j
+    double w = up ? FE(C_MRHO, j) : wi;  // m_P2 / rho_P2 at both ends (Thermal.cpp:127-131)
+    double kj = col(S, C_KT, N, j);
+    double kk = 4. * (ki * kj) / (ki + kj);
+    double dT = Ti - FE(C_T, j);
+    ltn += d * w * kk * g.GK;
+    double cx = d * w * kk * dT * g.dGr;
+    lxn[0] += cx * g.x0; lxn[1] += cx * g.x1; lxn[2] += cx * g.x2;
+    if (!up) lrhon += -d * w * kk * dT * g.GK * inv_rhoN;
+  }
+  out[0] = ltn; out[1] = lxn[0]; out[2] = lxn[1]; out[3] = lxn[2]; out[4] = lrhon;
+}
+template <int L>
+__global__ void __launch_bounds__(256) k_adj_thermal_stress(AdjPtrs A, DomainConst K) {
+  __shared__ double sh[5][L > 1 ? ADJ_LANE_BLOCK : 1];
+  const DevPtrs& S = A.S;
+  size_t N = K.N;
+  double sums[5] = {};
+  int i = blockIdx.x * (blockDim.x / L) + threadIdx.x / L;
+  if (i < K.N && icol(S, I_KIND, N, i) == 0) adj_conduction(A, K, i, threadIdx.x % L, L, sums);
+  if (!adj_fold<L>(sums, sh, K.N, i)) return;
   double dt = K.dt;
   if (icol(S, I_KIND, N, i) != 0) {
     for (int c = 0; c < 6; ++c) { LOUT(A_TAU + c) = 0.0; LOUT(A_INC + c) = 0.0; TMP(J_SR + c, i) = 0.0; }
@@ -109,9 +172,9 @@ __global__ void __launch_bounds__(BLOCK) k_adj_thermal_stress(AdjPtrs A, DomainC
     LOUT(A_PLS) = 0.0; LOUT(A_SY) = 0.0; LOUT(A_T) = 0.0; LOUT(A_DTDT) = 0.0; TMP(J_RHON, i) = 0.0;
     return;
   }
-  double lxn[3] = {LIN(A_X, i), LIN(A_X + 1, i), LIN(A_X + 2, i)};
-  double lrhon = LIN(A_RHO, i);
-  double ltn = LIN(A_T, i);
+  double lxn[3] = {LIN(A_X, i) + sums[1], LIN(A_X + 1, i) + sums[2], LIN(A_X + 2, i) + sums[3]};
+  double lrhon = LIN(A_RHO, i) + sums[4];
+  double ltn = LIN(A_T, i) + sums[0];
   double rhoN = FE(C_RHO, i);
   double lqpl = 0.0;
   // ---- M: T' = T + dt dTdt, dTdt' = (cond + q_src + frac q_pl) / (rho' cp)
@@ -121,28 +184,6 @@ __global__ void __launch_bounds__(BLOCK) k_adj_thermal_stress(AdjPtrs A, DomainC
     double inv_rhoN = 1.0 / rhoN;
     lrhon += -FE(C_DTDT, i) * ldT * inv_rhoN;
     if (K.pl_heating) lqpl = K.pl_work_heat_frac * lci;
-    double xi[3] = {FE(C_X, i), FE(C_X + 1, i), FE(C_X + 2, i)};
-    double hi = col(S, C_H, N, i), ki = col(S, C_KT, N, i), Ti = FE(C_T, i), wi = FE(C_MRHO, i);
-    double inv_hi = 1.0 / hi;
-    int len = S.row_len[i];
-    for (int k = 0; k < len; ++k) {
-      int e = S.nbr[(size_t)k * N + i];
-      int j = nb_index(e);
-      GeoD g = geo_d(xi, hi, inv_hi, FE(C_X, j), FE(C_X + 1, j), FE(C_X + 2, j), col(S, C_H, N, j));
-      A.gk_end[(size_t)k * N + i] = g.GK;  // R2 reads the same end-state geometry
-      A.dg_end[(size_t)k * N + i] = g.dGr;
-      double lcj = TMP(J_LC, j);
-      double d = lci - lcj;
-      bool up = nb_up(e);  // j has the larger original index: P2 = j
-      double w = up ? FE(C_MRHO, j) : wi;  // m_P2 / rho_P2 at both ends (Thermal.cpp:127-131)
-      double kj = col(S, C_KT, N, j);
-      double kk = 4. * (ki * kj) / (ki + kj);
-      double dT = Ti - FE(C_T, j);
-      ltn += d * w * kk * g.GK;
-      double cx = d * w * kk * dT * g.dGr;
-      lxn[0] += cx * g.x0; lxn[1] += cx * g.x1; lxn[2] += cx * g.x2;
-      if (!up) lrhon += -d * w * kk * dT * g.GK * inv_rhoN;
-    }
   }
   // ---- K + L: radial return (Particle.cpp:960-1067) and plastic-work heat
   double tau[6], sr[6], rr[3];
@@ -310,30 +351,21 @@ __global__ void __launch_bounds__(BLOCK) k_adj_thermal_stress(AdjPtrs A, DomainC
 }
 
 // ---------------------------------------------------------------- R2: rates + second kick + drift
-__global__ void __launch_bounds__(BLOCK) k_adj_rates_drift(AdjPtrs A, DomainConst K) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= K.N) return;
+// Rate adjoint sums: d/dx' (3), d/dv' (3), and sum L . B for d/drho'.
+__device__ __forceinline__ void adj_rates(const AdjPtrs& A, const DomainConst& K, int i, int k0, int dk, double (&out)[7]) {
   const DevPtrs& S = A.S;
   size_t N = K.N;
-  double dt = K.dt;
-  if (icol(S, I_KIND, N, i) != 0) {
-    for (int c = 0; c < 3; ++c) { TMP(J_VH + c, i) = 0.0; TMP(J_AH + c, i) = 0.0; LOUT(A_X + c) = 0.0; }
-    TMP(J_DRHO, i) = 0.0; LOUT(A_RHO) = 0.0;
-    return;
-  }
   double xi[3] = {FE(C_X, i), FE(C_X + 1, i), FE(C_X + 2, i)};
   double vi[3] = {FE(C_V, i), FE(C_V + 1, i), FE(C_V + 2, i)};
-  double hi = col(S, C_H, N, i), wi = FE(C_MRHO, i), rhoN = FE(C_RHO, i);
+  double hi = col(S, C_H, N, i), wi = FE(C_MRHO, i);
   double inv_hi = 1.0 / hi;
   double li[9];
   for (int c = 0; c < 6; ++c) li[c] = TMP(J_SR + c, i);
   for (int c = 0; c < 3; ++c) li[6 + c] = TMP(J_RR + c, i);
-  double lx[3] = {TMP(J_XN, i), TMP(J_XN + 1, i), TMP(J_XN + 2, i)};
-  double lv[3] = {TMP(J_VN, i), TMP(J_VN + 1, i), TMP(J_VN + 2, i)};
-  double lrhon = TMP(J_RHON, i);
+  double lx[3] = {0, 0, 0}, lv[3] = {0, 0, 0};
   double sumLT = 0.0;
   int len = S.row_len[i];
-  for (int k = 0; k < len; ++k) {
+  for (int k = k0; k < len; k += dk) {
     int j = nb_index(S.nbr[(size_t)k * N + i]);
     GeoD g;
     if (K.thermal_solver) {  // R1 formed this entry's end-state geometry
@@ -366,7 +398,27 @@ __global__ void __launch_bounds__(BLOCK) k_adj_rates_drift(AdjPtrs A, DomainCons
     lv[0] += f * db0; lv[1] += f * db1; lv[2] += f * db2;
     lx[0] += f * dx0 + gq * x0; lx[1] += f * dx1 + gq * x1; lx[2] += f * dx2 + gq * x2;
   }
-  lrhon += -(wi / rhoN) * sumLT;
+  for (int d = 0; d < 3; ++d) { out[d] = lx[d]; out[3 + d] = lv[d]; }
+  out[6] = sumLT;
+}
+template <int L>
+__global__ void __launch_bounds__(256) k_adj_rates_drift(AdjPtrs A, DomainConst K) {
+  __shared__ double sh[7][L > 1 ? ADJ_LANE_BLOCK : 1];
+  const DevPtrs& S = A.S;
+  size_t N = K.N;
+  double sums[7] = {};
+  int i = blockIdx.x * (blockDim.x / L) + threadIdx.x / L;
+  if (i < K.N && icol(S, I_KIND, N, i) == 0) adj_rates(A, K, i, threadIdx.x % L, L, sums);
+  if (!adj_fold<L>(sums, sh, K.N, i)) return;
+  double dt = K.dt;
+  if (icol(S, I_KIND, N, i) != 0) {
+    for (int c = 0; c < 3; ++c) { TMP(J_VH + c, i) = 0.0; TMP(J_AH + c, i) = 0.0; LOUT(A_X + c) = 0.0; }
+    TMP(J_DRHO, i) = 0.0; LOUT(A_RHO) = 0.0;
+    return;
+  }
+  const double lx[3] = {TMP(J_XN, i) + sums[0], TMP(J_XN + 1, i) + sums[1], TMP(J_XN + 2, i) + sums[2]};
+  const double lv[3] = {TMP(J_VN, i) + sums[3], TMP(J_VN + 1, i) + sums[4], TMP(J_VN + 2, i) + sums[5]};
+  const double lrhon = TMP(J_RHON, i) - (FE(C_MRHO, i) / FE(C_RHO, i)) * sums[6];
   double vb[3];
   bool isbc = bc_value(S.tab, icol(S, I_ID, N, i), A.time, vb);
   for (int d = 0; d < 3; ++d) {
@@ -380,25 +432,19 @@ __global__ void __launch_bounds__(BLOCK) k_adj_rates_drift(AdjPtrs A, DomainCons
 }
 
 // ---------------------------------------------------------------- R3: density + first kick + contact
-__global__ void __launch_bounds__(BLOCK) k_adj_density_contact(AdjPtrs A, DomainConst K) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= K.N) return;
+// Density adjoint sums: d/dv_half (3), d/dx (3), d/drho.
+__device__ __forceinline__ void adj_density(const AdjPtrs& A, const DomainConst& K, int i, int k0, int dk, double (&out)[7]) {
   const DevPtrs& S = A.S;
   size_t N = K.N;
-  double dt = K.dt;
-  if (icol(S, I_KIND, N, i) != 0) {
-    for (int c = 0; c < 3; ++c) { TMP(J_AACC + c, i) = 0.0; LOUT(A_V + c) = 0.0; }
-    return;
-  }
   double xi[3] = {col(S, C_X, N, i), col(S, C_X + 1, N, i), col(S, C_X + 2, N, i)};
   double vh[3] = {TXV(TX_VH, i), TXV(TX_VH + 1, i), TXV(TX_VH + 2, i)};
   double hi = col(S, C_H, N, i), rhoi = col(S, C_RHO, N, i), wi = col(S, C_MRHO, N, i);
   double inv_hi = 1.0 / hi, w_rho = -wi / rhoi;
   double ldr = TMP(J_DRHO, i);
-  double lvh[3] = {TMP(J_VH, i), TMP(J_VH + 1, i), TMP(J_VH + 2, i)};
+  double lvh[3] = {0, 0, 0};
   double lx[3] = {0, 0, 0}, lrho = 0.0, D = 0.0;
   int len = S.row_len[i];
-  for (int k = 0; k < len; ++k) {
+  for (int k = k0; k < len; k += dk) {
     int j = nb_index(S.nbr[(size_t)k * N + i]);
     GeoD g = geo_d(xi, hi, inv_hi, col(S, C_X, N, j), col(S, C_X + 1, N, j), col(S, C_X + 2, N, j), col(S, C_H, N, j));
     A.gk_start[(size_t)k * N + i] = g.GK;  // R4 reads the same start-state geometry
@@ -414,7 +460,27 @@ __global__ void __launch_bounds__(BLOCK) k_adj_density_contact(AdjPtrs A, Domain
     lx[0] += Lam * g.GK * b0 + c * g.x0; lx[1] += Lam * g.GK * b1 + c * g.x1; lx[2] += Lam * g.GK * b2 + c * g.x2;
     lrho += ldj * rhoj * w_rho * pd;
   }
-  lrho += ldr * D;
+  for (int d = 0; d < 3; ++d) { out[d] = lvh[d]; out[3 + d] = lx[d]; }
+  out[6] = lrho + ldr * D;
+}
+template <int L>
+__global__ void __launch_bounds__(256) k_adj_density_contact(AdjPtrs A, DomainConst K) {
+  __shared__ double sh[7][L > 1 ? ADJ_LANE_BLOCK : 1];
+  const DevPtrs& S = A.S;
+  size_t N = K.N;
+  double sums[7] = {};
+  int i = blockIdx.x * (blockDim.x / L) + threadIdx.x / L;
+  if (i < K.N && icol(S, I_KIND, N, i) == 0) adj_density(A, K, i, threadIdx.x % L, L, sums);
+  if (!adj_fold<L>(sums, sh, K.N, i)) return;
+  double dt = K.dt;
+  if (icol(S, I_KIND, N, i) != 0) {
+    for (int c = 0; c < 3; ++c) { TMP(J_AACC + c, i) = 0.0; LOUT(A_V + c) = 0.0; }
+    return;
+  }
+  const double xi[3] = {col(S, C_X, N, i), col(S, C_X + 1, N, i), col(S, C_X + 2, N, i)};
+  const double hi = col(S, C_H, N, i), rhoi = col(S, C_RHO, N, i);
+  const double lvh[3] = {TMP(J_VH, i) + sums[0], TMP(J_VH + 1, i) + sums[1], TMP(J_VH + 2, i) + sums[2]};
+  double lx[3] = {sums[3], sums[4], sums[5]}, lrho = sums[6];
   // second BC pass and the first half kick vh = v1 + a1 dt/2
   double vbi[3];
   bool isbc = bc_value(S.tab, icol(S, I_ID, N, i), A.time, vbi);
@@ -600,15 +666,10 @@ __global__ void __launch_bounds__(BLOCK) k_adj_density_contact(AdjPtrs A, Domain
 }
 
 // ---------------------------------------------------------------- R4: acceleration
-__global__ void __launch_bounds__(BLOCK) k_adj_accel(AdjPtrs A, DomainConst K) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= K.N) return;
+// Acceleration adjoint sums: d/dx (3), d/dv (3), d/d(Sigma/rho^2) (6), d/drho, d/dCs.
+__device__ __forceinline__ void adj_accel(const AdjPtrs& A, const DomainConst& K, int i, int k0, int dk, double (&out)[14]) {
   const DevPtrs& S = A.S;
   size_t N = K.N;
-  if (icol(S, I_KIND, N, i) != 0) {
-    for (int c = 0; c < 6; ++c) LOUT(A_SIG + c) = 0.0;
-    return;
-  }
   double xi[3] = {col(S, C_X, N, i), col(S, C_X + 1, N, i), col(S, C_X + 2, N, i)};
   double vi[3] = {col(S, C_V, N, i), col(S, C_V + 1, N, i), col(S, C_V + 2, N, i)};
   double hi = col(S, C_H, N, i), rhoi = col(S, C_RHO, N, i), csi = col(S, C_CS, N, i), mi = col(S, C_MASS, N, i);
@@ -619,7 +680,7 @@ __global__ void __launch_bounds__(BLOCK) k_adj_accel(AdjPtrs A, DomainConst K) {
   double lx[3] = {0, 0, 0}, lv[3] = {0, 0, 0}, lrho = 0.0, lcs = 0.0;
   double lSs[6] = {0, 0, 0, 0, 0, 0};
   int len = S.row_len[i];
-  for (int k = 0; k < len; ++k) {
+  for (int k = k0; k < len; k += dk) {
     int j = nb_index(S.nbr[(size_t)k * N + i]);
     double mj = col(S, C_MASS, N, j);
     double Gm[3];
@@ -670,14 +731,36 @@ __global__ void __launch_bounds__(BLOCK) k_adj_accel(AdjPtrs A, DomainConst K) {
       lv[0] += cb * g.x0; lv[1] += cb * g.x1; lv[2] += cb * g.x2;
     }
   }
+  for (int d = 0; d < 3; ++d) { out[d] = lx[d]; out[3 + d] = lv[d]; }
+  for (int c = 0; c < 6; ++c) out[6 + c] = lSs[c];
+  out[12] = lrho; out[13] = lcs;
+}
+template <int L>
+__global__ void __launch_bounds__(256) k_adj_accel(AdjPtrs A, DomainConst K) {
+  __shared__ double sh[14][L > 1 ? ADJ_LANE_BLOCK : 1];
+  const DevPtrs& S = A.S;
+  size_t N = K.N;
+  double sums[14] = {};
+  int i = blockIdx.x * (blockDim.x / L) + threadIdx.x / L;
+  if (i < K.N && icol(S, I_KIND, N, i) == 0) adj_accel(A, K, i, threadIdx.x % L, L, sums);
+  if (!adj_fold<L>(sums, sh, K.N, i)) return;
+  if (icol(S, I_KIND, N, i) != 0) {
+    for (int c = 0; c < 6; ++c) LOUT(A_SIG + c) = 0.0;
+    return;
+  }
+  const double rhoi = col(S, C_RHO, N, i);
+  const double* lx = sums;
+  const double* lv = sums + 3;
+  const double* lSs = sums + 6;
+  double lrho = sums[12];
   // S_i = Sigma_i / rho_i^2
   double inv2 = 1.0 / (rhoi * rhoi);
   double ls = 0.0;
-  for (int c = 0; c < 6; ++c) { LOUT(A_SIG + c) = lSs[c] * inv2; ls += lSs[c] * Si[c]; }
+  for (int c = 0; c < 6; ++c) { LOUT(A_SIG + c) = lSs[c] * inv2; ls += lSs[c] * col(S, C_SRHO + c, N, i); }
   lrho += -2.0 / rhoi * ls;
   for (int d = 0; d < 3; ++d) { LOUT(A_X + d) += lx[d]; LOUT(A_V + d) += lv[d]; }
   LOUT(A_RHO) += lrho;
-  QA(Q_CS) += lcs;
+  QA(Q_CS) += sums[13];
 }
 
 // ---------------------------------------------------------------- bookkeeping
@@ -750,22 +833,31 @@ __global__ void k_adj_conduction_factor(AdjPtrs A, DomainConst K) {
   TMP(J_LC, i) = icol(S, I_KIND, N, i) == 0 ? LIN(A_DTDT, i) / (FE(C_RHO, i) * col(S, C_CPT, N, i)) : 0.0;
 }
 
+template <int L>
+static void launch_adjoint_kernels(const AdjPtrs& A, const DomainConst& K, int nb, int tb, cudaStream_t s) {
+  k_adj_thermal_stress<L><<<nb, tb, 0, s>>>(A, K);
+  mark(s, "k_adj_thermal_stress");
+  k_adj_rates_drift<L><<<nb, tb, 0, s>>>(A, K);
+  mark(s, "k_adj_rates_drift");
+  k_adj_density_contact<L><<<nb, tb, 0, s>>>(A, K);
+  mark(s, "k_adj_density_contact");
+  k_adj_accel<L><<<nb, tb, 0, s>>>(A, K);
+  mark(s, "k_adj_accel");
+}
 void launch_adjoint_step(const AdjPtrs& A, const DomainConst& K, cudaStream_t s) {
-  // one thread per particle, no block-level sums: the domain's per-particle block size
+  // no block-level sums: the domain's per-particle block size with one lane
   int tb = K.pblock > 0 ? K.pblock : BLOCK;
   int nb = nblk(K.N, tb);
   if (K.thermal_solver) {
     k_adj_conduction_factor<<<nb, tb, 0, s>>>(A, K);
     mark(s, "k_adj_conduction_factor");
   }
-  k_adj_thermal_stress<<<nb, tb, 0, s>>>(A, K);
-  mark(s, "k_adj_thermal_stress");
-  k_adj_rates_drift<<<nb, tb, 0, s>>>(A, K);
-  mark(s, "k_adj_rates_drift");
-  k_adj_density_contact<<<nb, tb, 0, s>>>(A, K);
-  mark(s, "k_adj_density_contact");
-  k_adj_accel<<<nb, tb, 0, s>>>(A, K);
-  mark(s, "k_adj_accel");
+  const int nl = nblk(K.N, ADJ_LANE_BLOCK);
+  switch (adj_lanes(K.N)) {
+    case 2: launch_adjoint_kernels<2>(A, K, nl, 2 * ADJ_LANE_BLOCK, s); break;
+    case 4: launch_adjoint_kernels<4>(A, K, nl, 4 * ADJ_LANE_BLOCK, s); break;
+    default: launch_adjoint_kernels<1>(A, K, nb, tb, s);
+  }
 }
 void launch_unpermute(const int* perm, const double* src, double* dst, int ncol, int N, cudaStream_t s) {
   k_unpermute<<<152 * 4, 512, 0, s>>>(perm, src, dst, ncol, N);
