@@ -271,6 +271,7 @@ struct DomainConst {
   int auto_ts, auto_ts_acc;  // adaptive time step: velocity / acceleration criteria
   double CFL, sqrt_h_a;      // their coefficients (Domain::CFL, Domain::sqrt_h_a)
   int av_uniform;      // 1 when every solid particle has the same Alpha and Beta
+  int av_beta_zero, av_zero;  // uniform constants with beta 0; with both 0
   float av_alpha, av_beta;  // those values (the mixed acceleration gather skips their loads)
   // 1 when the two particles of every pair have the same mass: the mass is
   // uniform, or uniform within each batched specimen (no pair links two

@@ -1218,6 +1218,8 @@ struct wf_domain {
     }
     K.av_alpha = (float)a0;
     K.av_beta = (float)b0;
+    K.av_beta_zero = K.av_uniform && b0 == 0.0;
+    K.av_zero = K.av_beta_zero && a0 == 0.0;
     K.uni = (K.m_pair && h_uniform && cs_uniform && h0 > 0) ? 1 : 0;
     K.h_f = (float)h0;
     K.cs_f = (float)c0;

@@ -158,10 +158,12 @@ __device__ __forceinline__ PairGeo pair_geo(double xi0, double xi1, double xi2, 
 // cycles and SM; 85-87 % of that rate before, with 71 of them per pair in the
 // acceleration, 15 in the density and 80 in the rates).  The uniform-particle
 // forms below (DomainConst::uni, no tensile term, no gradient correction) take
-// 39, 11 and 41: constants of the one h are formed on the host, compares read
-// the exponent word, the pair mass is a factor of the whole sum, and the nine
+// 45, 13 and 44 (their times at 240,300 particles: 1849 -> 1165, 404 -> 333 and
+// 2092 -> 1267 us): constants of the one h are formed on the host, compares
+// read the exponent word, the pair mass is a factor of the whole sum, the nine
 // products v_k x_l are summed once instead of in symmetric and antisymmetric
-// parts.  Same FP64 throughout.
+// parts, and what a workload leaves out is left out at compile time.  Same
+// FP64 throughout.
 struct UniGeo {
   double r2, ir, GK;
 };
@@ -361,6 +363,11 @@ __device__ __forceinline__ void accel_sums(const DevPtrs& P, const DomainConst& 
   out[0] = a0; out[1] = a1; out[2] = a2;
 }
 // Uniform particles: a = m (sum g S_j + S_i sum g + sum PI g), g = GK x_ij.
+// REUSE: GradKernel comes from the last step's rate pass; VISC 0: no viscosity,
+// 1: uniform constants with beta 0, 2: anything.  Compile-time, because an
+// instruction that is predicated off in the loop still takes its slot of the
+// FP64 pipe.
+template <bool REUSE, int VISC>
 __device__ __forceinline__ void accel_sums_uni(const DevPtrs& P, const DomainConst& K, int i, int k0, int dk,
                                                double out[3]) {
   const size_t N = K.N;
@@ -368,33 +375,37 @@ __device__ __forceinline__ void accel_sums_uni(const DevPtrs& P, const DomainCon
   const double vi0 = col(P, C_V, N, i), vi1 = col(P, C_V + 1, N, i), vi2 = col(P, C_V + 2, N, i);
   const double rhoi = col(P, C_RHO, N, i), h = col(P, C_H, N, i), cs = col(P, C_CS, N, i);
   const double Alpha = col(P, C_ALPHA, N, i), Beta = col(P, C_BETA, N, i);
-  const bool visc = K.av_uniform ? Alpha != 0.0 || Beta != 0.0 : true;
-  const double eps = 0.01 * h * h;
+  const double eps = 0.01 * h * h, f1 = 2.0 * h * (Alpha * cs);
   double a0 = 0, a1 = 0, a2 = 0, G0 = 0, G1 = 0, G2 = 0;
   const int len = P.row_len[i];
-  const bool reuse = P.st->gk_valid && !P.st->do_search;  // as in accel_sums
   int next = k0 < len ? P.nbr[(size_t)k0 * N + i] : 0;
   for (int k = k0; k < len; k += dk) {
     const int j = nb_index(next);
     if (k + dk < len) next = P.nbr[(size_t)(k + dk) * N + i];
     const double x0 = xi0 - col(P, C_X, N, j), x1 = xi1 - col(P, C_X + 1, N, j), x2 = xi2 - col(P, C_X + 2, N, j);
     double GK;
-    if (reuse) {
+    if constexpr (REUSE) {
       GK = P.gk[(size_t)k * N + i];
     } else {
       GK = uni_geo(K, x0, x1, x2).GK;
       P.gk[(size_t)k * N + i] = GK;  // for the density pass (same x(n), h)
     }
     const double g0 = GK * x0, g1 = GK * x1, g2 = GK * x2;
-    if (visc) {
+    if constexpr (VISC > 0) {
       const double dvx = (vi0 - col(P, C_V, N, j)) * x0 + (vi1 - col(P, C_V + 1, N, j)) * x1 + (vi2 - col(P, C_V + 2, N, j)) * x2;
       if (__double2hiint(dvx) < 0) {  // the sign (-0 adds nothing): MU (alpha C + beta MU) / rho_bar, MU = h dvx / Dn
-        const double al = K.av_uniform ? Alpha : 0.5 * (Alpha + col(P, C_ALPHA, N, j));
-        const double be = K.av_uniform ? Beta : 0.5 * (Beta + col(P, C_BETA, N, j));
         const double Dn = eps + x0 * x0 + x1 * x1 + x2 * x2;
-        const double hv = h * dvx, rs = rhoi + col(P, C_RHO, N, j);
-        double num = 2.0 * hv * (al * cs), den = Dn * rs;
-        if (be != 0.0) { num = 2.0 * hv * (al * cs * Dn + be * hv); den *= Dn; }
+        const double rs = rhoi + col(P, C_RHO, N, j);
+        double num, den = Dn * rs;
+        if constexpr (VISC == 1) {
+          num = f1 * dvx;
+        } else {
+          const double al = K.av_uniform ? Alpha : 0.5 * (Alpha + col(P, C_ALPHA, N, j));
+          const double be = K.av_uniform ? Beta : 0.5 * (Beta + col(P, C_BETA, N, j));
+          const double hv = h * dvx;
+          num = 2.0 * hv * (al * cs * Dn + be * hv);
+          den *= Dn;
+        }
         const double PIs = num / den;
         a0 += PIs * g0; a1 += PIs * g1; a2 += PIs * g2;
       }
@@ -413,15 +424,20 @@ __device__ __forceinline__ void accel_sums_uni(const DevPtrs& P, const DomainCon
 }
 // L lanes per particle: with one, a small domain's few warps wait out each
 // other's FP64 latency (8,004 particles: two warps per SM).
-template <bool UNI, int L>
+// UNI: -1 the general form, else accel_sums_uni's VISC.
+template <int UNI, int L>
 __global__ void __launch_bounds__(512) k_accel(DevPtrs P, DomainConst K) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / L, sub = t % L;
   const size_t N = K.N;
   const bool live = i < K.N;
   double a[3] = {0.0, 0.0, 0.0};  // StartAcceleration resets a for every particle
   if (live && icol(P, I_KIND, N, i) == 0) {
-    if (UNI) accel_sums_uni(P, K, i, sub, L, a);
-    else accel_sums(P, K, i, sub, L, a);
+    if constexpr (UNI < 0) {
+      accel_sums(P, K, i, sub, L, a);
+    } else {  // the last step's rate pass formed GradKernel at these positions and rows?
+      if (P.st->gk_valid && !P.st->do_search) accel_sums_uni<true, UNI>(P, K, i, sub, L, a);
+      else accel_sums_uni<false, UNI>(P, K, i, sub, L, a);
+    }
   }
   if (L > 1) for (int d = 0; d < 3; ++d) a[d] = lane_sum<L>(a[d]);
   if (live && sub == 0)
@@ -774,6 +790,7 @@ __global__ void __launch_bounds__(BLOCK) k_contact_kick(DevPtrs P, DomainConst K
 
 // ---------------------------------------------------------------- density + drift + kick
 // rho_i dot / rho_i (with gradient correction: rho dot) over entries k0, k0 + dk, ...
+template <bool GC>
 __device__ __forceinline__ double density_sum(const DevPtrs& P, const DomainConst& K, int i, int k0, int dk) {
   const size_t N = K.N;
   const double xi0 = col(P, C_X, N, i), xi1 = col(P, C_X + 1, N, i), xi2 = col(P, C_X + 2, N, i);
@@ -789,7 +806,7 @@ __device__ __forceinline__ double density_sum(const DevPtrs& P, const DomainCons
     const double GK = P.gk[(size_t)k * N + i];
     const double x0 = xi0 - col(P, C_X, N, j), x1 = xi1 - col(P, C_X + 1, N, j), x2 = xi2 - col(P, C_X + 2, N, j);
     const double v0 = vi0 - col(P, C_V, N, j), v1 = vi1 - col(P, C_V + 1, N, j), v2 = vi2 - col(P, C_V + 2, N, j);
-    if (K.gradcorr) {  // locking form m_j (rho_i/rho_j) v_ij . vc_i (InteractionAlt.cpp:589-605)
+    if constexpr (GC) {  // locking form m_j (rho_i/rho_j) v_ij . vc_i (InteractionAlt.cpp:589-605)
       double vc[3];
       corr_grad(P, N, i, GK, x0, x1, x2, vc);
       dd += col(P, C_MASS, N, j) * (rhoi / col(P, C_RHO, N, j)) * (v0 * vc[0] + v1 * vc[1] + v2 * vc[2]);
@@ -801,14 +818,14 @@ __device__ __forceinline__ double density_sum(const DevPtrs& P, const DomainCons
 }
 // L lanes per particle; the lanes' sums go through shared memory, so that the
 // first blockDim / L threads finish a particle each in full warps.
-template <int L>
+template <bool GC, int L>
 __global__ void __launch_bounds__(512) k_density_drift(DevPtrs P, DomainConst K) {
   __shared__ double s_dd[L > 1 ? 256 : 1];
   const int PB = blockDim.x / L;  // particles per block
   const size_t N = K.N;
   int i = blockIdx.x * PB + threadIdx.x / L;
   double dd = 0.0;
-  if (i < K.N && icol(P, I_KIND, N, i) == 0) dd = density_sum(P, K, i, threadIdx.x % L, L);
+  if (i < K.N && icol(P, I_KIND, N, i) == 0) dd = density_sum<GC>(P, K, i, threadIdx.x % L, L);
   if (L > 1) {
     dd = lane_sum<L>(dd);
     if (threadIdx.x % L == 0) s_dd[threadIdx.x / L] = dd;
@@ -825,7 +842,7 @@ __global__ void __launch_bounds__(512) k_density_drift(DevPtrs P, DomainConst K)
   for (int d = 0; d < 3; ++d) { v[d] = col(P, C_V + d, N, i); x[d] = col(P, C_X + d, N, i); }
   if (P.tx)
     for (int d = 0; d < 3; ++d) P.tx[(size_t)(TX_VH + d) * N + i] = v[d];
-  if (solid && !K.gradcorr) dd *= rhoi;
+  if (solid && !GC) dd *= rhoi;
   colw(P, C_DRHO, N, i) = dd;
   double rn = rhoi + dt * dd;
   colw(P, C_RHON, N, i) = rn;
@@ -950,13 +967,14 @@ __device__ __forceinline__ void rate_sums(const DevPtrs& P, const DomainConst& K
   R.dkin = dkin; R.cond = cond;
 }
 // The same for uniform particles without gradient correction.
+template <bool THERMAL>
 __device__ __forceinline__ void rate_sums_uni(const DevPtrs& P, const DomainConst& K, int i, int k0, int dk, Rates& R) {
   const size_t N = K.N;
   const double xi0 = col(P, C_XN, N, i), xi1 = col(P, C_XN + 1, N, i), xi2 = col(P, C_XN + 2, N, i);
   const double vi0 = col(P, C_VN, N, i), vi1 = col(P, C_VN + 1, N, i), vi2 = col(P, C_VN + 2, N, i);
   const double pri = col(P, C_PR2N, N, i);
   double Ti = 0.0, ki = 0.0, mrhoi = 0.0;
-  if (K.thermal_solver) { Ti = col(P, C_TN, N, i); ki = col(P, C_KT, N, i); mrhoi = col(P, C_MRHON, N, i); }
+  if constexpr (THERMAL) { Ti = col(P, C_TN, N, i); ki = col(P, C_KT, N, i); mrhoi = col(P, C_MRHON, N, i); }
   double M[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // sum (m_j / rho_j) GK v_k x_l
   double dkin = 0.0, cond = 0.0;
   const int len = P.row_len[i];
@@ -977,7 +995,7 @@ __device__ __forceinline__ void rate_sums_uni(const DevPtrs& P, const DomainCons
     M[0] += u0 * x0; M[1] += u0 * x1; M[2] += u0 * x2;
     M[3] += u1 * x0; M[4] += u1 * x1; M[5] += u1 * x2;
     M[6] += u2 * x0; M[7] += u2 * x1; M[8] += u2 * x2;
-    if (K.thermal_solver) {
+    if constexpr (THERMAL) {
       // 4 ki kj / (ki + kj) (Ti - Tj) x.(GK x) / r^2 with x.x = r^2; the
       // reference's 0/0 of coincident particles stays a NaN
       const double kj = col(P, C_KT, N, j);
@@ -995,7 +1013,8 @@ __device__ __forceinline__ void rate_sums_uni(const DevPtrs& P, const DomainCons
 // L lanes per particle in the gather; the lanes' sums go through shared memory,
 // so that the first blockDim / L threads update a particle each in full warps
 // (the update is ~270 FP64 instructions, as many as a lane's share of a row).
-template <bool UNI, int L>
+// UNI: 0 the general gather, 1 uniform particles, 2 with conduction.
+template <int UNI, int L>
 __global__ void __launch_bounds__(L > 1 ? 512 : BLOCK) k_rate_stress(DevPtrs P, DomainConst K) {
   __shared__ double sh[6 * 32];
   __shared__ double s_r[L > 1 ? 11 : 1][L > 1 ? 256 : 1];
@@ -1006,7 +1025,7 @@ __global__ void __launch_bounds__(L > 1 ? 512 : BLOCK) k_rate_stress(DevPtrs P, 
   Rates R;
   int i = blockIdx.x * PB + threadIdx.x / L;
   if (i < K.N && icol(P, I_KIND, N, i) == 0) {
-    if (UNI) rate_sums_uni(P, K, i, threadIdx.x % L, L, R);
+    if (UNI > 0) rate_sums_uni<(UNI > 1)>(P, K, i, threadIdx.x % L, L, R);
     else rate_sums(P, K, i, threadIdx.x % L, L, R);
   }
   if constexpr (L > 1) {
@@ -1460,18 +1479,24 @@ void launch_tensile(const DevPtrs& P, const DomainConst& K, cudaStream_t s) {
   mark(s, "k_tensile");
 }
 
-template <bool UNI, int L>
+template <int L>
 static void launch_accel64(const DevPtrs& P, const DomainConst& K, cudaStream_t s) {
-  k_accel<UNI, L><<<K.nblocks, K.pblock * L, 0, s>>>(P, K);
+  const int g = K.nblocks, t = K.pblock * L;
+  if (!K.uni || K.ti || K.gradcorr) k_accel<-1, L><<<g, t, 0, s>>>(P, K);
+  else if (K.av_uniform && K.av_zero) k_accel<0, L><<<g, t, 0, s>>>(P, K);
+  else if (K.av_uniform && K.av_beta_zero) k_accel<1, L><<<g, t, 0, s>>>(P, K);
+  else k_accel<2, L><<<g, t, 0, s>>>(P, K);
 }
-template <bool UNI, int L>
+template <int L>
 static void launch_rate64(const DevPtrs& P, const DomainConst& K, cudaStream_t s) {
-  k_rate_stress<UNI, L><<<K.nblocks, K.pblock * L, 0, s>>>(P, K);
+  const int g = K.nblocks, t = K.pblock * L;
+  if (!K.uni || K.gradcorr) k_rate_stress<0, L><<<g, t, 0, s>>>(P, K);
+  else if (!K.thermal_solver) k_rate_stress<1, L><<<g, t, 0, s>>>(P, K);
+  else k_rate_stress<2, L><<<g, t, 0, s>>>(P, K);
 }
 void launch_step_fp64_body(const DevPtrs& P, const DomainConst& K, cudaStream_t s) {
   // lanes per particle within blocks of at most 512 threads
   const int L = K.lanes64 > 1 && K.pblock * K.lanes64 <= 512 ? K.lanes64 : 1;
-  const bool uni_a = K.uni && !K.ti && !K.gradcorr, uni_r = K.uni && !K.gradcorr;
   auto with_lanes = [&](auto f) {
     switch (L) {
       case 2: f(std::integral_constant<int, 2>{}); break;
@@ -1482,8 +1507,7 @@ void launch_step_fp64_body(const DevPtrs& P, const DomainConst& K, cudaStream_t 
   launch_tensile(P, K, s);
   with_lanes([&](auto l) {
     constexpr int LL = decltype(l)::value;
-    if (uni_a) launch_accel64<true, LL>(P, K, s);
-    else launch_accel64<false, LL>(P, K, s);
+    launch_accel64<LL>(P, K, s);
   });
   mark(s, "k_accel");
   launch_bc_before_kick(P, K, s);
@@ -1491,13 +1515,13 @@ void launch_step_fp64_body(const DevPtrs& P, const DomainConst& K, cudaStream_t 
   if (K.leapfrog) launch_bc(P, K, C_V, s);  // kick-drift: applied by the kick kernel
   with_lanes([&](auto l) {  // and the next-step BC by this one
     constexpr int LL = decltype(l)::value;
-    k_density_drift<LL><<<K.nblocks, K.pblock * LL, 0, s>>>(P, K);
+    if (K.gradcorr) k_density_drift<true, LL><<<K.nblocks, K.pblock * LL, 0, s>>>(P, K);
+    else k_density_drift<false, LL><<<K.nblocks, K.pblock * LL, 0, s>>>(P, K);
   });
   mark(s, "k_density_drift");
   with_lanes([&](auto l) {
     constexpr int LL = decltype(l)::value;
-    if (uni_r) launch_rate64<true, LL>(P, K, s);
-    else launch_rate64<false, LL>(P, K, s);
+    launch_rate64<LL>(P, K, s);
   });
   mark(s, "k_rate_stress");
   launch_step_tail(P, K, s);
