@@ -149,7 +149,20 @@ __device__ __forceinline__ float d2f(double v) {
   }
   return __double2float_rn(v);
 }
-// Float-float split of a double: hi = fl(v), lo = fl(v - hi).
+// Float-float split of a double: hi = fl(v), lo = fl(v - hi).  This form is for
+// ff_split3: it sets odd where v is neither zero nor in its range.
+__device__ __forceinline__ void ff_split_int(double v, float& hi, float& lo, bool& odd) {
+  const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v), a = h & 0x7fffffffu;
+  const bool normal = a - 0x3b500000u < 0x0c800000u;  // 2^-74 <= |v| < 2^126: the remainder's last bit is a normal FP32 too
+  odd = odd || !(normal || (a | l) == 0u);
+  const unsigned lsb = (l >> 29) & 1u, sign = h & 0x80000000u;
+  const unsigned long long r = (((unsigned long long)a << 32) | l) + 0x0fffffffu + lsb;
+  hi = __uint_as_float((normal ? (unsigned)(r >> 29) - 0xc0000000u : 0u) | sign);
+  // v - hi in units of the last place of v: the low 29 bits, less 2^29 where they rounded up
+  const unsigned low = l & 0x1fffffffu, up = (low + 0x0fffffffu + lsb) & 0x20000000u;
+  const unsigned scale = normal ? (((a >> 20) - 948u) << 23) | sign : 0u;  // 2^(exponent - 52)
+  lo = (float)((int)low - (int)up) * __uint_as_float(scale);
+}
 __device__ __forceinline__ void ff_split(double v, float& hi, float& lo) {
   const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v), a = h & 0x7fffffffu;
   if (a - 0x3b500000u < 0x0c800000u) {  // 2^-74 <= |v| < 2^126: the remainder's last bit is a normal FP32 too
@@ -165,6 +178,20 @@ __device__ __forceinline__ void ff_split(double v, float& hi, float& lo) {
   if ((a | l) == 0u) { hi = __uint_as_float(h); lo = 0.0f; return; }
   hi = __double2float_rn(v);
   lo = __double2float_rn(v - (double)hi);
+}
+// Three splits with one vote, so that a warp branches over the conversions
+// instead of running them predicated off, which still takes their slots of the
+// FP64 pipe (the kick kernel, whose work this is: 37.5 -> 31.4 us at 982,072
+// particles, with contact 69 -> 59 us at 1,171,832; the rate-stress and density
+// kernels lost more to the registers that grouping holds).
+__device__ __forceinline__ void ff_split3(const double v[3], float hi[3], float lo[3]) {
+  bool odd = false;
+  for (int d = 0; d < 3; ++d) ff_split_int(v[d], hi[d], lo[d], odd);
+  if (__any_sync(__activemask(), odd))
+    for (int d = 0; d < 3; ++d) {
+      hi[d] = __double2float_rn(v[d]);
+      lo[d] = __double2float_rn(v[d] - (double)hi[d]);
+    }
 }
 // Low-half group: x = (xlo0, xlo1), y = (xlo2, vlo0), z = (vlo1, vlo2) as bf16
 // pairs (first value in the low 16 bits), w = a float.  A bf16 is the upper
@@ -201,7 +228,7 @@ __device__ __forceinline__ void rec_set_v(const DevPtrs& P, size_t N, int i, int
 __device__ __forceinline__ void rec_set_v3(const DevPtrs& P, size_t N, int i, const double v[3]) {
   float4* r = P.rc + i;
   float h[3], l[3];
-  for (int d = 0; d < 3; ++d) ff_split(v[d], h[d], l[d]);
+  ff_split3(v, h, l);
   *rec_v_hi(r, N, 0) = h[0];
   *reinterpret_cast<float2*>(r + (size_t)RC_VW * N) = make_float2(h[1], h[2]);
   *lo_v_half(r + (size_t)RC_L * N, 0) = bf16_bits(l[0]);
