@@ -69,3 +69,28 @@ def test_box_rows_and_acceleration(box):
         d.close()
     assert out[0][0] == out[1][0]
     assert rel_l2(out[0][1], out[1][1]) <= 1.2e-5
+
+
+@pytest.mark.parametrize("skin", [0, 1])
+@pytest.mark.parametrize("hfac", [0.55, 0.7, 0.9, 1.2, 1.35])
+def test_rows_over_cell_occupancies(hfac, skin):
+    """From cells of one particle (more than 32 non-empty cells in a stencil,
+    every candidate opening one) to cells of twenty (none opening in some
+    rounds of 32), with and without the superset: rows equal to the oracle's."""
+    out = []
+    for d in (gpu_domain(), oracle_domain()):
+        if not out:
+            d.set_f64("nb_skin", 0.1 if skin else 0.0)
+        r = 0.00025
+        d.AddBoxLength(0, (0.0, 0.0, 0.0), 0.005, 0.004, 0.006, r, 7850.0, hfac * 2 * r, 1, 0, False, False)
+        n = d.particle_count
+        d.set_array("x", d.get_array("x") + np.random.default_rng(3).uniform(-0.1, 0.1, (n, 3)) * r)
+        for f, v in (("G", 7.7e10), ("Cs", 4600.0), ("Fail", 1), ("Sigmay", 3e8)):
+            d.set_particles(f, v)
+        d.prepare(2e-8)
+        d.set_array("x", d.get_array("x") * [1.0, 1.02, 0.97])
+        d.neighbour_search()
+        out.append(rows(*d.neighbours()))
+        d.close()
+    assert out[0] == out[1]
+    assert sum(len(r) for r in out[0]) > 0

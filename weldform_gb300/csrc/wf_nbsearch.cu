@@ -437,10 +437,13 @@ __global__ void __launch_bounds__(FILL_WARPS * 32) k_nbr_fill(DevPtrs P, DomainC
   // With the superset valid the filter forms the rows of the specimens that
   // search; this pass then only puts back the rows of those that do not.
   const bool keep_only = !SUPER && K.skin_on && P.st->sup_valid;
-  __shared__ __align__(16) unsigned s_key[FILL_ROWS][FILL_SLOTS];
+  constexpr int W = SUPER ? 5 : 3, NC = W * W * W;  // stencil
+  __shared__ __align__(16) unsigned s_key[FILL_WARPS][FILL_SLOTS];
   __shared__ int s_idx[FILL_ROWS][FILL_SLOTS];
+  __shared__ int2 s_rng[FILL_WARPS][NC];  // first candidate and count of a row's non-empty cells
   __shared__ int s_len[FILL_ROWS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
   size_t N = K.N;
   const int* ID = P.i + I_ID * N;
   const int* orig = P.i + I_ORIG * N;
@@ -452,15 +455,25 @@ __global__ void __launch_bounds__(FILL_WARPS * 32) k_nbr_fill(DevPtrs P, DomainC
   const int i0 = grp * FILL_ROWS;
   // Each warp builds FILL_PER_WARP consecutive rows, one after the other, so
   // the block barrier below averages the warps' row costs over several rows.
+  // Their cells, read for all of them at once: each is the end of a chain of
+  // three loads.
+  int key_l = 0, lin_l = 0;
+  {
+    const int il = i0 + w * FILL_PER_WARP + lane;
+    if (lane < FILL_PER_WARP && il < K.N) {
+      key_l = P.i[I_CELL * N + P.perm[il]];
+      if (key_l < K.ncells) lin_l = P.cell_lin[key_l];
+    }
+  }
   for (int rr = 0; rr < FILL_PER_WARP; ++rr) {
   const int row = w * FILL_PER_WARP + rr;
   const int i = i0 + row;
-  unsigned* rkey = &s_key[row][0];
+  unsigned* rkey = &s_key[w][0];
   int* ridx = &s_idx[row][0];
   int cnt = 0, split = 0;
   bool overflow = false, link = false;
   // A particle in a shadow bucket (non-finite position) has an empty row.
-  const int key_i = i < K.N ? P.i[I_CELL * N + P.perm[i]] : 0;
+  const int key_i = __shfl_sync(0xffffffffu, key_l, rr), lin = __shfl_sync(0xffffffffu, lin_l, rr);
   // Batched domain: a specimen that does not search keeps its rows (saved by
   // k_rows_save in canonical order; their keys here keep that order).
   const bool keep = !SUPER && K.nspec > 0 && i < K.N && !P.sp[P.i[I_SPEC * N + i]].do_search;
@@ -482,73 +495,84 @@ __global__ void __launch_bounds__(FILL_WARPS * 32) k_nbr_fill(DevPtrs P, DomainC
     // The particle's cell: the key it was sorted by (k_cell_keys evaluated the
     // reference's FP64 cell formula once per particle), mapped back to grid
     // coordinates.
-    int lin = P.cell_lin[key_i];
     int c[3] = {lin / (K.CellNo[1] * K.CellNo[2]), (lin / K.CellNo[2]) % K.CellNo[1], lin % K.CellNo[2]};
     int idi = ID[i], oi = orig[i], mi = material[i];
     bool ci = K.contact && is_contact_id(K, idi);
     const int spec_i = !SUPER && K.nspec > 0 ? P.i[I_SPEC * N + i] : 0;
-    // Lane c < 27 fetches the range of neighbour cell c; a warp scan of the
-    // counts flattens the candidates so all lanes work on every iteration.
-    // A cell whose box lies farther from x_i than the largest pair radius
-    // Cellfac * hmax holds no neighbour and is left out (about a quarter of
-    // the candidates: most corner and some edge cells).  Boxes of the
-    // outermost cells extend to infinity outwards, since the cell index is
-    // clamped there.
-    // The superset's stencil is 5 x 5 x 5 cells, taken 32 cells per round.
-    constexpr int W = SUPER ? 5 : 3, NC = W * W * W, ROUNDS = (NC + 31) / 32;
+    // Cells of the stencil, 32 per round.  A cell whose box lies farther from
+    // x_i than the largest pair radius holds no neighbour and is left out
+    // (about a quarter of the candidates of the 27-cell stencil, most of the
+    // outer cells of the 125-cell one).  Boxes of the outermost cells extend
+    // to infinity outwards, since the cell index is clamped there.  The
+    // distance is a sum over the axes: lane W * d + q holds the square of the
+    // distance along axis d to the stencil's layer q (NaN off the grid).
+    // FP32 on the prefilter coordinates x - BLPF; the radius carries a margin
+    // above the FP32 rounding of those coordinates and of the cell bounds.
     const float skip_r2 = SUPER ? K.sup_skip_r2 : K.cell_skip_r2;
-    for (int round = 0; round < ROUNDS; ++round) {
-    const int nq = NC - 32 * round < 32 ? NC - 32 * round : 32;  // stencil cells in this round
-    const int qc = 32 * round + lane;
-    int cs = 0, cc = 0;
-    if (lane < nq) {
-      int q3[3] = {c[0] + qc / (W * W) - W / 2, c[1] + (qc / W) % W - W / 2, c[2] + qc % W - W / 2};
-      if (q3[0] >= 0 && q3[0] < K.CellNo[0] && q3[1] >= 0 && q3[1] < K.CellNo[1] && q3[2] >= 0 && q3[2] < K.CellNo[2]) {
-        // FP32 on the prefilter coordinates x - BLPF (GB300 runs FP64 at 1/64
-        // of the FP32 rate); the radius carries a margin above the FP32
-        // rounding of those coordinates and of the cell bounds.
-        const float xf[3] = {pi.x, pi.y, pi.z};
-        float g2 = 0.f;
-        bool inside = true;  // a particle outside the grid (clamped cell) keeps all 27 cells
-        for (int d = 0; d < 3; ++d) {
-          float lo = (float)q3[d] * K.CellSizef[d], hi = lo + K.CellSizef[d];
-          float g = 0.f;
-          if (q3[d] > 0 && xf[d] < lo) g = lo - xf[d];
-          if (q3[d] < K.CellNo[d] - 1 && xf[d] > hi) g = xf[d] - hi;
-          g2 += g * g;
-          inside = inside && xf[d] >= 0.f && xf[d] <= (float)K.CellNo[d] * K.CellSizef[d];
-        }
-        if (!inside) g2 = 0.f;
-        if (g2 <= skip_r2) {
-          int key = P.cell_rank[(q3[0] * K.CellNo[1] + q3[1]) * K.CellNo[2] + q3[2]];
-          cs = P.cell_start[key];
-          cc = P.cell_start[key + 1] - cs;
-        }
-      }
+    float g2_l = 0.f;
+    {
+      const int d = lane / W, q = lane - d * W;
+      const int cd = d == 0 ? c[0] : d == 1 ? c[1] : c[2];
+      const int nd = d == 0 ? K.CellNo[0] : d == 1 ? K.CellNo[1] : K.CellNo[2];
+      const float sz = d == 0 ? K.CellSizef[0] : d == 1 ? K.CellSizef[1] : K.CellSizef[2];
+      const float xd = d == 0 ? pi.x : d == 1 ? pi.y : pi.z;
+      const int qd = cd + q - W / 2;
+      const float lo = (float)qd * sz, hi = lo + sz;
+      float g = 0.f;
+      if (qd > 0 && xd < lo) g = lo - xd;
+      if (qd < nd - 1 && xd > hi) g = xd - hi;
+      // a particle outside the grid (clamped cell) keeps all cells
+      const bool in = lane >= 3 * W || (xd >= 0.f && xd <= (float)nd * sz);
+      g2_l = __all_sync(0xffffffffu, in) ? g * g : 0.f;
+      if (qd < 0 || qd >= nd) g2_l = __int_as_float(0x7fffffff);  // NaN: no radius takes the cell
     }
-    int incl = cc;
+    int2* rng = &s_rng[w][0];
+    int ncell = 0;
+#pragma unroll
+    for (int q0 = 0; q0 < NC; q0 += 32) {
+      const int qc = q0 + lane;
+      const int qx = qc / (W * W), qy = (qc / W) % W, qz = qc % W;
+      // lanes past the stencil read lane 31's value or less and are masked out
+      const float gx = __shfl_sync(0xffffffffu, g2_l, qx), gy = __shfl_sync(0xffffffffu, g2_l, W + qy),
+                  gz = __shfl_sync(0xffffffffu, g2_l, 2 * W + qz);
+      int cs = 0, cc = 0;
+      if (qc < NC && gx + gy + gz <= skip_r2) {
+        int key = P.cell_rank[((c[0] + qx - W / 2) * K.CellNo[1] + c[1] + qy - W / 2) * K.CellNo[2] + c[2] + qz - W / 2];
+        cs = P.cell_start[key];
+        cc = P.cell_start[key + 1] - cs;
+      }
+      const unsigned full = __ballot_sync(0xffffffffu, cc > 0);
+      if (cc > 0) rng[ncell + __popc(full & lt)] = make_int2(cs, cc);
+      ncell += __popc(full);
+    }
+    __syncwarp();
+    // Candidates, flattened over 32 non-empty cells at a time so that all
+    // lanes work on every iteration: a scan of the counts gives the cells'
+    // first flat indices, and the cells that begin within an iteration's 32
+    // candidates set one bit each, so a candidate's cell is the number of
+    // bits up to its own.  Issue binds this kernel: a binary search over the
+    // cells per candidate, in four rounds over all 125 cells, made the superset
+    // build take 841 us at 240,300 particles, this 610 us.
+    for (int r0 = 0; r0 < ncell; r0 += 32) {
+    const int2 rg = r0 + lane < ncell ? rng[r0 + lane] : make_int2(0, 0);
+    int incl = rg.y;
     for (int off = 1; off < 32; off <<= 1) {
       int v = __shfl_up_sync(0xffffffffu, incl, off);
       if (lane >= off) incl += v;
     }
-    int total = __shfl_sync(0xffffffffu, incl, 31);
-    int excl = incl - cc;
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    const int excl = incl - rg.y;
+    int begun = -1;  // the last cell that began before this iteration
     for (int base = 0; base < total; base += 32) {
-      int t = base + lane;
-      // cell of flat candidate t: the last lane q < 27 whose exclusive prefix
-      // is <= t (prefixes are non-decreasing in q: binary search, 5 shuffles)
-      int cell = 0;
-      for (int step = 16; step > 0; step >>= 1) {
-        int q = cell + step;
-        int ex = __shfl_sync(0xffffffffu, excl, q < nq ? q : nq - 1);
-        if (q < nq && ex <= t) cell = q;
-      }
-      int cstart = __shfl_sync(0xffffffffu, cs, cell);
-      int cexcl = __shfl_sync(0xffffffffu, excl, cell);
+      const int t = base + lane;
+      const int at = excl - base;
+      const unsigned starts = __reduce_or_sync(0xffffffffu, rg.y > 0 && at >= 0 && at < 32 ? 1u << at : 0u);
+      const int cell = begun + __popc(starts & (lt | (1u << lane)));
+      begun += __popc(starts);
+      const int slot = __shfl_sync(0xffffffffu, rg.x - excl, cell) + t;
       bool ok = false;
       int j = -1, oj = 0;
       if (t < total) {
-        const int slot = cstart + (t - cexcl);
         const int4 mj = P.cand_m[slot];
         const float4 pj = P.cand_x[slot];
         j = mj.x;
@@ -567,14 +591,14 @@ __global__ void __launch_bounds__(FILL_WARPS * 32) k_nbr_fill(DevPtrs P, DomainC
       }
       unsigned m = __ballot_sync(0xffffffffu, ok);
       if (ok) {
-        int pos = cnt + __popc(m & ((1u << lane) - 1u));
+        int pos = cnt + __popc(m & lt);
         // stored entry: the index, with bit 31 set when j has the larger
         // original index (P2 of the reference's (min, max) pair)
         if (pos < FILL_SLOTS) { rkey[pos] = (unsigned)(oj - oi - 1); ridx[pos] = (int)((unsigned)j | (oj > oi ? NB_UP : 0u)); }
       }
       cnt += __popc(m);
     }
-    }  // stencil rounds
+    }  // cells
     if (cnt > (SUPER ? SUP_W : MAX_NB)) overflow = true;
     if (cnt > FILL_SLOTS) cnt = FILL_SLOTS;
     if (__any_sync(0xffffffffu, link) && lane == 0) atomicOr(&P.st->errors, ERR_SPEC_LINK);
@@ -596,6 +620,7 @@ __global__ void __launch_bounds__(FILL_WARPS * 32) k_nbr_fill(DevPtrs P, DomainC
     idx[r] = e < cnt ? ridx[e] : 0;
   }
   if (nk <= 2) rank_row<2>(rkey, cnt4, key, rank);
+  else if (nk == 3) rank_row<3>(rkey, cnt4, key, rank);
   else rank_row<4>(rkey, cnt4, key, rank);
   __syncwarp();
   for (int r = 0; r < 4; ++r)
@@ -606,7 +631,6 @@ __global__ void __launch_bounds__(FILL_WARPS * 32) k_nbr_fill(DevPtrs P, DomainC
       s_len[row] = cnt;
       P.sup_len[i] = cnt;
       if (overflow) P.st->sup_valid = 0;
-      for (int d = 0; d < 3; ++d) P.xref[(size_t)d * N + i] = P.f[(C_X + d) * N + i];
     } else if (lane == 0) {
       s_len[row] = 0;
     }
@@ -633,7 +657,8 @@ __global__ void __launch_bounds__(FILL_WARPS * 32) k_nbr_fill(DevPtrs P, DomainC
   // Block-wide coalesced ELL write: thread (k, t) stores entry k of particle i0 + t.
   int maxlen = 0;
   for (int t = 0; t < FILL_ROWS; ++t) maxlen = max(maxlen, s_len[t]);
-  if (SUPER) {  // superset rows are row-major (SUP_W entries per particle): a warp reads 32 in one line
+  if (SUPER) {  // reference positions; superset rows are row-major (SUP_W entries per particle): a warp reads 32 in one line
+    if (w < 3 && i0 + lane < K.N) P.xref[w * N + i0 + lane] = P.f[(C_X + w) * N + i0 + lane];
     for (int q = threadIdx.x; q < FILL_ROWS * SUP_W; q += blockDim.x) {
       int t = q / SUP_W, k = q - t * SUP_W;
       if (k < s_len[t]) P.sup[(size_t)(i0 + t) * SUP_W + k] = s_idx[t][k];
