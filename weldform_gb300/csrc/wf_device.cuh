@@ -278,8 +278,9 @@ struct DomainConst {
   // specimens, ERR_SPEC_LINK).  The gathers then take m_j = m_i.
   int m_pair;
   // Uniform-particle layout of the mixed records: every solid particle has the
-  // same h and Cs and the pairs' masses agree (m_pair).  The current records then carry Sigma/rho^2 xz and yz in the last two
-  // fields of RC_VW (instead of h and rho), so the acceleration gather reads four
+  // same h and Cs and the pairs' masses agree (m_pair).  The current records
+  // then carry Sigma/rho^2 xz and yz in the last two fields of RC_VW (instead
+  // of h and rho), so the acceleration gather reads four
   // groups per neighbour instead of five, rho_j = m_i / (m/rho)_j, and every
   // gather uses the kernel constants of the one h below instead of forming
   // 1/h per pair.

@@ -121,14 +121,14 @@ uint64_t spread3(uint64_t v) {
 
 namespace wf {
 // One region of a state copy.  ELL: entry k of particle i at k * N + i, k below
-// len[i]; ROWS: row-major, `width` ints per particle, len[i] of them in use.
-enum CopyKind : int { COPY_BYTES = 0, COPY_ELL, COPY_ROWS };
+// len[i].
+enum CopyKind : int { COPY_BYTES = 0, COPY_ELL };
 struct CopyJob {
   const int* src;
   int* dst;
   const int* len;
   unsigned long long bytes;  // COPY_BYTES
-  int kind, width;
+  int kind;
 };
 constexpr int MAX_COPY_JOBS = 32;
 struct CopyJobs {
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(256) k_copy_state(const __grid_constant__ Copy
       }
       for (; k < n16; k += stride) d[k] = s[k];
       for (size_t w = n16 * 4 + t0; w < c.bytes / 4; w += stride) c.dst[w] = c.src[w];
-    } else if (c.kind == COPY_ELL) {
+    } else {
       for (size_t i = t0; i < N; i += stride) {
         const int len = c.len[i];
         int k = 0;
@@ -168,13 +168,6 @@ __global__ void __launch_bounds__(256) k_copy_state(const __grid_constant__ Copy
           c.dst[(size_t)(k + 2) * N + i] = e; c.dst[(size_t)(k + 3) * N + i] = f;
         }
         for (; k < len; ++k) c.dst[(size_t)k * N + i] = c.src[(size_t)k * N + i];
-      }
-    } else {
-      const int lane = threadIdx.x & 31, w4 = c.width / 4;
-      for (size_t i = t0 / 32; i < N; i += stride / 32) {
-        const int len = c.len[i];
-        for (int k = lane; k < w4 && 4 * k < len; k += 32)
-          reinterpret_cast<int4*>(c.dst)[i * w4 + k] = reinterpret_cast<const int4*>(c.src)[i * w4 + k];
       }
     }
   }
@@ -253,8 +246,8 @@ struct wf_domain {
     return (((gblock_now() * 1024 + pblock_now()) * 16 + glanes_now()) * 2 + (stage_ready && stage ? 1 : 0)) * 2 +
            (fuse_rs ? 1 : 0);
   }
-  // kind, width, len: as in wf::CopyJob (len: region index of the lengths); mixed: the mixed form's records
-  struct Region { void* p; size_t bytes; int kind = wf::COPY_BYTES; int width = 0; int len = -1; bool mixed = false; };
+  // kind, len: as in wf::CopyJob (len: region index of the lengths); mixed: the mixed form's records
+  struct Region { void* p; size_t bytes; int kind = wf::COPY_BYTES; int len = -1; bool mixed = false; };
   std::vector<Region> regions;           // every mutable device region of the state
   std::vector<std::vector<void*>> slots; // checkpoint copies, one vector per slot
   std::vector<char> slot_shadows;        // whether the slot holds valid mixed records
@@ -974,15 +967,15 @@ struct wf_domain {
     regions = {{d_f, sizeof(double) * NF64_PERSIST * n}, {d_i, sizeof(int) * NI32 * n}};
     auto add = [&](Region r) { regions.push_back(r); return (int)regions.size() - 1; };
     add({d_f + (size_t)C_TIR * n, sizeof(double) * 6 * n});
-    add({P.rc, sizeof(float4) * RC_N * n, COPY_BYTES, 0, -1, true});
+    add({P.rc, sizeof(float4) * RC_N * n, COPY_BYTES, -1, true});
     add({P.st, sizeof(StepState)});
     add({P.inv, sizeof(int) * n});
     add({P.row_split, sizeof(int) * n});
     const int row_len = add({P.row_len, sizeof(int) * n});
-    add({P.nbr, sizeof(int) * MAX_NB * n, COPY_ELL, MAX_NB, row_len});
+    add({P.nbr, sizeof(int) * MAX_NB * n, COPY_ELL, row_len});
     const int cp_len = add({P.cp_len, sizeof(int) * n});
     if (contact) {
-      add({P.cp, sizeof(int) * MAX_CP * n, COPY_ELL, MAX_CP, cp_len});
+      add({P.cp, sizeof(int) * MAX_CP * n, COPY_ELL, cp_len});
       add({P.cp_list, sizeof(int) * n});
     }
     add({P.node, sizeof(double) * hnode.size()});
@@ -998,7 +991,7 @@ struct wf_domain {
     if (K.nspec > 0) add({P.sp, sizeof(SpecState) * K.nspec});
     if (K.skin_on) {
       const int sup_len = add({P.sup_len, sizeof(int) * n});
-      add({P.sup, sizeof(int) * SUP_W * n, COPY_ROWS, SUP_W, sup_len});
+      add({P.sup, sizeof(int) * SUP_W * n, COPY_ELL, sup_len});
       add({P.xref, sizeof(double) * 3 * n});
     }
     launch_prologue(P, K, stream);
@@ -1181,7 +1174,6 @@ struct wf_domain {
       c.len = r.len < 0 ? nullptr : (const int*)(save ? regions[r.len].p : sl[r.len]);
       c.bytes = r.bytes;
       c.kind = r.kind;
-      c.width = r.width;
     }
     long long b = ((long long)hp.N + 255) / 256 * 4;
     k_copy_state<<<(int)std::min<long long>(std::max<long long>(b, 1), 152 * 8), 256, 0, stream>>>(J);

@@ -387,16 +387,21 @@ __device__ __forceinline__ bool radius_exact(const DevPtrs& P, size_t N, int i, 
   return __ddiv_rn(rij, hh) <= Cellfac;
 }
 
-// Radius test: FP32 prefilter, exact FP64 decision inside the margin.
-__device__ __forceinline__ bool radius_ok(const DevPtrs& P, const DomainConst& K, size_t N, int i, int j, float xi,
-                                          float yi, float zi, float hi, float4 pj) {
-  float dx = xi - pj.x, dy = yi - pj.y, dz = zi - pj.z;
+// FP32 prefilter of the radius test (positions in x, y, z, h in w): 1 inside,
+// -1 outside, 0 within the margin that only the exact test decides.
+__device__ __forceinline__ int radius_near(const DomainConst& K, float4 pi, float4 pj) {
+  float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
   float d2 = dx * dx + dy * dy + dz * dz;
-  float R = K.half_cellfac_f * (hi + pj.w);
+  float R = K.half_cellfac_f * (pi.w + pj.w);
   float R2 = R * R;
-  if (d2 < R2 * (1.0f - K.pre_eps)) return true;
-  if (d2 > R2 * (1.0f + K.pre_eps)) return false;
-  return radius_exact(P, N, i, j, K.Cellfac);
+  return d2 < R2 * (1.0f - K.pre_eps) ? 1 : d2 > R2 * (1.0f + K.pre_eps) ? -1 : 0;
+}
+
+// Radius test: FP32 prefilter, exact FP64 decision inside the margin.
+__device__ __forceinline__ bool radius_ok(const DevPtrs& P, const DomainConst& K, size_t N, int i, int j, float4 pi,
+                                          float4 pj) {
+  const int near = radius_near(K, pi, pj);
+  return near > 0 || (near == 0 && radius_exact(P, N, i, j, K.Cellfac));
 }
 
 // SM neighbour rows in canonical order: one warp per particle, 32 consecutive
@@ -584,7 +589,7 @@ __global__ void __launch_bounds__(FILL_WARPS * 32) k_nbr_fill(DevPtrs P, DomainC
             float Rs = K.half_cellfac_f * (pi.w + pj.w) + (float)K.skin;
             ok = dx * dx + dy * dy + dz * dz <= Rs * Rs * (1.0f + 4.0f * K.pre_eps);
           } else {
-            ok = radius_ok(P, K, N, i, j, pi.x, pi.y, pi.z, pi.w, pj);
+            ok = radius_ok(P, K, N, i, j, pi, pj);
             if (ok && K.nspec > 0 && mj.w != spec_i) link = true;
           }
         }
@@ -657,17 +662,11 @@ __global__ void __launch_bounds__(FILL_WARPS * 32) k_nbr_fill(DevPtrs P, DomainC
   // Block-wide coalesced ELL write: thread (k, t) stores entry k of particle i0 + t.
   int maxlen = 0;
   for (int t = 0; t < FILL_ROWS; ++t) maxlen = max(maxlen, s_len[t]);
-  if (SUPER) {  // reference positions; superset rows are row-major (SUP_W entries per particle): a warp reads 32 in one line
-    if (w < 3 && i0 + lane < K.N) P.xref[w * N + i0 + lane] = P.f[(C_X + w) * N + i0 + lane];
-    for (int q = threadIdx.x; q < FILL_ROWS * SUP_W; q += blockDim.x) {
-      int t = q / SUP_W, k = q - t * SUP_W;
-      if (k < s_len[t]) P.sup[(size_t)(i0 + t) * SUP_W + k] = s_idx[t][k];
-    }
-  } else {
-    for (int q = threadIdx.x; q < maxlen * FILL_ROWS; q += blockDim.x) {
-      int k = q / FILL_ROWS, t = q - k * FILL_ROWS;
-      if (k < s_len[t]) P.nbr[(size_t)k * N + i0 + t] = s_idx[t][k];
-    }
+  int* ell = SUPER ? P.sup : P.nbr;
+  if (SUPER && w < 3 && i0 + lane < K.N) P.xref[w * N + i0 + lane] = P.f[(C_X + w) * N + i0 + lane];
+  for (int q = threadIdx.x; q < maxlen * FILL_ROWS; q += blockDim.x) {
+    int k = q / FILL_ROWS, t = q - k * FILL_ROWS;
+    if (k < s_len[t]) ell[(size_t)k * N + i0 + t] = s_idx[t][k];
   }
   __syncthreads();  // the shared buffers are reused by the next group
   }
@@ -737,98 +736,123 @@ __device__ __forceinline__ bool cells_adjacent(long long a, long long b) {
 // COVER: every cell is wider than the largest pair radius (DomainConst::
 // cells_cover), so a pair that passes the radius rule is in adjacent cells
 // and the cell test is left out (a non-finite position fails the radius rule).
-// One warp per particle, 32 superset entries per round (one coalesced line of
-// the row-major superset); the kept entries are compacted by ballot in order
-// into shared memory, and the block writes its FILL_ROWS rows to the ELL
-// array one coalesced line per entry index.  In a batched domain the rows of
-// specimens that do not search stay as they are (untouched, or put back by
-// k_nbr_fill after a reordering).
-template <bool COVER>
-__global__ void __launch_bounds__(FILL_WARPS * 32, 4) k_nbr_filter(DevPtrs P, DomainConst K) {
+// L lanes per particle: each turn they test the next 4 L superset entries,
+// entry and position loads issued before the first test and the next turn's
+// entries before that, and append the kept ones to the row in order.  The
+// superset is an ELL array like the rows, so a warp's lanes read the same
+// entries of consecutive particles, whose positions share cache lines in the
+// brick order, and their appends fall in the same lines of the rows.  Issue
+// and load latency bind it.  A warp per particle over a row-major superset,
+// compacted by ballot into shared memory, spent ~450 warp instructions per
+// row, most of them on the row rather than its entries: 580 us at 982,072
+// particles, this 232 us (three and five blocks per SM: 253 and 269 us).
+// In a batched domain the rows of specimens that do not search stay as they
+// are (untouched, or put back by k_nbr_fill after a reordering).
+constexpr int FILTER_T = 256;
+template <bool COVER, int L>
+__global__ void __launch_bounds__(FILTER_T, 4) k_nbr_filter(DevPtrs P, DomainConst K) {
   if (!searching(P) || !K.skin_on || !P.st->sup_valid) return;
-  __shared__ int s_idx[FILL_ROWS][MAX_NB];
-  __shared__ int s_len[FILL_ROWS];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  __shared__ unsigned s_pairs;
+  if (threadIdx.x == 0) s_pairs = 0;
+  __syncthreads();
   const size_t N = K.N;
+  const int lane = threadIdx.x & 31, sub = lane & (L - 1);
+  const unsigned grp = ((1u << L) - 1u) << (lane - sub);  // the row's lanes
+  const unsigned below = grp & ((1u << lane) - 1u);
   const float4* xs = reinterpret_cast<const float4*>(P.xs);
-  const int ngroups = (K.N + FILL_ROWS - 1) / FILL_ROWS;
-  unsigned long long pairs = 0;  // this warp's entries (lane 0), one atomic at the end
-  for (int grp = blockIdx.x; grp < ngroups; grp += gridDim.x) {
-    const int i0 = grp * FILL_ROWS;
-    for (int rr = 0; rr < FILL_PER_WARP; ++rr) {
-      const int row = w * FILL_PER_WARP + rr;
-      const int i = i0 + row;
-      int cnt = 0;
-      if (K.nspec > 0 && i < K.N && !P.sp[P.i[I_SPEC * N + i]].do_search) {
-        if (lane == 0) { s_len[row] = 0; pairs += (unsigned long long)P.row_len[i]; }
-        continue;
+  unsigned pairs = 0;
+  const int rows = FILTER_T / L;
+  const int nblocks = (K.N + rows - 1) / rows;
+  for (int b = blockIdx.x; b < nblocks; b += gridDim.x) {
+    const int i = b * rows + threadIdx.x / L;
+    bool mine = i < K.N;
+    if (mine && K.nspec > 0 && !P.sp[P.i[I_SPEC * N + i]].do_search) {
+      mine = false;
+      if (sub == 0) pairs += (unsigned)P.row_len[i];
+    }
+    const int spec_i = K.nspec > 0 && mine ? P.i[I_SPEC * N + i] : 0;
+    const long long ci = mine ? P.cellc[i] : -1;
+    int len = 0;
+    float4 pi = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (mine && P.i[I_KIND * N + i] == 0 && ci >= 0) {
+      pi = xs[i];
+      len = P.sup_len[i];
+    }
+    // lanes of a warp take the same number of turns (ballots below)
+    const int most = L == 1 ? len : __reduce_max_sync(0xffffffffu, len);
+    constexpr int U = 4;
+    const int* sup = P.sup + i;
+    int e[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) e[u] = u * L + sub < len ? sup[(size_t)(u * L + sub) * N] : 0;
+    int cnt = 0, split = 0;
+    bool link = false;
+    for (int k0 = 0; k0 < most; k0 += U * L) {
+      float4 pj[U];
+      long long cj[U];
+      int en[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (k0 + u * L + sub < len) {
+          pj[u] = xs[nb_index(e[u])];
+          if (!COVER) cj[u] = P.cellc[nb_index(e[u])];
+        }
       }
-      const int spec_i = K.nspec > 0 && i < K.N ? P.i[I_SPEC * N + i] : 0;
-      bool link = false;
-      const long long ci = i < K.N ? P.cellc[i] : -1;
-      if (i < K.N && P.i[I_KIND * N + i] == 0 && ci >= 0) {
-        const float4 pi = xs[i];
-        const int len = P.sup_len[i];
-        const int* sr = P.sup + (size_t)i * SUP_W;
-        // All of the row's loads are issued before any is used: the lane's up
-        // to four entries (k = lane + 32 r), then their positions, so a row
-        // costs two memory latencies rather than two per 32 entries.
-        constexpr int R = SUP_W / 32;
-        int e[R];
-        float4 pj[R];
-        long long cj[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) e[r] = lane + 32 * r < len ? sr[lane + 32 * r] : 0;
+      for (int u = 0; u < U; ++u) {
+        const int k = k0 + (U + u) * L + sub;
+        en[u] = k < len ? sup[(size_t)k * N] : 0;
+      }
+      // the FP32 prefilter's decisions, and the pairs inside its margin
+      unsigned in = 0, edge = 0;
 #pragma unroll
-        for (int r = 0; r < R; ++r)
-          if (lane + 32 * r < len) {
-            pj[r] = xs[nb_index(e[r])];
-            if (!COVER) cj[r] = P.cellc[nb_index(e[r])];
-          }
+      for (int u = 0; u < U; ++u) {
+        if (k0 + u * L + sub < len && (COVER || (cj[u] >= 0 && cells_adjacent(ci, cj[u])))) {
+          const int near = radius_near(K, pi, pj[u]);
+          in |= (near > 0 ? 1u : 0u) << u;
+          edge |= (near == 0 ? 1u : 0u) << u;
+        }
+      }
+#pragma unroll 1
+      for (int u = 0; edge; ++u, edge >>= 1)
+        if ((edge & 1u) && radius_exact(P, N, i, nb_index(u == 0 ? e[0] : u == 1 ? e[1] : u == 2 ? e[2] : e[3]), K.Cellfac))
+          in |= 1u << u;
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          if (32 * r >= len) break;  // warp-uniform
-          bool ok = false;
-          if (lane + 32 * r < len) {
-            ok = COVER || (cj[r] >= 0 && cells_adjacent(ci, cj[r]));
-            if (ok) ok = radius_ok(P, K, N, i, nb_index(e[r]), pi.x, pi.y, pi.z, pi.w, pj[r]);
-            if (ok && K.nspec > 0 && P.i[I_SPEC * N + nb_index(e[r])] != spec_i) link = true;
-          }
+      for (int u = 0; u < U; ++u) {
+        const bool ok = in >> u & 1u;
+        if (ok && K.nspec > 0 && P.i[I_SPEC * N + nb_index(e[u])] != spec_i) link = true;
+        int pos = cnt;
+        if (L == 1) {
+          cnt += ok ? 1 : 0;
+        } else {
           const unsigned m = __ballot_sync(0xffffffffu, ok);
-          if (ok) {
-            const int pos = cnt + __popc(m & ((1u << lane) - 1u));
-            if (pos < MAX_NB) s_idx[row][pos] = e[r];
-          }
-          cnt += __popc(m);
+          pos += __popc(m & below);
+          cnt += __popc(m & grp);
         }
-      }
-      if (cnt > MAX_NB && lane == 0) atomicOr(&P.st->errors, ERR_NBR_OVERFLOW);
-      if (__any_sync(0xffffffffu, link) && lane == 0) atomicOr(&P.st->errors, ERR_SPEC_LINK);
-      if (cnt > MAX_NB) cnt = MAX_NB;
-      __syncwarp();
-      int split = 0;
-      for (int e = lane; e < cnt; e += 32) split += s_idx[row][e] < 0 ? 1 : 0;
-      for (int off = 16; off > 0; off >>= 1) split += __shfl_down_sync(0xffffffffu, split, off);
-      if (lane == 0) {
-        s_len[row] = i < K.N ? cnt : 0;
-        if (i < K.N) {
-          P.row_len[i] = cnt;
-          P.row_split[i] = split;
-          P.i[I_NB * N + i] = cnt;
-          pairs += (unsigned long long)cnt;
+        if (ok && pos < MAX_NB) {
+          P.nbr[(size_t)pos * N + i] = e[u];
+          split += e[u] < 0 ? 1 : 0;
         }
+        e[u] = en[u];
       }
     }
-    __syncthreads();
-    int maxlen = 0;
-    for (int t = 0; t < FILL_ROWS; ++t) maxlen = max(maxlen, s_len[t]);
-    for (int q = threadIdx.x; q < maxlen * FILL_ROWS; q += blockDim.x) {
-      int k = q / FILL_ROWS, t = q - k * FILL_ROWS;
-      if (k < s_len[t]) P.nbr[(size_t)k * N + i0 + t] = s_idx[t][k];
+    if (link) atomicOr(&P.st->errors, ERR_SPEC_LINK);
+    if (cnt > MAX_NB) {
+      cnt = MAX_NB;
+      if (sub == 0) atomicOr(&P.st->errors, ERR_NBR_OVERFLOW);
     }
-    __syncthreads();  // the shared rows are reused by the next group
+    for (int off = 1; off < L; off <<= 1) split += __shfl_xor_sync(0xffffffffu, split, off);
+    if (mine && sub == 0) {
+      P.row_len[i] = cnt;
+      P.row_split[i] = split;
+      P.i[I_NB * N + i] = cnt;
+      pairs += (unsigned)cnt;
+    }
   }
-  if (lane == 0 && pairs) atomicAdd(&P.st->pair_count, pairs);
+  pairs = __reduce_add_sync(0xffffffffu, pairs);
+  if (lane == 0 && pairs) atomicAdd(&s_pairs, pairs);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_pairs) atomicAdd(&P.st->pair_count, (unsigned long long)s_pairs);
 }
 
 // CalculateSurface (Domain.cpp:1415-1491): n_i = sum_j m_j (x_i - x_j) in row
@@ -986,9 +1010,14 @@ void launch_neighbour_search(const DevPtrs& P, const DomainConst& K, double* fsc
   }
   mark(s, "k_nbr_fill");
   if (K.skin_on) {
-    int groups = nblk(K.N, FILL_ROWS), cap = 152 * 4;
-    if (K.cells_cover) k_nbr_filter<true><<<groups < cap ? groups : cap, FILL_WARPS * 32, 0, s>>>(P, K);
-    else k_nbr_filter<false><<<groups < cap ? groups : cap, FILL_WARPS * 32, 0, s>>>(P, K);
+    // Lanes per row: a filtered search of 8,004 / 30,600 / 63,612 / 120,416 /
+    // 240,300 particles takes 85 / 87 / 93 / 111 / 145 us with one, 75 / 82 /
+    // 92 / 110 / 153 with four (eight: 74 / 84 / 95 / 118 / 172).
+    const int L = K.N < 100000 ? 4 : 1;
+    const int blocks = nblk((long long)K.N * L, FILTER_T), cap = 152 * 16;
+    const auto k = K.cells_cover ? (L == 4 ? k_nbr_filter<true, 4> : k_nbr_filter<true, 1>)
+                                 : (L == 4 ? k_nbr_filter<false, 4> : k_nbr_filter<false, 1>);
+    k<<<blocks < cap ? blocks : cap, FILTER_T, 0, s>>>(P, K);
     mark(s, "k_nbr_filter");
   }
   if (P.halo) launch_halo_build(P, K, s);
