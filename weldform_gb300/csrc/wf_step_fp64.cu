@@ -5,27 +5,27 @@
 //   k_schedule          neighbour-search decision (SolverKickDrift.cpp:153-186)
 //   [search pipeline]   gated on the decision (wf_nbsearch.cu)
 //   k_accel             CalcAccel + AccelReduction (InteractionAlt.cpp:12-260)
-//   k_bc                GeneralAfter (WeldForm.cpp:51-120)
-//   k_contact_kick      CalcContactForcesWang (Contact_Wang.cpp:15-348) + v += a dt/2
-//   k_bc
+//   k_bc                GeneralAfter (WeldForm.cpp:51-120), where a rigid mesh or the
+//                       leapfrog order needs it (the kick applies it otherwise)
+//   k_contact_force     CalcContactForcesWang (Contact_Wang.cpp:15-348), one rigid mesh
+//   k_contact_kick      v += a dt/2, and the contact pass where k_contact_force did not run
 //   k_density_drift     CalcDensInc + DensReduction (InteractionAlt.cpp:483-640) with the
 //                       acceleration pass's GradKernel per row entry (same x(n), h),
 //                       rho += dt drho, x += v dt, v += a dt/2 (SolverKickDrift.cpp:236-265);
 //                       next-step p/rho^2 and T for the rate gather
-//   k_bc                (on the next-step velocity buffer)
 //   k_rate_stress       CalcRateTensors + RateTensorsReduction (InteractionAlt.cpp:263-479),
 //                       CalcStressStrain (Particle.cpp:960-1067), CalcPlasticWorkHeat
 //                       (ThermalStuct.cpp:14-39), T += dt dTdt (Thermal.cpp:727-734),
 //                       and in the same neighbour loop CalcTempInc (Thermal.cpp:53-219),
 //                       CalcKinEnergyEqn (Domain.cpp:1752-1808); then CalcThermalExpStrainRate
 //                       and CalcIntEnergyEqn (Domain.cpp:1810-1829)
-//   k_finalize          deterministic reduction of the per-block partial sums
-//   k_mesh_*            TriMesh::Update (Mesh.cpp:273-293), UpdateContactParticles
-//                       (Contact.cpp:41-55)
-//   k_step_end          Time += dt and the neighbour-clear schedule (:299-324)
+//   k_finalize          deterministic reduction of the per-block partial sums, the
+//                       nodes of TriMesh::Update (Mesh.cpp:273-293), then Time += dt and
+//                       the neighbour-clear schedule (:299-324)
+//   k_mesh_elems        the rest of TriMesh::Update, UpdateContactParticles (Contact.cpp:41-55)
 //
-// Each gather kernel runs one thread per particle over its neighbour row in
-// canonical order; a pair term is evaluated from the particle's own side
+// Each gather kernel runs one thread per particle (two or four on small
+// domains) over its neighbour row in canonical order; a pair term is evaluated from the particle's own side
 // (x_i - x_j), which equals the reference's (min, max)-ordered pair value
 // with the reduction's sign applied.
 #include <type_traits>

@@ -23,7 +23,8 @@
 // rate tensors fused with the kinetic-energy and conduction sums, which use
 // the same positions, velocities and the pressure of the updated density.
 // Each walks a particle's row with one thread, or on small domains with
-// 2-8 lanes whose partial sums are combined by warp shuffles.
+// 2-8 lanes whose partial sums are combined by warp shuffles.  With one thread
+// the rate gather also runs the stress update (k_rate_stress_mx).
 #include <type_traits>
 
 #include "wf_step_common.cuh"
@@ -444,8 +445,8 @@ __global__ void __launch_bounds__(512) k_accel_mx_lanes(DevPtrs P, DomainConst K
 }
 
 // Staged acceleration gather (uniform viscosity constants, no tensile
-// instability, no gradient correction): block b copies its halo's five groups
-// into shared memory once, then two threads share each particle's row, which
+// instability, no gradient correction): block b copies its halo's groups (four
+// in the uniform-particle layout, five else) into shared memory once, then two threads share each particle's row, which
 // doubles the warps per SM that the shared-memory footprint allows.  The
 // block's first STAGE_B threads sum the even row entries of its particles,
 // the other STAGE_B the odd ones, so a warp's lanes still read the same entry
