@@ -37,31 +37,42 @@ static_assert(ADJ_BLOCK == BLOCK, "the finish kernel's partials are sized by ADJ
 // with C = 1 / (pi hh^4):
 //   q < 1:      GK = C/hh (-3 + 9/4 q),     dGK/dr = C/hh^2 9/4
 //   1 <= q < 2: GK = -3/4 C (2 - q)^2 / r,  dGK/dr = 3/4 C (4 - q^2) / r^2
-// with r and 1/r from one reciprocal square root per pair, plus 1/hh when
-// the pair's smoothing lengths differ (inv_hi = 1/h_i is the caller's).  The
-// values equal the forward's to rounding.
+// with r and 1/r from one reciprocal square root per pair and the constants of
+// the own smoothing length formed once; a pair of different lengths forms its
+// own (behind a vote, so that a warp without one branches over the division
+// instead of running it predicated off).  The values equal the forward's to
+// rounding.
 struct GeoD {
   double x0, x1, x2, r, GK, dGr;  // dGr = (dGK/dr) / r
 };
-__device__ __forceinline__ GeoD geo_d(const double xi[3], double hi, double inv_hi, double xj0, double xj1, double xj2,
-                                      double hj) {
+struct GeoH {
+  double h, inv_h, near0, near1, far;  // GK = near0 + near1 r, far (2 - q)^2 / r
+};
+__device__ __forceinline__ GeoH geo_h(double h, double inv_h) {
+  const double ih2 = inv_h * inv_h, C = ih2 * ih2 * (1.0 / WF_PI);
+  return {h, inv_h, -3.0 * (C * inv_h), 2.25 * (C * ih2), -0.75 * C};
+}
+__device__ __forceinline__ GeoD geo_d(const double xi[3], const GeoH& own, double xj0, double xj1, double xj2, double hj) {
   GeoD g;
   g.x0 = xi[0] - xj0; g.x1 = xi[1] - xj1; g.x2 = xi[2] - xj2;
-  double r2 = g.x0 * g.x0 + g.x1 * g.x1 + g.x2 * g.x2;
-  double rinv = r2 > 0.0 ? rsqrt(r2) : 0.0;
+  const double r2 = g.x0 * g.x0 + g.x1 * g.x1 + g.x2 * g.x2;
+  const double rinv = r2 > 0.0 ? rsqrt(r2) : 0.0;
   g.r = r2 * rinv;
-  double inv_h = hj == hi ? inv_hi : 2.0 / (hi + hj);
-  double q = g.r * inv_h;
-  double ih2 = inv_h * inv_h;
-  double C = ih2 * ih2 * (1.0 / WF_PI);
+  GeoH H = own;
+  if (__any_sync(__activemask(), hj != own.h)) {
+    if (hj != own.h) H = geo_h(0.5 * (own.h + hj), 2.0 / (own.h + hj));
+  }
+  const double q = g.r * H.inv_h;
   double dG = 0.0;
-  if (q == 0.0) g.GK = C * inv_h * -3.0;
-  else if (q < 1.0) { g.GK = C * inv_h * (-3.0 + 2.25 * q); dG = C * ih2 * 2.25; }
-  else if (q < 2.0) {
-    double t = 2.0 - q;
-    g.GK = C * rinv * (-0.75 * t * t);
-    dG = C * 0.75 * (4.0 - q * q) * (rinv * rinv);
-  } else g.GK = 0.0;
+  g.GK = 0.0;
+  if (q < 1.0) {  // r = 0 leaves dGr = 0 through 1/r = 0
+    g.GK = H.near0 + H.near1 * g.r;
+    dG = H.near1;
+  } else if (q < 2.0) {
+    const double fr = H.far * rinv, t = 2.0 - q;
+    g.GK = fr * (t * t);
+    dG = fr * rinv * (q * q - 4.0);
+  }
   g.dGr = dG * rinv;
   return g;
 }
@@ -101,9 +112,10 @@ __device__ __forceinline__ bool bc_value(const DomainTables* T, int id, double t
 // which finish a particle each in full warps (R1's and R3's epilogues are as
 // long as a row).  At 18,258 particles one thread per particle is four warps
 // per SM, too few to cover the FP64 latency.
-// Reverse sweep of 20 steps, ms with 1, 2 and 4 lanes: 25.2, 19.0, 18.4 at 5,682
-// particles; 25.6, 19.4, 18.6 at 9,156; 30.0, 28.7, 29.4 at 18,258; from there
-// the FP64 pipe is full (45.4, 47.0, 47.0 at 32,912).
+// Reverse sweep of 20 steps, ms with 1, 2 and 4 lanes, when a pair took ~1.3
+// times today's FP64 instructions: 25.2, 19.0, 18.4 at 5,682 particles; 25.6,
+// 19.4, 18.6 at 9,156; 30.0, 28.7, 29.4 at 18,258; from there the FP64 pipe is
+// full (45.4, 47.0, 47.0 at 32,912).
 static int adj_lanes(long long n) { return n < 14000 ? 4 : (n < 24000 ? 2 : 1); }
 constexpr int ADJ_LANE_BLOCK = 64;  // particles per block with more than one lane
 template <int L, int NS>
@@ -134,12 +146,12 @@ __device__ __forceinline__ void adj_conduction(const AdjPtrs& A, const DomainCon
   const double lci = TMP(J_LC, i), inv_rhoN = 1.0 / FE(C_RHO, i);
   double xi[3] = {FE(C_X, i), FE(C_X + 1, i), FE(C_X + 2, i)};
   double hi = col(S, C_H, N, i), ki = col(S, C_KT, N, i), Ti = FE(C_T, i), wi = FE(C_MRHO, i);
-  double inv_hi = 1.0 / hi;
+  const GeoH Hi = geo_h(hi, 1.0 / hi);
   int len = S.row_len[i];
   for (int k = k0; k < len; k += dk) {
     int e = S.nbr[(size_t)k * N + i];
     int j = nb_index(e);
-    GeoD g = geo_d(xi, hi, inv_hi, FE(C_X, j), FE(C_X + 1, j), FE(C_X + 2, j), col(S, C_H, N, j));
+    GeoD g = geo_d(xi, Hi, FE(C_X, j), FE(C_X + 1, j), FE(C_X + 2, j), col(S, C_H, N, j));
     A.gk_end[(size_t)k * N + i] = g.GK;  // R2 reads the same end-state geometry
     A.dg_end[(size_t)k * N + i] = g.dGr;
     double lcj = TMP(J_LC, j);
@@ -147,7 +159,10 @@ __device__ __forceinline__ void adj_conduction(const AdjPtrs& A, const DomainCon
     bool up = nb_up(e);  // j has the larger original index: P2 = j
     double w = up ? FE(C_MRHO, j) : wi;  // m_P2 / rho_P2 at both ends (Thermal.cpp:127-131)
     double kj = col(S, C_KT, N, j);
-    double kk = 4. * (ki * kj) / (ki + kj);
+    // equal conductivities need no division (a vote, so that a warp whose pairs
+    // all agree branches over it: predicated off it would keep its pipe slots)
+    double kk = ki + ki;
+    if (__any_sync(__activemask(), kj != ki)) kk = kj != ki ? 4. * (ki * kj) / (ki + kj) : kk;
     double dT = Ti - FE(C_T, j);
     ltn += d * w * kk * g.GK;
     double cx = d * w * kk * dT * g.dGr;
@@ -167,8 +182,9 @@ __global__ void __launch_bounds__(256) k_adj_thermal_stress(AdjPtrs A, DomainCon
   if (!adj_fold<L>(sums, sh, K.N, i)) return;
   double dt = K.dt;
   if (icol(S, I_KIND, N, i) != 0) {
-    for (int c = 0; c < 6; ++c) { LOUT(A_TAU + c) = 0.0; LOUT(A_INC + c) = 0.0; TMP(J_SR + c, i) = 0.0; }
-    for (int c = 0; c < 3; ++c) { TMP(J_RR + c, i) = 0.0; TMP(J_XN + c, i) = 0.0; TMP(J_VN + c, i) = 0.0; }
+    for (int c = 0; c < 6; ++c) { LOUT(A_TAU + c) = 0.0; LOUT(A_INC + c) = 0.0; }
+    for (int c = 0; c < 9; ++c) TMP(J_M + c, i) = 0.0;
+    for (int c = 0; c < 3; ++c) { TMP(J_XN + c, i) = 0.0; TMP(J_VN + c, i) = 0.0; }
     LOUT(A_PLS) = 0.0; LOUT(A_SY) = 0.0; LOUT(A_T) = 0.0; LOUT(A_DTDT) = 0.0; TMP(J_RHON, i) = 0.0;
     return;
   }
@@ -338,8 +354,12 @@ __global__ void __launch_bounds__(256) k_adj_thermal_stress(AdjPtrs A, DomainCon
   ltau0[3] += lS[0][1] + lS[1][0]; ltau0[4] += lS[0][2] + lS[2][0]; ltau0[5] += lS[1][2] + lS[2][1];
   lrr[0] = lW[0][1] - lW[1][0]; lrr[1] = lW[0][2] - lW[2][0]; lrr[2] = lW[1][2] - lW[2][1];
 
-  for (int c = 0; c < 6; ++c) { LOUT(A_TAU + c) = ltau0[c]; LOUT(A_INC + c) = linc0[c]; TMP(J_SR + c, i) = lsr[c]; }
-  for (int c = 0; c < 3; ++c) { TMP(J_RR + c, i) = lrr[c]; TMP(J_XN + c, i) = lxn[c]; TMP(J_VN + c, i) = LIN(A_V + c, i); }
+  for (int c = 0; c < 6; ++c) { LOUT(A_TAU + c) = ltau0[c]; LOUT(A_INC + c) = linc0[c]; }
+  // SR and RR adjoints as the matrix of the pair's bilinear form (adj_rates)
+  TMP(J_M + 0, i) = 2.0 * lsr[0]; TMP(J_M + 1, i) = lsr[3] + lrr[0]; TMP(J_M + 2, i) = lsr[4] + lrr[1];
+  TMP(J_M + 3, i) = lsr[3] - lrr[0]; TMP(J_M + 4, i) = 2.0 * lsr[1]; TMP(J_M + 5, i) = lsr[5] + lrr[2];
+  TMP(J_M + 6, i) = lsr[4] - lrr[1]; TMP(J_M + 7, i) = lsr[5] - lrr[2]; TMP(J_M + 8, i) = 2.0 * lsr[2];
+  for (int c = 0; c < 3; ++c) { TMP(J_XN + c, i) = lxn[c]; TMP(J_VN + c, i) = LIN(A_V + c, i); }
   LOUT(A_PLS) = lpls0;
   LOUT(A_SY) = lsy0;
   LOUT(A_T) = ltn + lT0;
@@ -352,17 +372,25 @@ __global__ void __launch_bounds__(256) k_adj_thermal_stress(AdjPtrs A, DomainCon
 
 // ---------------------------------------------------------------- R2: rates + second kick + drift
 // Rate adjoint sums: d/dx' (3), d/dv' (3), and sum L . B for d/drho'.
+// A particle's nine rate adjoints enter a pair as b.(M x) with one 3x3 matrix
+// M (b the velocity and x the position difference), so the pair's derivatives
+// are M x and M^T b of either end, and the own end's are taken out of the sum:
+// M_i times the sums of f w_j x and f w_j b.  The FP64 pipe binds this kernel;
+// the nine components summed one by one took ~110 FP64 instructions per pair
+// instead of ~60: reverse sweep of 20 steps 45.4 -> 39.1 ms at 32,912
+// particles, with the kernel constants of one length (geo_d) and one division
+// for two in the acceleration's viscosity.
 __device__ __forceinline__ void adj_rates(const AdjPtrs& A, const DomainConst& K, int i, int k0, int dk, double (&out)[7]) {
   const DevPtrs& S = A.S;
   size_t N = K.N;
   double xi[3] = {FE(C_X, i), FE(C_X + 1, i), FE(C_X + 2, i)};
   double vi[3] = {FE(C_V, i), FE(C_V + 1, i), FE(C_V + 2, i)};
   double hi = col(S, C_H, N, i), wi = FE(C_MRHO, i);
-  double inv_hi = 1.0 / hi;
-  double li[9];
-  for (int c = 0; c < 6; ++c) li[c] = TMP(J_SR + c, i);
-  for (int c = 0; c < 3; ++c) li[6 + c] = TMP(J_RR + c, i);
-  double lx[3] = {0, 0, 0}, lv[3] = {0, 0, 0};
+  const GeoH Hi = geo_h(hi, 1.0 / hi);
+  double Mi[9];
+  for (int c = 0; c < 9; ++c) Mi[c] = TMP(J_M + c, i);
+  // sums of f w_j x, f M_j x, f w_j b, f M_j^T b and the GradKernel's derivative
+  double fx[3] = {0, 0, 0}, fp[3] = {0, 0, 0}, fb[3] = {0, 0, 0}, fq[3] = {0, 0, 0}, gx[3] = {0, 0, 0};
   double sumLT = 0.0;
   int len = S.row_len[i];
   for (int k = k0; k < len; k += dk) {
@@ -373,32 +401,34 @@ __device__ __forceinline__ void adj_rates(const AdjPtrs& A, const DomainConst& K
       g.GK = A.gk_end[(size_t)k * N + i];
       g.dGr = A.dg_end[(size_t)k * N + i];
     } else {
-      g = geo_d(xi, hi, inv_hi, FE(C_X, j), FE(C_X + 1, j), FE(C_X + 2, j), col(S, C_H, N, j));
+      g = geo_d(xi, Hi, FE(C_X, j), FE(C_X + 1, j), FE(C_X + 2, j), col(S, C_H, N, j));
     }
     double b0 = vi[0] - FE(C_V, j), b1 = vi[1] - FE(C_V + 1, j), b2 = vi[2] - FE(C_V + 2, j);
     double wj = FE(C_MRHO, j);
-    double lj[9], L[9];
-    for (int c = 0; c < 6; ++c) lj[c] = TMP(J_SR + c, j);
-    for (int c = 0; c < 3; ++c) lj[6 + c] = TMP(J_RR + c, j);
-    for (int c = 0; c < 9; ++c) L[c] = wj * li[c] + wi * lj[c];
-    double x0 = g.x0, x1 = g.x1, x2 = g.x2;
-    double B[9] = {2.0 * b0 * x0, 2.0 * b1 * x1, 2.0 * b2 * x2, b0 * x1 + b1 * x0, b0 * x2 + b2 * x0,
-                   b1 * x2 + b2 * x1, b0 * x1 - b1 * x0, b0 * x2 - b2 * x0, b1 * x2 - b2 * x1};
-    double Q = 0.0, Qj = 0.0;
-    for (int c = 0; c < 9; ++c) { Q += L[c] * B[c]; Qj += lj[c] * B[c]; }
-    double f = -0.5 * g.GK;
+    double M[9];
+    for (int c = 0; c < 9; ++c) M[c] = TMP(J_M + c, j);
+    const double x[3] = {g.x0, g.x1, g.x2}, b[3] = {b0, b1, b2};
+    double Qi = 0.0, Qj = 0.0, p[3], q[3];
+    for (int d = 0; d < 3; ++d) {
+      p[d] = M[3 * d] * x[0] + M[3 * d + 1] * x[1] + M[3 * d + 2] * x[2];
+      q[d] = M[d] * b[0] + M[3 + d] * b[1] + M[6 + d] * b[2];
+      Qj += b[d] * p[d];
+      Qi += b[d] * (Mi[3 * d] * x[0] + Mi[3 * d + 1] * x[1] + Mi[3 * d + 2] * x[2]);
+    }
+    const double f = -0.5 * g.GK, fw = f * wj, gq = (-0.5 * g.dGr) * (wj * Qi + wi * Qj);
     sumLT += f * Qj;
-    double db0 = 2.0 * L[0] * x0 + L[3] * x1 + L[4] * x2 + L[6] * x1 + L[7] * x2;
-    double db1 = 2.0 * L[1] * x1 + L[3] * x0 + L[5] * x2 - L[6] * x0 + L[8] * x2;
-    double db2 = 2.0 * L[2] * x2 + L[4] * x0 + L[5] * x1 - L[7] * x0 - L[8] * x1;
-    double dx0 = 2.0 * L[0] * b0 + L[3] * b1 + L[4] * b2 - L[6] * b1 - L[7] * b2;
-    double dx1 = 2.0 * L[1] * b1 + L[3] * b0 + L[5] * b2 + L[6] * b0 - L[8] * b2;
-    double dx2 = 2.0 * L[2] * b2 + L[4] * b0 + L[5] * b1 + L[7] * b0 + L[8] * b1;
-    double gq = -0.5 * Q * g.dGr;
-    lv[0] += f * db0; lv[1] += f * db1; lv[2] += f * db2;
-    lx[0] += f * dx0 + gq * x0; lx[1] += f * dx1 + gq * x1; lx[2] += f * dx2 + gq * x2;
+    for (int d = 0; d < 3; ++d) {
+      fx[d] += fw * x[d];
+      fp[d] += f * p[d];
+      fb[d] += fw * b[d];
+      fq[d] += f * q[d];
+      gx[d] += gq * x[d];
+    }
   }
-  for (int d = 0; d < 3; ++d) { out[d] = lx[d]; out[3 + d] = lv[d]; }
+  for (int d = 0; d < 3; ++d) {
+    out[d] = Mi[d] * fb[0] + Mi[3 + d] * fb[1] + Mi[6 + d] * fb[2] + wi * fq[d] + gx[d];
+    out[3 + d] = Mi[3 * d] * fx[0] + Mi[3 * d + 1] * fx[1] + Mi[3 * d + 2] * fx[2] + wi * fp[d];
+  }
   out[6] = sumLT;
 }
 template <int L>
@@ -439,14 +469,15 @@ __device__ __forceinline__ void adj_density(const AdjPtrs& A, const DomainConst&
   double xi[3] = {col(S, C_X, N, i), col(S, C_X + 1, N, i), col(S, C_X + 2, N, i)};
   double vh[3] = {TXV(TX_VH, i), TXV(TX_VH + 1, i), TXV(TX_VH + 2, i)};
   double hi = col(S, C_H, N, i), rhoi = col(S, C_RHO, N, i), wi = col(S, C_MRHO, N, i);
-  double inv_hi = 1.0 / hi, w_rho = -wi / rhoi;
+  const GeoH Hi = geo_h(hi, 1.0 / hi);
+  const double w_rho = -wi / rhoi;
   double ldr = TMP(J_DRHO, i);
   double lvh[3] = {0, 0, 0};
   double lx[3] = {0, 0, 0}, lrho = 0.0, D = 0.0;
   int len = S.row_len[i];
   for (int k = k0; k < len; k += dk) {
     int j = nb_index(S.nbr[(size_t)k * N + i]);
-    GeoD g = geo_d(xi, hi, inv_hi, col(S, C_X, N, j), col(S, C_X + 1, N, j), col(S, C_X + 2, N, j), col(S, C_H, N, j));
+    GeoD g = geo_d(xi, Hi, col(S, C_X, N, j), col(S, C_X + 1, N, j), col(S, C_X + 2, N, j), col(S, C_H, N, j));
     A.gk_start[(size_t)k * N + i] = g.GK;  // R4 reads the same start-state geometry
     A.dg_start[(size_t)k * N + i] = g.dGr;
     double b0 = vh[0] - TXV(TX_VH, j), b1 = vh[1] - TXV(TX_VH + 1, j), b2 = vh[2] - TXV(TX_VH + 2, j);
@@ -698,10 +729,13 @@ __device__ __forceinline__ void adj_accel(const AdjPtrs& A, const DomainConst& K
       double dvx = b0 * g.x0 + b1 * g.x1 + b2 * g.x2;
       if (dvx < 0) {
         hh = (hi + col(S, C_H, N, j)) / 2;
-        iDn = 1.0 / (g.x0 * g.x0 + g.x1 * g.x1 + g.x2 * g.x2 + 0.01 * hh * hh);
+        // 1/Dn and 2/(rho_i + rho_j) from one division
+        const double Dn = g.x0 * g.x0 + g.x1 * g.x1 + g.x2 * g.x2 + 0.01 * hh * hh;
+        const double rs = rhoi + col(S, C_RHO, N, j), inv = 1.0 / (Dn * rs);
+        iDn = rs * inv;
         MU = hh * dvx * iDn;
         Cij = 0.5 * (csi + col(S, C_CS, N, j));
-        irbar = 2.0 / (rhoi + col(S, C_RHO, N, j));
+        irbar = 2.0 * Dn * inv;
         PIs = (Alpha * Cij * MU + Beta * MU * MU) * irbar;
         av = true;
       }

@@ -31,8 +31,7 @@ enum AdjTmp : int {
   J_XN = 0,    // x(n+1) (3)
   J_VN = 3,    // v(n+1) (3)
   J_RHON = 6,  // rho(n+1)
-  J_SR = 7,    // StrainRate (6)
-  J_RR = 13,   // RotationRate (3)
+  J_M = 7,     // StrainRate and RotationRate, as the 3x3 matrix of adj_rates (row-major)
   J_VH = 16,   // half-step velocity (3)
   J_AH = 19,   // acceleration of the second kick (3)
   J_DRHO = 22, // density rate
