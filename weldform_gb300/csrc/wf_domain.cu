@@ -121,14 +121,15 @@ uint64_t spread3(uint64_t v) {
 
 namespace wf {
 // One region of a state copy.  ELL: entry k of particle i at k * N + i, k below
-// len[i].
+// len[i] and below width, the entries per particle that the array has room for
+// (a length is data: it never takes the copy past the array).
 enum CopyKind : int { COPY_BYTES = 0, COPY_ELL };
 struct CopyJob {
   const int* src;
   int* dst;
   const int* len;
   unsigned long long bytes;  // COPY_BYTES
-  int kind;
+  int kind, width;
 };
 constexpr int MAX_COPY_JOBS = 32;
 struct CopyJobs {
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(256) k_copy_state(const __grid_constant__ Copy
       for (size_t w = n16 * 4 + t0; w < c.bytes / 4; w += stride) c.dst[w] = c.src[w];
     } else {
       for (size_t i = t0; i < N; i += stride) {
-        const int len = c.len[i];
+        const int len = min(c.len[i], c.width);
         int k = 0;
         for (; k + 3 < len; k += 4) {
           const int a = c.src[(size_t)k * N + i], b = c.src[(size_t)(k + 1) * N + i], e = c.src[(size_t)(k + 2) * N + i],
@@ -952,8 +953,9 @@ struct wf_domain {
     if (K.skin_on) {
       P.sup = dalloc<int>((size_t)SUP_W * n);
       P.sup_len = dalloc<int>(n);
+      CK(cudaMemsetAsync(P.sup_len, 0, sizeof(int) * n, stream));  // no superset yet: a checkpoint may come first
       P.xref = dalloc<double>((size_t)3 * n);
-      }
+    }
     if (K.nspec > 0) {  // one rebuild schedule per specimen, as a run of it alone starts
       std::vector<SpecState> sp(K.nspec);
       for (SpecState& q : sp) { memset(&q, 0, sizeof(q)); q.nb_cleared = 1; }
@@ -1174,6 +1176,7 @@ struct wf_domain {
       c.len = r.len < 0 ? nullptr : (const int*)(save ? regions[r.len].p : sl[r.len]);
       c.bytes = r.bytes;
       c.kind = r.kind;
+      c.width = (int)(r.bytes / (sizeof(int) * J.N));
     }
     long long b = ((long long)hp.N + 255) / 256 * 4;
     k_copy_state<<<(int)std::min<long long>(std::max<long long>(b, 1), 152 * 8), 256, 0, stream>>>(J);
