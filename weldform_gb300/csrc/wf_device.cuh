@@ -239,8 +239,41 @@ struct SpecState {
   long long searches;
 };
 
+// What the solid particles' fields h, Alpha, Beta, mass and Cs have in common,
+// by which kernels and their constants are chosen.  It belongs to the state: a
+// write of one of those fields forms it anew, a checkpoint keeps it.
+struct UniformConst {
+  int av_uniform;      // 1 when every solid particle has the same Alpha and Beta
+  int av_beta_zero, av_zero;  // uniform constants with beta 0; with both 0
+  float av_alpha, av_beta;  // those values (the mixed acceleration gather skips their loads)
+  // 1 when the two particles of every pair have the same mass: the mass is
+  // uniform, or uniform within each batched specimen (no pair links two
+  // specimens, ERR_SPEC_LINK).  The gathers then take m_j = m_i.
+  int m_pair;
+  // Uniform-particle layout of the mixed records: every solid particle has the
+  // same h and Cs and the pairs' masses agree (m_pair).  The current records
+  // then carry Sigma/rho^2 xz and yz in the last two fields of RC_VW (instead
+  // of h and rho), so the acceleration gather reads four
+  // groups per neighbour instead of five, rho_j = m_i / (m/rho)_j, and every
+  // gather uses the kernel constants of the one h below instead of forming
+  // 1/h per pair.
+  int uni;
+  float h_f, cs_f;     // that h and Cs
+  float inv_h_f;       // 1 / h
+  float gk_c_f;        // 1 / (pi h^5): the 3D cubic spline's gradient factor GK = gk_c_f * w(q)
+  // the plain form's kernel constants for uni: 1/h, and GradKernel = near0 +
+  // near1 q for q < 1, far (2 - q)^2 / r for q < 2
+  double u_inv_h, u_near0, u_near1, u_far;
+  bool operator==(const UniformConst& o) const {
+    return av_uniform == o.av_uniform && av_beta_zero == o.av_beta_zero && av_zero == o.av_zero &&
+           av_alpha == o.av_alpha && av_beta == o.av_beta && m_pair == o.m_pair && uni == o.uni && h_f == o.h_f &&
+           cs_f == o.cs_f && inv_h_f == o.inv_h_f && gk_c_f == o.gk_c_f && u_inv_h == o.u_inv_h &&
+           u_near0 == o.u_near0 && u_near1 == o.u_near1 && u_far == o.u_far;
+  }
+};
+
 // Per-domain constants (set once at the solver prologue; small, by value).
-struct DomainConst {
+struct DomainConst : UniformConst {
   int N, Nsolid, nbc_particles;
   double Cellfac, hmax, dt;
   double inv_dt;       // 1 / dt (the fixed time step)
@@ -270,27 +303,6 @@ struct DomainConst {
   int gradcorr;        // 1: kernel-gradient correction (Domain::gradKernelCorr)
   int auto_ts, auto_ts_acc;  // adaptive time step: velocity / acceleration criteria
   double CFL, sqrt_h_a;      // their coefficients (Domain::CFL, Domain::sqrt_h_a)
-  int av_uniform;      // 1 when every solid particle has the same Alpha and Beta
-  int av_beta_zero, av_zero;  // uniform constants with beta 0; with both 0
-  float av_alpha, av_beta;  // those values (the mixed acceleration gather skips their loads)
-  // 1 when the two particles of every pair have the same mass: the mass is
-  // uniform, or uniform within each batched specimen (no pair links two
-  // specimens, ERR_SPEC_LINK).  The gathers then take m_j = m_i.
-  int m_pair;
-  // Uniform-particle layout of the mixed records: every solid particle has the
-  // same h and Cs and the pairs' masses agree (m_pair).  The current records
-  // then carry Sigma/rho^2 xz and yz in the last two fields of RC_VW (instead
-  // of h and rho), so the acceleration gather reads four
-  // groups per neighbour instead of five, rho_j = m_i / (m/rho)_j, and every
-  // gather uses the kernel constants of the one h below instead of forming
-  // 1/h per pair.
-  int uni;
-  float h_f, cs_f;     // that h and Cs
-  float inv_h_f;       // 1 / h
-  float gk_c_f;        // 1 / (pi h^5): the 3D cubic spline's gradient factor GK = gk_c_f * w(q)
-  // the plain form's kernel constants for uni: 1/h, and GradKernel = near0 +
-  // near1 q for q < 1, far (2 - q)^2 / r for q < 2
-  double u_inv_h, u_near0, u_near1, u_far;
   int lanes64;         // lanes per particle of the plain form's gathers (1, 2 or 4)
   int stage_cap;       // halo capacity of the staged gathers (0: staging off)
   int freeze_nb;       // 1: neighbour and contact topology searched only at the first step

@@ -251,7 +251,11 @@ struct wf_domain {
   struct Region { void* p; size_t bytes; int kind = wf::COPY_BYTES; int len = -1; bool mixed = false; };
   std::vector<Region> regions;           // every mutable device region of the state
   std::vector<std::vector<void*>> slots; // checkpoint copies, one vector per slot
-  std::vector<char> slot_shadows;        // whether the slot holds valid mixed records
+  struct SlotHost {
+    bool shadows = false;      // the slot holds valid mixed records
+    wf::UniformConst uniform;  // the flags and constants of its fields (the records' layout is one of them)
+  };
+  std::vector<SlotHost> slot_host;
   bool shadows_valid = false;  // float shadows of the mixed form match the FP64 state
   long long launches_per_step = 0;     // launches every replay of the step graph makes
   long long search_launches = 0;       // launches in its conditional search body (0: gated form)
@@ -1245,18 +1249,29 @@ struct wf_domain {
     CK(cudaStreamSynchronize(stream));
     set_uniform(a.data(), b.data(), m.data(), h.data(), cs.data(), kind.data(), spec.data(), n);
     shadows_valid = false;
+    drop_graph();
+  }
+  void drop_graph() {  // the next step captures it again
     if (graph) { CK(cudaGraphExecDestroy(graph)); graph = nullptr; }
   }
   void checkpoint_save(int slot) {
     use_device();
-    if ((int)slots.size() <= slot) { slots.resize(slot + 1); slot_shadows.resize(slot + 1, 0); }
+    if ((int)slots.size() <= slot) { slots.resize(slot + 1); slot_host.resize(slot + 1); }
     save_to(slots[slot]);
-    slot_shadows[slot] = shadows_valid;
+    slot_host[slot].shadows = shadows_valid;
+    slot_host[slot].uniform = K;
   }
   void checkpoint_restore(int slot) {
     use_device();
     if ((int)slots.size() <= slot || slots[slot].empty()) throw CudaError{WF_ERR_STATE, "checkpoint slot is empty"};
-    restore_from(slots[slot], slot_shadows[slot]);
+    restore_from(slots[slot], slot_host[slot].shadows);
+    // The flags of the restored fields, and with them the kernels and constants
+    // of the step: captured again where those in force come from other fields.
+    wf::UniformConst& uniform = K;
+    if (!(uniform == slot_host[slot].uniform)) {
+      uniform = slot_host[slot].uniform;
+      drop_graph();
+    }
   }
   void checkpoint_free(int slot) {
     if ((int)slots.size() <= slot) return;
