@@ -147,6 +147,7 @@ __device__ __forceinline__ void adj_conduction(const AdjPtrs& A, const DomainCon
   double xi[3] = {FE(C_X, i), FE(C_X + 1, i), FE(C_X + 2, i)};
   double hi = col(S, C_H, N, i), ki = col(S, C_KT, N, i), Ti = FE(C_T, i), wi = FE(C_MRHO, i);
   const GeoH Hi = geo_h(hi, 1.0 / hi);
+  const double kii = 4. * (ki * ki) / (ki + ki);  // a pair of equal conductivities (0/0 at k = 0, as forward)
   int len = S.row_len[i];
   for (int k = k0; k < len; k += dk) {
     int e = S.nbr[(size_t)k * N + i];
@@ -161,7 +162,7 @@ __device__ __forceinline__ void adj_conduction(const AdjPtrs& A, const DomainCon
     double kj = col(S, C_KT, N, j);
     // equal conductivities need no division (a vote, so that a warp whose pairs
     // all agree branches over it: predicated off it would keep its pipe slots)
-    double kk = ki + ki;
+    double kk = kii;
     if (__any_sync(__activemask(), kj != ki)) kk = kj != ki ? 4. * (ki * kj) / (ki + kj) : kk;
     double dT = Ti - FE(C_T, j);
     ltn += d * w * kk * g.GK;

@@ -973,8 +973,11 @@ __device__ __forceinline__ void rate_sums_uni(const DevPtrs& P, const DomainCons
   const double xi0 = col(P, C_XN, N, i), xi1 = col(P, C_XN + 1, N, i), xi2 = col(P, C_XN + 2, N, i);
   const double vi0 = col(P, C_VN, N, i), vi1 = col(P, C_VN + 1, N, i), vi2 = col(P, C_VN + 2, N, i);
   const double pri = col(P, C_PR2N, N, i);
-  double Ti = 0.0, ki = 0.0, mrhoi = 0.0;
-  if constexpr (THERMAL) { Ti = col(P, C_TN, N, i); ki = col(P, C_KT, N, i); mrhoi = col(P, C_MRHON, N, i); }
+  double Ti = 0.0, ki = 0.0, kii = 0.0, mrhoi = 0.0;
+  if constexpr (THERMAL) {
+    Ti = col(P, C_TN, N, i); ki = col(P, C_KT, N, i); mrhoi = col(P, C_MRHON, N, i);
+    kii = 4. * (ki * ki) / (ki + ki);  // of a pair of equal conductivities: formed once, 0/0 at k = 0 as in every form
+  }
   double M[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // sum (m_j / rho_j) GK v_k x_l
   double dkin = 0.0, cond = 0.0;
   const int len = P.row_len[i];
@@ -999,7 +1002,7 @@ __device__ __forceinline__ void rate_sums_uni(const DevPtrs& P, const DomainCons
       // 4 ki kj / (ki + kj) (Ti - Tj) x.(GK x) / r^2 with x.x = r^2; the
       // reference's 0/0 of coincident particles stays a NaN
       const double kj = col(P, C_KT, N, j);
-      const double c = kj == ki ? ki + ki : 4. * (ki * kj) / (ki + kj);
+      const double c = kj == ki ? kii : 4. * (ki * kj) / (ki + kj);
       const double gr = g.r2 > 0.0 ? g.GK : __longlong_as_double(0x7ff8000000000000ll);
       cond += (nb_up(e) ? mrhoj : mrhoi) * c * (Ti - col(P, C_TN, N, j)) * gr;  // m_P2 / rho_P2 for both ends
     }
