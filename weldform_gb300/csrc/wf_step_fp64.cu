@@ -174,10 +174,10 @@ __device__ __forceinline__ UniGeo uni_geo(const DomainConst& K, double x0, doubl
   g.r2 = fma(x2, x2, fma(x1, x1, __dmul_rn(x0, x0)));
   g.ir = g.r2 > 0.0 ? rsqrt(g.r2) : 0.0;
   const double q = __dmul_rn(__dmul_rn(g.r2, g.ir), K.u_inv_h);
-  const int hq = __double2hiint(q);  // q >= 0: its high word orders as q does (NaN above both bounds)
+  const unsigned hq = (unsigned)__double2hiint(q);  // q >= 0: its high word orders as q does (a NaN of either sign above both bounds)
   const double t = __dsub_rn(2.0, q);
   const double near = fma(K.u_near1, q, K.u_near0), far = __dmul_rn(__dmul_rn(K.u_far, g.ir), __dmul_rn(t, t));
-  g.GK = hq < 0x3ff00000 ? near : (hq < 0x40000000 ? far : 0.0);
+  g.GK = hq < 0x3ff00000u ? near : (hq < 0x40000000u ? far : 0.0);
   return g;
 }
 // Sum over the L lanes of a particle (all lanes end with it).
