@@ -275,23 +275,15 @@ struct wf_domain {
     cudaEvent_t ready = nullptr, done = nullptr;  // gathered; copied out
     bool used = false;
   };
-  // Staging of synchronous transfers, kept from one to the next (at most 9
-  // doubles per particle): allocated and freed on every call, with the stream
-  // synchronised in between, a read of 8,004 particles took 200 us, of which
-  // the gather and the copy are 20.
-  void* xfer = nullptr;
-  size_t xfer_bytes = 0;
-  template <class T> T* staging(size_t n) {
-    const size_t bytes = std::max<size_t>(n * sizeof(T), 1);
-    if (bytes > xfer_bytes) {
-      if (xfer) CK(cudaFree(xfer));  // no transfer is in flight between calls
-      xfer = nullptr;
-      xfer_bytes = 0;
-      cudaError_t e = cudaMalloc(&xfer, bytes);
-      if (e != cudaSuccess) throw CudaError{WF_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
-      xfer_bytes = bytes;
-    }
-    return (T*)xfer;
+  // Staging of synchronous transfers (at most 9 doubles per particle): the
+  // search's permutation scratch, which is larger.  Transfers and searches
+  // follow one another on the domain's stream, and a transfer is over when its
+  // call returns.  Allocated and freed on every call, a read of 8,004 particles
+  // took 200 us, of which the gather and the copy are 20; a buffer of its own,
+  // grown at the first reads, cost a new domain of 522,972 particles 3.4 ms.
+  template <class T> T* staging() const {
+    static_assert(wf::NF64_PERSIST >= 9, "room for a 3x3 tensor per particle");
+    return reinterpret_cast<T*>(d_fscratch);
   }
   std::vector<Snapshot> snaps = std::vector<Snapshot>(4);  // a ring: four reads in flight
   size_t snap_next = 0;
@@ -399,7 +391,6 @@ struct wf_domain {
     if (graph) { cudaGraphExecDestroy(graph); graph = nullptr; }
     for (void* p : allocs) cudaFree(p);
     allocs.clear();
-    if (xfer) { cudaFree(xfer); xfer = nullptr; xfer_bytes = 0; }
     if (body_stream) { cudaStreamDestroy(body_stream); body_stream = nullptr; }
     if (copy_stream) { cudaStreamSynchronize(copy_stream); cudaStreamDestroy(copy_stream); copy_stream = nullptr; }
     for (auto& sn : snaps) {
@@ -1566,7 +1557,7 @@ struct wf_domain {
       return;
     }
     use_device();
-    double* tmp = staging<double>(n * ncomp);
+    double* tmp = staging<double>();
     wf::launch_gather_orig(P, K, d_f + (size_t)c * n, tmp, ncomp, stream);
     CK(cudaMemcpyAsync(dst, tmp, sizeof(double) * n * ncomp, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
@@ -1576,7 +1567,7 @@ struct wf_domain {
   void get_f64_tensor(int c, int anti, double* dst) {
     size_t n = hp.N;
     use_device();
-    double* tmp = staging<double>(n * 9);
+    double* tmp = staging<double>();
     wf::launch_gather_orig_tensor(P, K, d_f + (size_t)c * n, tmp, anti, stream);
     CK(cudaMemcpyAsync(dst, tmp, sizeof(double) * n * 9, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
@@ -1622,7 +1613,7 @@ struct wf_domain {
       return;
     }
     use_device();
-    double* tmp = staging<double>(n * ncomp);
+    double* tmp = staging<double>();
     CK(cudaMemcpyAsync(tmp, src, sizeof(double) * n * ncomp, cudaMemcpyHostToDevice, stream));
     wf::launch_scatter_orig(P, K, tmp, d_f + (size_t)c * n, ncomp, stream);
     wf::launch_refresh_derived(P, K, stream);
@@ -1636,7 +1627,7 @@ struct wf_domain {
     size_t n = hp.N;
     if (!prepared) { for (size_t p = 0; p < n; ++p) dst[p] = hp.i[c][p]; return; }
     use_device();
-    int* tmp = staging<int>(n);
+    int* tmp = staging<int>();
     wf::launch_gather_orig_i32(P, K, d_i + (size_t)c * n, tmp, stream);
     CK(cudaMemcpyAsync(dst, tmp, sizeof(int) * n, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
