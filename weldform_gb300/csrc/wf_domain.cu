@@ -666,11 +666,12 @@ struct wf_domain {
       auto fullest = [&] {  // particles of the fullest brick
         const int nb[3] = {(CellNo[0] - 1) / BK[0] + 1, (CellNo[1] - 1) / BK[1] + 1, (CellNo[2] - 1) / BK[2] + 1};
         std::vector<int> bc((size_t)nb[0] * nb[1] * nb[2], 0);
-        size_t lin = 0;
+        const int* n = cc.data();
         for (int a = 0; a < CellNo[0]; ++a)
-          for (int b = 0; b < CellNo[1]; ++b)
-            for (int c = 0; c < CellNo[2]; ++c, ++lin)
-              bc[((size_t)(a / BK[0]) * nb[1] + b / BK[1]) * nb[2] + c / BK[2]] += cc[lin];
+          for (int b = 0; b < CellNo[1]; ++b) {
+            int* row = bc.data() + ((size_t)(a / BK[0]) * nb[1] + b / BK[1]) * nb[2];
+            for (int c = 0; c < CellNo[2]; ++c) row[c] += *n++;  // BK[2] is 1
+          }
         return *std::max_element(bc.begin(), bc.end());
       };
       while (BK[0] * BK[1] > 1 && fullest() > BRICK_CAP - BRICK_CAP / 16) {
@@ -679,21 +680,25 @@ struct wf_domain {
         else BK[0] /= 2;
       }
     }
-    std::vector<std::pair<uint64_t, int>> mc((size_t)ncells);
-    for (int a = 0; a < CellNo[0]; ++a)
-      for (int b = 0; b < CellNo[1]; ++b)
-        for (int c = 0; c < CellNo[2]; ++c) {
-          int lin = (a * CellNo[1] + b) * CellNo[2] + c;
-          mc[lin] = {spread3(a / BK[0]) | (spread3(b / BK[1]) << 1) | (spread3(c / BK[2]) << 2), lin};
+    std::vector<std::pair<uint64_t, int>> bm;  // bricks by Morton code
+    const int nby = (CellNo[1] - 1) / BK[1] + 1, nbz = CellNo[2];
+    for (int a = 0; a * BK[0] < CellNo[0]; ++a)
+      for (int b = 0; b < nby; ++b)
+        for (int c = 0; c < nbz; ++c) bm.push_back({spread3(a) | (spread3(b) << 1) | (spread3(c) << 2), (a * nby + b) * nbz + c});
+    std::sort(bm.begin(), bm.end());
+    std::vector<int> rank((size_t)ncells), lin((size_t)ncells), brick;
+    int r = 0;
+    for (const auto& m : bm) {
+      brick.push_back(r);
+      const int a0 = m.second / nbz / nby * BK[0], b0 = m.second / nbz % nby * BK[1], c = m.second % nbz;
+      for (int a = a0; a < std::min(a0 + BK[0], CellNo[0]); ++a)
+        for (int b = b0; b < std::min(b0 + BK[1], CellNo[1]); ++b, ++r) {
+          lin[r] = (a * CellNo[1] + b) * CellNo[2] + c;
+          rank[lin[r]] = r;
         }
-    std::sort(mc.begin(), mc.end());
-    std::vector<int> brick;
-    for (long long r = 0; r < ncells; ++r)
-      if (r == 0 || mc[r].first != mc[r - 1].first) brick.push_back((int)r);
-    for (long long r = ncells; r < 2 * ncells; r += BK[0] * BK[1] * BK[2]) brick.push_back((int)r);
+    }
+    for (long long q = ncells; q < 2 * ncells; q += BK[0] * BK[1]) brick.push_back((int)q);
     brick.push_back((int)(2 * ncells));
-    std::vector<int> rank((size_t)ncells);
-    for (long long r = 0; r < ncells; ++r) rank[mc[r].second] = (int)r;
 
     // Device allocations.
     size_t n = N;
@@ -719,14 +724,9 @@ struct wf_domain {
     int* crank = dalloc<int>(ncells);
     CK(cudaMemcpyAsync(crank, rank.data(), sizeof(int) * ncells, cudaMemcpyHostToDevice, stream));
     P.cell_rank = crank;
-    {
-      std::vector<int> lin(ncells);
-      for (size_t c = 0; c < (size_t)ncells; ++c) lin[rank[c]] = (int)c;
-      int* clin = dalloc<int>(ncells);
-      CK(cudaMemcpyAsync(clin, lin.data(), sizeof(int) * ncells, cudaMemcpyHostToDevice, stream));
-      CK(cudaStreamSynchronize(stream));  // the host vector dies at the end of this scope
-      P.cell_lin = clin;
-    }
+    int* clin = dalloc<int>(ncells);
+    CK(cudaMemcpyAsync(clin, lin.data(), sizeof(int) * ncells, cudaMemcpyHostToDevice, stream));
+    P.cell_lin = clin;
     // grid cells, then as many shadow buckets for particles with a non-finite position
     P.cell_start = dalloc<int>(2 * ncells + 1);
     P.cell_count = dalloc<int>(2 * ncells);
