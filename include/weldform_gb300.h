@@ -144,7 +144,11 @@ int wf_set_domain_i32(wf_domain* d, const char* name, int value);
  * "uniform_layout" (1 when the mixed records take the four-group
  * uniform-particle layout: h and Cs uniform, and every pair's masses equal —
  * uniform, or uniform within each batched specimen), "skin_reuse" (1 when the
- * Verlet-skin reuse of the search is on). */
+ * Verlet-skin reuse of the search is on), "cell_order" (1 when the program's
+ * numbering does not run through space, fewer than 4 of 5 successive solid
+ * particles being in the same or neighbouring cells at the prologue: storage
+ * then follows the cells, else the numbering; results do not depend on it but
+ * for the order of the energy sums). */
 int wf_get_domain_f64(wf_domain* d, const char* name, double* value);
 int wf_get_domain_i32(wf_domain* d, const char* name, int64_t* value);
 

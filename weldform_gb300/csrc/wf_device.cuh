@@ -282,6 +282,7 @@ struct DomainConst : UniformConst {
   double rec_origin[3];  // the mixed form's position records hold x - rec_origin (the cell grid's centre)
   int ncells;
   int nbricks;         // bricks of cells (with those of the shadow buckets): the units of the storage order
+  int cell_order;      // 1: a brick's particles cell after cell, 0: in original order throughout
   float pre_eps;       // relative margin of the FP32 neighbour prefilter
   float cell_skip_r2;  // (Cellfac * hmax + FP32 rounding margin)^2: cells farther hold no neighbour
   float CellSizef[3];  // FP32 copy of the cell size

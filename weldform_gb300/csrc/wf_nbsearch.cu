@@ -217,21 +217,32 @@ __global__ void k_scatter(DevPtrs P, DomainConst K) {
 // a cell's particles are no longer contiguous.  A brick above BRICK_CAP
 // particles (bodies crushed into few cells) ranks its slots by counting the
 // smaller keys tile by tile.  Shadow buckets are grouped into bricks as well.
+// Where the numbering does not run through space (DomainConst::cell_order) the
+// key begins with the cell, so that a brick's particles lie cell by cell.
 constexpr int BRICK_T = 1024;
 constexpr int BRICK_PER = BRICK_CAP / BRICK_T;  // slots per thread
 __global__ void __launch_bounds__(BRICK_T) k_sort_bricks(DevPtrs P, DomainConst K) {
   if (!searching_full(P)) return;
-  __shared__ unsigned long long kv[BRICK_CAP];  // (original index, slot)
+  __shared__ unsigned long long kv[BRICK_CAP];  // (cell of the brick,) original index, slot
   const int t = threadIdx.x;
   const int* orig = P.i + I_ORIG * (size_t)K.N;
+  const int* cell = P.i + I_CELL * (size_t)K.N;
+  static_assert(BRICK_CAP <= 1 << 12, "a slot in 12 bits of the key");
   for (int b = blockIdx.x; b < K.nbricks; b += gridDim.x) {
     const int s0 = P.cell_start[P.brick_cell[b]], n = P.cell_start[P.brick_cell[b + 1]] - s0;
     if (n <= 0) continue;  // uniform over the block
     if (n <= BRICK_CAP) {
       int P2 = 2;
       while (P2 < n) P2 <<= 1;
-      for (int e = t; e < P2; e += BRICK_T)
-        kv[e] = e < n ? ((unsigned long long)(unsigned)orig[P.perm[s0 + e]] << 32) | (unsigned)e : ~0ull;
+      for (int e = t; e < P2; e += BRICK_T) {
+        unsigned long long v = ~0ull;
+        if (e < n) {
+          const int q = P.perm[s0 + e];
+          v = ((unsigned long long)(unsigned)orig[q] << 12) | (unsigned)e;
+          if (K.cell_order) v |= (unsigned long long)(cell[q] - P.brick_cell[b]) << 44;
+        }
+        kv[e] = v;
+      }
       __syncthreads();
       for (int size = 2; size <= P2; size <<= 1)
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
@@ -247,7 +258,7 @@ __global__ void __launch_bounds__(BRICK_T) k_sort_bricks(DevPtrs P, DomainConst 
       for (int r = 0; r < BRICK_PER; ++r) {
         const int q = t + r * BRICK_T;
         if (q < n) {
-          const int e = (int)(kv[q] & 0xffffffffu);
+          const int e = (int)(kv[q] & 0xfffu);
           p[r] = P.perm[s0 + e];
           P.cell_list[s0 + e] = s0 + q;
         }
