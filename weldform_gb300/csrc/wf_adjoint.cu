@@ -39,9 +39,7 @@ static_assert(ADJ_BLOCK == BLOCK, "the finish kernel's partials are sized by ADJ
 //   1 <= q < 2: GK = -3/4 C (2 - q)^2 / r,  dGK/dr = 3/4 C (4 - q^2) / r^2
 // with r and 1/r from one reciprocal square root per pair and the constants of
 // the own smoothing length formed once; a pair of different lengths forms its
-// own (behind a vote, so that a warp without one branches over the division
-// instead of running it predicated off).  The values equal the forward's to
-// rounding.
+// own (branch_over).  The values equal the forward's to rounding.
 struct GeoD {
   double x0, x1, x2, r, GK, dGr;  // dGr = (dGK/dr) / r
 };
@@ -59,9 +57,7 @@ __device__ __forceinline__ GeoD geo_d(const double xi[3], const GeoH& own, doubl
   const double rinv = r2 > 0.0 ? rsqrt(r2) : 0.0;
   g.r = r2 * rinv;
   GeoH H = own;
-  if (__any_sync(__activemask(), hj != own.h)) {
-    if (hj != own.h) H = geo_h(0.5 * (own.h + hj), 2.0 / (own.h + hj));
-  }
+  branch_over(hj != own.h, [&] { H = geo_h(0.5 * (own.h + hj), 2.0 / (own.h + hj)); });
   const double q = g.r * H.inv_h;
   double dG = 0.0;
   g.GK = 0.0;
@@ -160,10 +156,8 @@ __device__ __forceinline__ void adj_conduction(const AdjPtrs& A, const DomainCon
     bool up = nb_up(e);  // j has the larger original index: P2 = j
     double w = up ? FE(C_MRHO, j) : wi;  // m_P2 / rho_P2 at both ends (Thermal.cpp:127-131)
     double kj = col(S, C_KT, N, j);
-    // equal conductivities need no division (a vote, so that a warp whose pairs
-    // all agree branches over it: predicated off it would keep its pipe slots)
-    double kk = kii;
-    if (__any_sync(__activemask(), kj != ki)) kk = kj != ki ? 4. * (ki * kj) / (ki + kj) : kk;
+    double kk = kii;  // equal conductivities need no division
+    branch_over(kj != ki, [&] { kk = 4. * (ki * kj) / (ki + kj); });
     double dT = Ti - FE(C_T, j);
     ltn += d * w * kk * g.GK;
     double cx = d * w * kk * dT * g.dGr;

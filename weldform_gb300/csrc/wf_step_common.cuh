@@ -179,19 +179,34 @@ __device__ __forceinline__ void ff_split(double v, float& hi, float& lo) {
   hi = __double2float_rn(v);
   lo = __double2float_rn(v - (double)hi);
 }
-// Three splits with one vote, so that a warp branches over the conversions
-// instead of running them predicated off, which still takes their slots of the
-// FP64 pipe (the kick kernel, whose work this is: 37.5 -> 31.4 us at 982,072
-// particles, with contact 69 -> 59 us at 1,171,832; the rate-stress and density
-// kernels lost more to the registers that grouping holds).
+// f() where c holds, behind a branch that a warp without such a lane takes.  A
+// short body would be compiled to instructions predicated off, which still take
+// their slots of the FP64 pipe; the count of this loop is hidden from the
+// compiler.  No vote: the lanes here need not be together.
+template <class F>
+__device__ __forceinline__ void branch_over(bool c, F f) {
+  int n = c ? 1 : 0;
+  asm volatile("" : "+r"(n));
+#pragma unroll 1
+  while (n > 0) {
+    f();
+    --n;
+    asm volatile("" : "+r"(n));
+  }
+}
+// Three splits that share one branch over the conversions (the kick kernel,
+// whose work this is: 37.5 -> 31.4 us at 982,072 particles, with contact 69 ->
+// 59 us at 1,171,832; the rate-stress and density kernels lost more to the
+// registers that grouping holds).
 __device__ __forceinline__ void ff_split3(const double v[3], float hi[3], float lo[3]) {
   bool odd = false;
   for (int d = 0; d < 3; ++d) ff_split_int(v[d], hi[d], lo[d], odd);
-  if (__any_sync(__activemask(), odd))
+  branch_over(odd, [&] {
     for (int d = 0; d < 3; ++d) {
       hi[d] = __double2float_rn(v[d]);
       lo[d] = __double2float_rn(v[d] - (double)hi[d]);
     }
+  });
 }
 // Low-half group: x = (xlo0, xlo1), y = (xlo2, vlo0), z = (vlo1, vlo2) as bf16
 // pairs (first value in the low 16 bits), w = a float.  A bf16 is the upper
