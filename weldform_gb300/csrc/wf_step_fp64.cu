@@ -1438,8 +1438,8 @@ void launch_contact_kick(const DevPtrs& P, const DomainConst& K, cudaStream_t s)
   }
   if (!K.contact) k_contact_kick<0><<<K.nblocks, K.pblock, 0, s>>>(P, K);
   else if (K.nmeshes == 1) {
-    // a few blocks per SM stride over the particles in contact
-    const long long most = (32LL * K.Nsolid + 127) / 128;
+    // a few blocks per SM stride over the particles in contact (one block where there is no solid particle)
+    const long long most = K.Nsolid > 0 ? (32LL * K.Nsolid + 127) / 128 : 1;
     k_contact_force<<<(int)(most < 152 * 4 ? most : 152 * 4), 128, 0, s>>>(P, K);
     mark(s, "k_contact_force");
     k_contact_kick<1><<<K.nblocks, K.pblock, 0, s>>>(P, K);
