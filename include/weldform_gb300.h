@@ -13,7 +13,7 @@
  *    No exception ever crosses the ABI (the reference throws `new Fatal`,
  *    External/fatal.h:58-63, or calls abort(), Functions.cpp:64-70).
  *  - Particles are addressed in the reference's insertion order ("original
- *    index"); the library reorders them internally (cell-sorted) and maps
+ *    index"); the library reorders them internally (by cells) and maps
  *    indices back on every host transfer.
  *  - Vectors are passed as double[3]; per-particle arrays as flat host
  *    buffers (n * components, row-major).  The library copies inputs and

@@ -1,8 +1,9 @@
 // Device-side data layout of the GB300 kick-drift SPH step (host + device).
 //
 // Particle state lives in one structure-of-arrays arena in HBM, one column of
-// N values per scalar component, in cell-sorted order.  The host keeps the map
-// between this order and the reference's particle order ("original index").
+// N values per scalar component, in the search's storage order (bricks of
+// cells, k_sort_bricks).  The host keeps the map between this order and the
+// reference's particle order ("original index").
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -63,7 +64,7 @@ enum I32Col : int {
 // ---- float4 field groups of the mixed form -----------------------------------
 // The FP32 data a neighbour's gather reads is packed four fields to a float4,
 // one float4 column per group (group q of particle i at rc[q * N + i]).  In
-// cell-sorted order the k-th neighbours of a warp's 32 consecutive particles
+// storage order the k-th neighbours of a warp's 32 consecutive particles
 // have nearly consecutive indices, so each 16-byte load coalesces into a few
 // lines — better than one column per field (more load instructions) and
 // better than one record per particle (one line per lane).  Positions,
@@ -133,7 +134,7 @@ constexpr int SUP_W = 128;   // superset entries per particle (skin reuse of the
 constexpr int BRICK_CAP = 4096;  // particles of a brick that the search orders in shared memory
 
 // Shared-memory staging of the mixed form's gathers.  Particles are taken in
-// blocks of STAGE_B consecutive (cell-sorted) particles; at every search each
+// blocks of STAGE_B consecutive particles; at every search each
 // block's distinct neighbours are listed once, sorted by index (its halo,
 // at most stage_cap of them), and every row entry gets its neighbour's slot
 // in that list.  A staged gather copies the halo's float4 groups into shared

@@ -5,7 +5,8 @@
 // reference's insertion order (generators, zones, per-particle fields).  The
 // prologue uploads it into the device arena, builds the cell grid
 // (CellInitiate, Neighbour.cpp:10-139) and from then on all state lives in
-// HBM in cell-sorted order; host transfers map through the original index.
+// HBM in the search's storage order (bricks of cells); host transfers map
+// through the original index.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -279,8 +280,9 @@ struct wf_domain {
   // search's permutation scratch, which is larger.  Transfers and searches
   // follow one another on the domain's stream, and a transfer is over when its
   // call returns.  Allocated and freed on every call, a read of 8,004 particles
-  // took 200 us, of which the gather and the copy are 20; a buffer of its own,
-  // grown at the first reads, cost a new domain of 522,972 particles 3.4 ms.
+  // took 200 us, of which the gather and the copy are 20; a buffer of its own
+  // was allocated twice by the first reads (vector, then tensor: 0.3 ms at
+  // 522,972 particles).
   template <class T> T* staging() const {
     static_assert(wf::NF64_PERSIST >= 9, "room for a 3x3 tensor per particle");
     return reinterpret_cast<T*>(d_fscratch);

@@ -128,10 +128,10 @@ struct PairGeo {
 // (Functions.cpp:74-87), C = 1 / (pi h^4):
 //   q < 1:      GK = C/h (-3 + 9/4 q)
 //   1 <= q < 2: GK = -3/4 C (2 - q)^2 / (q h) = -3/4 C (2 - q)^2 / r
-// GB300 runs FP64 division as a multi-instruction sequence at 1/64 of the
-// FP32 rate, so the pair takes one division (C / r, only for q >= 1) plus
-// 1/h when the two smoothing lengths differ; inv_hi = 1/h_i comes from the
-// caller.  Equal to the reference's expression to rounding.
+// GB300 runs an FP64 division as a multi-instruction sequence (61 G/s against
+// 504 G/s fused multiply-adds), so the pair takes one division (C / r, only
+// for q >= 1) plus 1/h when the two smoothing lengths differ; inv_hi = 1/h_i
+// comes from the caller.  Equal to the reference's expression to rounding.
 __device__ __forceinline__ PairGeo pair_geo(double xi0, double xi1, double xi2, double hi, double inv_hi, double xj0,
                                            double xj1, double xj2, double hj) {
   PairGeo g;

@@ -9,7 +9,7 @@
 //    load from each of ~20 separate columns;
 //  * relative positions, velocities and temperatures come from float-float
 //    pairs, (hi_i - hi_j) + (lo_i - lo_j), with FP32 instructions only (GB300
-//    issues FP64 at 1/72 of its FP32 rate).  Temperature low halves are FP32,
+//    runs FP64 at a measured 1/72 of its FP32 rate).  Temperature low halves are FP32,
 //    which gives the FP32 rounding of the FP64 difference; position and
 //    velocity low halves are bf16, which adds at most ~2^-33 |x - O| (O the
 //    records' origin, the cell grid's centre) or ~2^-33 |v| to the difference
@@ -144,7 +144,8 @@ __device__ __forceinline__ void run_rows(const DomainConst& K, Body body) {
 // entries ahead alone; with the packed arithmetic 1.069 with one record and
 // 0.972 with two (at 64, 72 and 96 registers the rate-stress kernel took 499,
 // 473 and 514 us against 425 at 80; the acceleration 291, 288 and 333 us
-// against 255).
+// against 255).  Since then the rate-stress kernel lost conversions (393 us) and
+// the acceleration had the roundings of its pair terms spelled out (270 us).
 template <class Key, class Load, class Body>
 __device__ __forceinline__ void walk_row(int k0, int dk, int len, Key key, Load load, Body body) {
   int n0 = k0 < len ? key(k0) : 0, n1 = k0 + dk < len ? key(k0 + dk) : 0;
@@ -600,8 +601,6 @@ struct MoveRec {
 };
 
 // ---------------------------------------------------------------- density + drift + kick
-// GC: the locking sum with corrected gradients, m_j (rho_i / rho_j) v_ij . vc_i
-// (InteractionAlt.cpp:589-605), which carries rho_i inside the sum.
 // L lanes per particle (L = 1: one thread walks the row): lane `sub` sums
 // entries sub, sub + L, ...; with L > 1 the lanes' compensated values are
 // added in FP64 by a butterfly of warp shuffles (every thread of the warp
