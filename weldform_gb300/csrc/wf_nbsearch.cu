@@ -214,9 +214,11 @@ __global__ void k_scatter(DevPtrs P, DomainConst K) {
 // particles went from 87 to 54 % of its rate).  One block per brick sorts its
 // slots by a bitonic sort in shared memory, writes the particles in their
 // order (perm) and where each slot of the cells' lists went (cell_list), since
-// a cell's particles are no longer contiguous.  A brick above BRICK_CAP
-// particles (bodies crushed into few cells) ranks its slots by counting the
-// smaller keys tile by tile.  Shadow buckets are grouped into bricks as well.
+// a cell's particles are no longer contiguous.  A brick that has come to hold
+// more than BRICK_CAP particles (a body that left the grid is binned into its
+// edge cells) is taken in parts of whole cells that fit, and a cell that does
+// not fit by itself ranks its slots by counting the smaller keys tile by tile.
+// Shadow buckets are grouped into bricks as well.
 // Where the numbering does not run through space (DomainConst::cell_order) the
 // key begins with the cell, so that a brick's particles lie cell by cell.
 constexpr int BRICK_T = 1024;
@@ -228,9 +230,16 @@ __global__ void __launch_bounds__(BRICK_T) k_sort_bricks(DevPtrs P, DomainConst 
   const int* orig = P.i + I_ORIG * (size_t)K.N;
   const int* cell = P.i + I_CELL * (size_t)K.N;
   static_assert(BRICK_CAP <= 1 << 12, "a slot in 12 bits of the key");
-  for (int b = blockIdx.x; b < K.nbricks; b += gridDim.x) {
-    const int s0 = P.cell_start[P.brick_cell[b]], n = P.cell_start[P.brick_cell[b + 1]] - s0;
-    if (n <= 0) continue;  // uniform over the block
+  for (int b = blockIdx.x; b < K.nbricks; b += gridDim.x)
+  for (int c0 = P.brick_cell[b], c1 = P.brick_cell[b + 1], ce; c0 < c1; c0 = ce) {  // uniform over the block
+    const int s0 = P.cell_start[c0];
+    ce = c1;
+    if (P.cell_start[c1] - s0 > BRICK_CAP) {  // as many cells as fit, one at least (a brick has up to 256)
+      const int fit = __syncthreads_count(c0 + t < c1 && P.cell_start[c0 + t + 1] - s0 <= BRICK_CAP);
+      ce = c0 + (fit > 1 ? fit : 1);
+    }
+    const int n = P.cell_start[ce] - s0;
+    if (n <= 0) continue;
     if (n <= BRICK_CAP) {
       int P2 = 2;
       while (P2 < n) P2 <<= 1;
@@ -239,7 +248,7 @@ __global__ void __launch_bounds__(BRICK_T) k_sort_bricks(DevPtrs P, DomainConst 
         if (e < n) {
           const int q = P.perm[s0 + e];
           v = ((unsigned long long)(unsigned)orig[q] << 12) | (unsigned)e;
-          if (K.cell_order) v |= (unsigned long long)(cell[q] - P.brick_cell[b]) << 44;
+          if (K.cell_order) v |= (unsigned long long)(cell[q] - c0) << 44;
         }
         kv[e] = v;
       }
@@ -299,8 +308,8 @@ __global__ void __launch_bounds__(BRICK_T) k_sort_bricks(DevPtrs P, DomainConst 
       for (int e = t; e < n; e += BRICK_T) P.perm[s0 + e] = tmp[s0 + e];
     }
     // the cells' counts (the scatter's cursors) back to zero for the next search
-    for (int c = P.brick_cell[b] + t; c < P.brick_cell[b + 1]; c += BRICK_T) P.cell_count[c] = 0;
-    __syncthreads();  // the shared keys are reused by the next brick
+    for (int c = c0 + t; c < ce; c += BRICK_T) P.cell_count[c] = 0;
+    __syncthreads();  // the shared keys are reused by the next cells
   }
 }
 
